@@ -127,7 +127,7 @@ NBSP_HIDDEN void nbsp_centre_of_mass(const double* x, const double* y, const dou
                                      cudaStream_t stream);
 
 /* O(N^2) FP64 potential energy -G sum_{i<j} m_i m_j / sqrt(d^2 + eps^2).
- * `rows` >= n doubles; result in out[0]. */
+ * `rows` >= max(n, 11264) doubles (partial sums); result in out[0]. */
 NBSP_HIDDEN void nbsp_potential_energy(const double* x, const double* y, const double* z,
                                        const double* m, size_t n, double gravitational_constant,
                                        double softening_squared, double* rows, double* out,
