@@ -531,33 +531,40 @@ struct Tree {
   int n;
   int2* range;        // [n-1] first, last of internal nodes
   int2* child;        // [n-1] binary ids of the two children
-  int* cell;          // [2n-1] octree level of a cell node, -1 otherwise
-  int* oparent;       // [2n-1] octree parent (binary id) of a cell node, from keep_kernel
+  int* cell;          // [2n-1] octree level of a cell node, -1 otherwise; keep_kernel
+                      // adds 32 times a kept cell's place among its siblings
+  int* oparent;       // [2n-1] octree parent (binary id) of a kept cell, from keep_kernel
+  int2* below;        // [n-1] splitting cells: walk id of the first child, children
+  int* split;         // [n-1] the splitting cells' binary ids
+  int* split_child;   // [8(n-1)] their octree children's binary ids, -1 behind the last
   uint32_t* mask;     // [n]   levels of kept nodes starting at particle k
   uint32_t* offset;   // [n+1] exclusive scan of popcounts; offset[n] = node count
   uint32_t* block_sums;  // scan scratch
-  // octree nodes, depth-first order, capacity 2n-1
-  int4* info;         // next, begin, leaf count (0: internal), parent
+  // Octree nodes carry two numberings, capacity 2n-1 each.  Depth-first (info,
+  // dnode) with skip links: the stackless walk and the training pairs.  Walk
+  // ids (everything else): the root is 0 and the children of every node are
+  // consecutive, in Morton order, so a node's record names them by the first
+  // one and a count, their records share cache lines, and neither the
+  // interaction-list walk nor the moments pass reads a list of children.
+  int4* info;         // depth-first: next, first particle, leaf count (0: internal), walk id
+  float4* dnode;      // depth-first, 2 per node: wnode's first six words
+  int4* link;         // parent, first child (or first particle), count as in wnode, depth-first id
   int* level;
-  int* nchild;
   int* arrive;
   int* height;
   double4* mom;       // mass, com xyz (relative to the centre of mass)
   double* quad64;     // 6 per node: xx xy xz yy yz zz (trace-free)
-  float4* com;        // walk format: com xyz, mass
-  float* ropen2;      // (2h / theta)^2
-  float4* quad;       // 2 per node: (xx, xy, xz, yy), (yz, 0, 0, 0)
-  int* children;      // 8 per internal node, depth-first order (interaction-list walk)
   double* trace64;    // sum m |x - com|^2 per node (FP64)
-  float* side;        // cell side 2h = root side / 2^level
-  float* spread;      // sum m |x - com|^2 / (M side^2): the correction MLP's 10th feature
-  float* shift;       // distance from the cell's geometric centre to its centre of mass
-  float* kmass;       // M side^2: the relative opening test's cell term
-  // what the interaction-list walk reads of a node, in one 32-byte record:
-  // (com xyz, mass), (ropen2, kmass, first particle, count as int bits: the
-  // particle count of a bucket, minus the number of children of an internal node)
+  // what the interaction-list walk reads of a node, in one 32-byte record: (com
+  // xyz, mass), (ropen2 = (2h / theta)^2, kmass = M (2h)^2 of the relative test,
+  // first particle of a bucket or first child, count as int bits: the particles
+  // of a bucket, minus the children of an internal node)
   float4* wnode;      // 2 per node
-  unsigned long long* leaves;  // [1]
+  // quadrupole walk and correction, 2 per node: (xx, xy, xz, yy), (yz, side =
+  // 2h, spread = sum m |x - com|^2 / (M side^2), shift = distance from the
+  // cell's geometric centre to its centre of mass)
+  float4* wquad;
+  unsigned long long* leaves;  // [2]: buckets; splitting cells << 32 | walk ids below the root
 };
 
 constexpr int kScanItems = 2048;
@@ -580,27 +587,24 @@ __host__ __device__ inline Tree tree_layout(uintptr_t p, size_t n_, uintptr_t* e
   t.child = carve<int2>(p, ni);
   t.cell = carve<int>(p, nb);
   t.oparent = carve<int>(p, nb);
+  t.below = carve<int2>(p, ni);
+  t.split = carve<int>(p, ni);
+  t.split_child = carve<int>(p, 8 * ni);
   t.mask = carve<uint32_t>(p, n);
   t.offset = carve<uint32_t>(p, n + 1);
   t.block_sums = carve<uint32_t>(p, (n + kScanItems - 1) / kScanItems + 1);
   t.info = carve<int4>(p, nb);
+  t.dnode = carve<float4>(p, 2 * nb);
+  t.link = carve<int4>(p, nb);
   t.level = carve<int>(p, nb);
-  t.nchild = carve<int>(p, nb);
   t.arrive = carve<int>(p, nb);
   t.height = carve<int>(p, nb);
   t.mom = carve<double4>(p, nb);
   t.quad64 = carve<double>(p, 6 * nb);
-  t.com = carve<float4>(p, nb);
-  t.ropen2 = carve<float>(p, nb);
-  t.quad = carve<float4>(p, 2 * nb);
-  t.children = carve<int>(p, 8 * nb);
   t.trace64 = carve<double>(p, nb);
-  t.side = carve<float>(p, nb);
-  t.spread = carve<float>(p, nb);
-  t.shift = carve<float>(p, nb);
-  t.kmass = carve<float>(p, nb);
   t.wnode = carve<float4>(p, 2 * nb);
-  t.leaves = carve<unsigned long long>(p, 1);
+  t.wquad = carve<float4>(p, 2 * nb);
+  t.leaves = carve<unsigned long long>(p, 2);
   if (end != nullptr) *end = p;
   return t;
 }
@@ -685,74 +689,160 @@ __device__ __forceinline__ int last_of(const Tree& t, int b) {
 // its octree parent splits; the root always is.)
 __device__ __forceinline__ bool splits(const Tree& t, int b, int leaf_capacity) {
   if (b >= t.n - 1) return false;  // a particle
-  const int lvl = t.cell[b];
-  if (lvl < 0 || lvl >= 21) return false;
+  const int cell = t.cell[b];
+  if (cell < 0 || (cell & 31) >= 21) return false;
   const int2 r = t.range[b];
   return r.y - r.x + 1 > leaf_capacity;
 }
 
 // The octree children of splitting cell b, in Morton order: the cells met
-// first below b in the binary tree.  The binary nodes passed on the way have
-// b's own level (they are not cells), at most 7 of them, so the descent is a
-// stack of at most 8 entries; visit(c) is called for each child cell c.
-template <typename Visit>
-__device__ __forceinline__ int octree_children(const Tree& t, int b, int* status, Visit visit) {
-  int stack[8];
-  int top = 0, kids = 0;
+// first below b in the binary tree, at most three binary levels down.  The
+// eight slots are the binary paths; a node that is no cell (it has b's own
+// level) makes room for its two children.  Cell marks, children and ranges of
+// a level's nodes are loaded together, so the descent waits for three loads.
+// first[k] is the first particle of children[k]; returns how many there are.
+__device__ __forceinline__ int octree_children(const Tree& t, int b, int (&children)[8],
+                                               int (&first)[8], int* status) {
+  const int n = t.n;
+  int slot[8], begin[8];
   const int2 c0 = t.child[b];
-  stack[top++] = c0.y;  // right pushed first: the left subtree is visited first
-  stack[top++] = c0.x;
-  for (int guard = 0; top > 0; ++guard) {
-    const int c = stack[--top];
-    if (guard > 16 || c < 0 || c >= 2 * t.n - 1) {
-      atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-      return kids;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) slot[q] = q == 0 ? c0.x : q == 4 ? c0.y : -1;
+  bool bad = false;
+#pragma unroll
+  for (int stride = 4; stride >= 1; stride >>= 1) {
+    int mark[8];
+    int2 below[8];
+#pragma unroll
+    for (int q = 0; q < 8; q += stride) {
+      const int c = slot[q];
+      const bool there = c >= 0 && c < 2 * n - 1, inner = there && c < n - 1;
+      bad |= c >= 2 * n - 1;
+      mark[q] = there ? t.cell[c] : 0;
+      below[q] = inner && stride > 1 ? t.child[c] : make_int2(-1, -1);
+      begin[q] = inner ? t.range[c].x : c - (n - 1);
     }
-    if (t.cell[c] >= 0) {
-      if (kids == 8) {
-        atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-        return kids;
+#pragma unroll
+    for (int q = 0; q < 8; q += stride) {
+      if (mark[q] >= 0) continue;
+      // a particle that is no cell, or a descent deeper than one octree level
+      bad |= below[q].x < 0;
+      slot[q] = below[q].x;
+      if (stride > 1) slot[q + stride / 2] = below[q].y;
+    }
+  }
+  int kids = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (slot[q] < 0) continue;
+    bad |= begin[q] < 0 || begin[q] >= n;
+#pragma unroll
+    for (int k = 0; k <= q; ++k)
+      if (k == kids) {
+        children[k] = slot[q];
+        first[k] = begin[q];
       }
-      visit(c, kids++);
-    } else if (c < t.n - 1 && top <= 6) {  // a binary node at b's level: its children
-      const int2 cc = t.child[c];
-      stack[top++] = cc.y;
-      stack[top++] = cc.x;
-    } else {  // a particle that is no cell, or a descent deeper than one octree level
-      atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-      return kids;
-    }
+    ++kids;
+  }
+  if (bad) {
+    atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+    return 0;
   }
   return kids;
 }
 
+// Octree level of cell node b, and its place among its octree siblings.
+__device__ __forceinline__ int level_of(const Tree& t, int b) { return t.cell[b] & 31; }
+__device__ __forceinline__ int sibling_of(const Tree& t, int b) { return t.cell[b] >> 5; }
+
 // The kept cells, marked in mask[first particle] at their level (the depth-
 // first numbering counts them): the root, and the octree children of every
-// splitting cell, found by the splitting cell's own thread, which also records
-// itself as their octree parent.  One thread per internal binary node; only
-// the splitting cells (~N / leaf capacity of them) do work.
-__global__ void keep_kernel(Tree t, int leaf_capacity, int* status) {
+// splitting cell, found by one thread per splitting cell, which also records
+// itself as their octree parent and takes consecutive walk ids for them.  A
+// block looks at kKeepNodes internal binary nodes and gathers the splitting ones
+// (~N / leaf capacity of them) in shared memory first, so that their descents —
+// chains of dependent loads — run side by side in whole warps; a descent per
+// thread where it was found left one or two lanes of each warp working.  One
+// atomic per block takes its places in the list of splitting cells and its walk
+// ids (the order of blocks decides where records lie, nothing else).
+// (keep and place, which takes a thread per child: 81 -> 41 us at 1M, 29 -> 20 us at 20k.)
+constexpr int kKeepThreads = 256;
+constexpr int kKeepNodes = 1024;
+__global__ void __launch_bounds__(kKeepThreads) keep_kernel(Tree t, int leaf_capacity, int* status) {
+  __shared__ int s_b[kKeepNodes];
+  __shared__ int s_child[kKeepNodes * 8];
+  __shared__ int warp_kids[kKeepThreads / 32];
+  __shared__ int s_count;
+  __shared__ unsigned long long s_base;
   const int n = t.n;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n - 1) return;
-  if (b == 0) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) s_count = 0;
+  __syncthreads();
+  if (blockIdx.x == 0 && tid == 0) {
     t.oparent[0] = -1;
     if (t.cell[0] < 0) {
       atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-      return;
-    }
-    atomicOr(&t.mask[0], 1u << t.cell[0]);
-  }
-  if (!splits(t, b, leaf_capacity)) return;
-  octree_children(t, b, status, [&](int c, int) {
-    t.oparent[c] = b;
-    const int f = first_of(t, c);
-    if (f >= 0 && f < n) {
-      atomicOr(&t.mask[f], 1u << t.cell[c]);
     } else {
-      atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+      atomicOr(&t.mask[0], 1u << t.cell[0]);
     }
-  });
+  }
+#pragma unroll
+  for (int i = 0; i < kKeepNodes / kKeepThreads; ++i) {
+    const int b = blockIdx.x * kKeepNodes + i * kKeepThreads + tid;
+    const bool split = b < n - 1 && splits(t, b, leaf_capacity);
+    const unsigned m = __ballot_sync(kFull, split);
+    int at = 0;
+    if (lane == 0 && m != 0u) at = atomicAdd(&s_count, __popc(m));
+    at = __shfl_sync(kFull, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (split) s_b[at] = b;
+  }
+  __syncthreads();
+  const int count = s_count;
+  int own = 0;
+  for (int e = tid; e < count; e += kKeepThreads) {
+    const int b = s_b[e];
+    int child[8], begin[8];
+    const int kids = octree_children(t, b, child, begin, status);
+    own += kids;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      s_child[8 * e + k] = k < kids ? child[k] : -1;
+      if (k < kids) {
+        const int lvl = level_of(t, child[k]);
+        t.oparent[child[k]] = b;
+        t.cell[child[k]] = lvl + 32 * k;
+        atomicOr(&t.mask[begin[k]], 1u << lvl);
+      }
+    }
+  }
+  int incl = own;
+  for (int off = 1; off < 32; off <<= 1) {
+    const int u = __shfl_up_sync(kFull, incl, off);
+    if (lane >= off) incl += u;
+  }
+  if (lane == 31) warp_kids[w] = incl;
+  __syncthreads();
+  if (tid == 0) {
+    int total = 0;
+#pragma unroll
+    for (int q = 0; q < kKeepThreads / 32; ++q) {
+      const int c = warp_kids[q];
+      warp_kids[q] = total;
+      total += c;
+    }
+    s_base = count > 0 ? atomicAdd(&t.leaves[1], (unsigned long long)count << 32 | (unsigned)total) : 0;
+  }
+  __syncthreads();
+  int first = 1 + (int)(unsigned)s_base + warp_kids[w] + incl - own;
+  const size_t slot = (size_t)(s_base >> 32);
+  for (int e = tid; e < count; e += kKeepThreads) {
+    int kids = 0;
+    for (int k = 0; k < 8; ++k) kids += s_child[8 * e + k] >= 0;
+    t.below[s_b[e]] = make_int2(first, kids);
+    first += kids;
+  }
+  for (int e = tid; e < count; e += kKeepThreads) t.split[slot + e] = s_b[e];
+  for (int e = tid; e < 8 * count; e += kKeepThreads) t.split_child[8 * slot + e] = s_child[e];
 }
 // Exclusive scan of popc(mask[k]) into offset[0..n].
 __global__ void scan_reduce_kernel(Tree t) {
@@ -844,72 +934,70 @@ __device__ __forceinline__ int dfs_index(const Tree& t, int begin, int lvl) {
   return (int)(t.offset[begin] + __popc(t.mask[begin] & ((1u << lvl) - 1u)));
 }
 
-// The record of kept cell b at depth-first index `node`: next (the first node
-// after its subtree), first particle, particle count (0: internal) and octree
-// parent (-1: the root).
-__device__ __forceinline__ void write_node(const Tree& t, int b, int node, int parent_node,
-                                           bool leaf, int total) {
+// The records of kept cell b, walk id `w` under parent `pw` (-1: the root):
+// skip link (the first node after its subtree), first particle and particle
+// count; a bucket's count is its particles, an internal node's is minus its
+// children.
+__device__ __forceinline__ void write_node(const Tree& t, int b, int w, int pw, bool leaf,
+                                           int total, int* status) {
   const int begin = first_of(t, b), end = last_of(t, b) + 1;
+  const int lvl = level_of(t, b);
+  const int node = dfs_index(t, begin, lvl);
+  int2 below = make_int2(begin, end - begin);
+  if (!leaf) {
+    below = t.below[b];
+    below.y = -below.y;
+  }
+  if (node < 0 || node >= total || w < 0 || w >= total) {
+    atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+    return;
+  }
   const int next = end >= t.n ? total : (int)t.offset[end];
-  t.info[node] = make_int4(next, begin, leaf ? end - begin : 0, parent_node);
-  t.level[node] = t.cell[b];
-  t.arrive[node] = 0;
-  t.height[node] = 1;
+  t.info[node] = make_int4(next, begin, leaf ? end - begin : 0, w);
+  t.link[w] = make_int4(pw, below.x, below.y, node);
+  t.level[w] = lvl;
+  t.arrive[w] = 0;
+  t.height[w] = 1;
 }
 
-// Octree records in depth-first order.  Every splitting cell writes its own
-// record, its children list (in Morton order, which is depth-first order) and
-// the records of its children that are buckets; a splitting child writes its
-// own.  One thread per internal binary node, like keep_kernel.
-__global__ void place_kernel(Tree t, int leaf_capacity, int* status) {
+// Octree records: eight threads per splitting cell, each writing one child's
+// (whose parent's walk id is its place among its own parent's children); the
+// root's by the first thread.
+constexpr int kPlaceBlocks = 8 * 148;
+__global__ void __launch_bounds__(256) place_kernel(Tree t, int leaf_capacity, int* status) {
   const int n = t.n;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
   const int total = (int)t.offset[n];
+  const unsigned long long made = t.leaves[1];
+  const int splitting = (int)(made >> 32);
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+  if (total < 1 || total > 2 * n - 1 || total != 1 + (int)(unsigned)made || splitting > n - 1) {
+    if (thread == 0) atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+    return;
+  }
   int leaves = 0;
-  if (b < n - 1 && (total < 1 || total > 2 * n - 1)) {
-    if (b == 0) atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-  } else if (b < n - 1) {
-    const bool split = splits(t, b, leaf_capacity);
-    if (b == 0 && !split) {  // the root is the only node: one bucket
-      if (total == 1) {
-        write_node(t, 0, 0, -1, true, total);
-        t.nchild[0] = 0;
-        leaves = 1;
-      } else {
+  if (thread == 0) {  // the root may be the only node: one bucket
+    write_node(t, 0, 0, -1, splitting == 0, total, status);
+    leaves = splitting == 0;
+  }
+  for (long long q = thread; q < 8ll * splitting; q += (long long)gridDim.x * blockDim.x) {
+    const int b = t.split[q >> 3], c = t.split_child[q];
+    if (c < 0) continue;
+    if (b < 0 || b >= n - 1 || c >= 2 * n - 1) {
+      atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+      continue;
+    }
+    int w = 0;
+    if (b != 0) {
+      const int p = t.oparent[b];  // keep_kernel: the splitting cell that found b
+      w = p >= 0 && p < n - 1 ? t.below[p].x + sibling_of(t, b) : -1;
+      if (w < 1 || w >= total) {
         atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-      }
-    } else if (split) {
-      const int node = dfs_index(t, first_of(t, b), t.cell[b]);
-      int parent_node = -1;
-      bool ok = node >= 0 && node < total;
-      if (b != 0) {
-        const int p = t.oparent[b];  // keep_kernel: the splitting cell that found b
-        ok = ok && p >= 0 && p < n - 1;
-        if (ok) parent_node = dfs_index(t, first_of(t, p), t.cell[p]);
-        ok = ok && parent_node >= 0 && parent_node < node;  // parents precede children
-      }
-      if (!ok) {
-        atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-      } else {
-        write_node(t, b, node, parent_node, false, total);
-        const int kids = octree_children(t, b, status, [&](int c, int k) {
-          const int cn = dfs_index(t, first_of(t, c), t.cell[c]);
-          if (cn <= node || cn >= total) {
-            atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-            t.children[8 * node + k] = -1;
-            return;
-          }
-          t.children[8 * node + k] = cn;
-          if (!splits(t, c, leaf_capacity)) {  // a bucket
-            write_node(t, c, cn, node, true, total);
-            t.nchild[cn] = 0;
-            ++leaves;
-          }
-        });
-        for (int k = kids; k < 8; ++k) t.children[8 * node + k] = -1;
-        t.nchild[node] = kids;
+        continue;
       }
     }
+    const bool leaf = !splits(t, c, leaf_capacity);
+    write_node(t, c, t.below[b].x + sibling_of(t, c), w, leaf, total, status);
+    leaves += leaf;
   }
   leaves = (int)__reduce_add_sync(kFull, (unsigned)leaves);
   if ((threadIdx.x & 31) == 0 && leaves > 0) atomicAdd(t.leaves, (unsigned long long)leaves);
@@ -945,29 +1033,31 @@ struct Opening {
   int criterion;         // NBSP_BH_OPENING_*
 };
 
+// The records of node `w` from its moments; `first` and `count` as its link has
+// them, `particle` its first particle.
 template <bool QUAD>
-__device__ void finish_node(const Tree& t, int node, const Moments& mo, int first, int lvl,
-                            const Opening& o, int count) {
-  t.mom[node] = make_double4(mo.m, mo.cx, mo.cy, mo.cz);
-  if (QUAD) {
-    for (int k = 0; k < 6; ++k) t.quad64[6 * node + k] = mo.q[k];
-    t.trace64[node] = mo.t2;
-  }
-  t.com[node] = make_float4((float)mo.cx, (float)mo.cy, (float)mo.cz, (float)mo.m);
-  // cell side 2h = root side / 2^lvl; the cell's centre from the first key's
-  // top 3 lvl bits, in the particles' frame (relative to the centre of mass)
+__device__ __forceinline__ void finish_node(const Tree& t, int w, const Moments& mo, int first,
+                                            int count, int dfs, int particle, int lvl,
+                                            const Opening& o) {
+  t.mom[w] = make_double4(mo.m, mo.cx, mo.cy, mo.cz);
+  // cell side 2h = root side / 2^lvl
   const int l = min(lvl, 21);
   const double half = o.geometry[3];
   const double side = ldexp(2.0 * half, -l);
-  const uint64_t key = o.keys[first];
-  double shift2 = 0.0;
-  for (int a = 0; a < 3; ++a) {
-    const double lo = o.geometry[a] - half - o.geometry[4 + a];
-    const double centre = lo + ((double)(compact3(key >> a) >> (21 - l)) + 0.5) * side;
-    const double d = (a == 0 ? mo.cx : a == 1 ? mo.cy : mo.cz) - centre;
-    shift2 += d * d;
+  double shift = 0.0;
+  if (o.criterion == NBSP_BH_OPENING_OFFSET) {
+    // the cell's centre from the first key's top 3 lvl bits, in the particles'
+    // frame (relative to the centre of mass)
+    const uint64_t key = o.keys[particle];
+    double shift2 = 0.0;
+    for (int a = 0; a < 3; ++a) {
+      const double lo = o.geometry[a] - half - o.geometry[4 + a];
+      const double centre = lo + ((double)(compact3(key >> a) >> (21 - l)) + 0.5) * side;
+      const double d = (a == 0 ? mo.cx : a == 1 ? mo.cy : mo.cz) - centre;
+      shift2 += d * d;
+    }
+    shift = sqrt(shift2);
   }
-  const double shift = sqrt(shift2);
   // Without previous accelerations every target's relative test passes (its
   // tolerance is +inf), so the geometric test alone decides: at the start
   // angle, not at the loose bound the relative test runs under.
@@ -979,17 +1069,20 @@ __device__ void finish_node(const Tree& t, int node, const Moments& mo, int firs
   const double r2 = o.criterion == NBSP_BH_OPENING_OFFSET
                         ? (side * it + shift) * (side * it + shift)
                         : side * side * it2;
-  t.ropen2[node] = (float)r2;
-  t.side[node] = (float)side;
-  t.shift[node] = (float)shift;
-  t.kmass[node] = (float)(mo.m * side * side);
-  t.wnode[2 * node] = make_float4((float)mo.cx, (float)mo.cy, (float)mo.cz, (float)mo.m);
-  t.wnode[2 * node + 1] = make_float4((float)r2, (float)(mo.m * side * side), __int_as_float(first),
-                                      __int_as_float(count));
+  const float4 a = make_float4((float)mo.cx, (float)mo.cy, (float)mo.cz, (float)mo.m);
+  const float4 b = make_float4((float)r2, (float)(mo.m * side * side), __int_as_float(first),
+                               __int_as_float(count));
+  t.wnode[2 * w] = a;
+  t.wnode[2 * w + 1] = b;
+  t.dnode[2 * dfs] = a;
+  t.dnode[2 * dfs + 1] = b;
   if (QUAD) {
-    t.spread[node] = mo.m > 0.0 ? (float)(mo.t2 / (mo.m * side * side)) : 0.f;
-    t.quad[2 * node] = make_float4((float)mo.q[0], (float)mo.q[1], (float)mo.q[2], (float)mo.q[3]);
-    t.quad[2 * node + 1] = make_float4((float)mo.q[4], 0.f, 0.f, 0.f);
+    for (int k = 0; k < 6; ++k) t.quad64[6 * w + k] = mo.q[k];
+    t.trace64[w] = mo.t2;
+    t.wquad[2 * w] = make_float4((float)mo.q[0], (float)mo.q[1], (float)mo.q[2], (float)mo.q[3]);
+    t.wquad[2 * w + 1] =
+        make_float4((float)mo.q[4], (float)side,
+                    mo.m > 0.0 ? (float)(mo.t2 / (mo.m * side * side)) : 0.f, (float)shift);
   }
 }
 
@@ -1010,27 +1103,32 @@ __device__ __forceinline__ int arrive_acq_rel(int* p) {
 }
 
 // Bottom-up moments: leaves sum their particles, the last child to finish
-// combines its parent.  place_kernel wrote each children list in depth-first
-// (= octant) order, so the combine's sums run in a fixed order and the result
-// is deterministic; it loads all the children at once.
+// combines its parent, whose children are consecutive and in Morton order, so
+// the combine's sums run in a fixed order and the result is deterministic.
 // QUAD: also the trace-free quadrupoles and the spread (the quadrupole walk,
 // the correction's features); the monopole walk reads neither.
-// Monopole pass at 6 blocks per SM (40 registers, a few spilled to L1): it is
-// bound by the latency of its loads and of the climb, and the extra warps hide
-// more of it (0.246 -> 0.228 ms at 10M); the quadrupole pass is left to the
-// compiler (its moments would spill hundreds of bytes per thread at 40 or 64)
+// Bound by the latency of the climb: per level one atomic, then the children's
+// moments.  The parent's link does not depend on the arrival, so it is loaded
+// beside the atomic (and the grandparent's beside the moments); with lists of
+// children and per-node arrays the climb waited for two more loads a level.
+// Monopole pass at 6 blocks per SM (40 registers, a few spilled to L1): the
+// extra warps hide more of it (0.246 -> 0.228 ms at 10M); the quadrupole pass
+// is left to the compiler (its moments would spill hundreds of bytes per thread
+// at 40 or 64)
 template <bool QUAD>
 __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4* __restrict__ pos, Tree t,
                                                       Opening open, int* status) {
   const int total = (int)t.offset[t.n];
   for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < total;
        node += gridDim.x * blockDim.x) {
-    const int4 info = t.info[node];
-    if (info.z == 0) continue;  // internal nodes are finished by their last child
-    if (info.z < 0 || info.y < 0 || info.y + info.z > t.n) {
+    const int4 info = t.link[node];
+    if (info.z < 0) continue;  // internal nodes are finished by their last child
+    if (info.z == 0 || info.y < 0 || info.y + info.z > t.n || info.w < 0 || info.w >= total) {
       atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
       continue;
     }
+    int parent = info.x;
+    int4 up = parent >= 0 && parent < total ? t.link[parent] : make_int4(-1, 0, 0, 0);
     Moments mo;
     {
       double m = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
@@ -1071,39 +1169,26 @@ __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4
         mo.q[5] += w * (3.0 * dz * dz - r2);
       }
     }
-    finish_node<QUAD>(t, node, mo, info.y, t.level[node], open, info.z);
-    int parent = info.w;
+    const int particle = info.y;
+    finish_node<QUAD>(t, node, mo, info.y, info.z, info.w, particle, t.level[node], open);
     for (int climb = 0; parent >= 0; ++climb) {
-      if (climb > 64 || parent >= total) {  // octree depth <= 23 levels
+      const int nc = -up.z, first = up.y;
+      if (climb > 64 || parent >= total || nc < 1 || nc > 8 || first < 1 ||
+          first + nc > total || up.w < 0 || up.w >= total) {  // octree depth <= 23 levels
         atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
         break;
       }
-      const int nc = __ldcg(&t.nchild[parent]);
-      const int arrived = arrive_acq_rel(&t.arrive[parent]);
-      if (arrived != nc - 1) break;
-      if (nc < 1 || nc > 8) {
-        atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-        break;
-      }
-      const int4 pinfo = __ldcg(&t.info[parent]);
-      const int4 ca = __ldcg(reinterpret_cast<const int4*>(t.children) + 2 * parent);
-      const int4 cb = __ldcg(reinterpret_cast<const int4*>(t.children) + 2 * parent + 1);
-      const int ch[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-      bool bad = false;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) bad |= k < nc && (ch[k] <= parent || ch[k] >= total);
-      if (bad) {
-        atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
-        break;
-      }
+      const int level = t.level[parent];
+      if (arrive_acq_rel(&t.arrive[parent]) != nc - 1) break;
+      const int4 next = up.x >= 0 && up.x < total ? t.link[up.x] : make_int4(-1, 0, 0, 0);
       double4 cm[8];
       int hmax = 0;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         cm[k] = make_double4(0.0, 0.0, 0.0, 0.0);
         if (k < nc) {
-          cm[k] = ldcg_d4(&t.mom[ch[k]]);
-          hmax = max(hmax, __ldcg(&t.height[ch[k]]));
+          cm[k] = ldcg_d4(&t.mom[first + k]);
+          hmax = max(hmax, __ldcg(&t.height[first + k]));
         }
       }
       double m = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
@@ -1126,7 +1211,7 @@ __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         if (QUAD && k < nc) {
-          const int c = ch[k];
+          const int c = first + k;
           const double dx = cm[k].y - pm.cx, dy = cm[k].z - pm.cy, dz = cm[k].w - pm.cz;
           const double r2 = dx * dx + dy * dy + dz * dz;
           const double w = cm[k].x;
@@ -1140,8 +1225,11 @@ __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4
         }
       }
       t.height[parent] = hmax + 1;
-      finish_node<QUAD>(t, parent, pm, pinfo.y, __ldcg(&t.level[parent]), open, -nc);
-      parent = pinfo.w;
+      // (the particle that names the cell's corner: any of the node's will do,
+      // its key's top bits are the cell's)
+      finish_node<QUAD>(t, parent, pm, first, -nc, up.w, particle, level, open);
+      parent = up.x;
+      up = next;
     }
   }
 }
@@ -1202,7 +1290,8 @@ __device__ __forceinline__ void stackless_walk(const float4* __restrict__ pos, i
       break;
     }
     const int4 info = t.info[node];
-    if (info.z < 0 || info.y < 0 || info.y + info.z > n || info.x <= node) {
+    if (info.z < 0 || info.y < 0 || info.y + info.z > n || info.x <= node || info.w < 0 ||
+        info.w >= total) {
       if (lane == 0) atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
       break;
     }
@@ -1210,11 +1299,10 @@ __device__ __forceinline__ void stackless_walk(const float4* __restrict__ pos, i
     // used when every lane's opening test passes (barnes_hut.c:596-599).
     bool direct = info.z == 1;
     if (info.z >= 2) {
-      const float4 c = t.com[node];
+      const float4 c = t.dnode[2 * node], o = t.dnode[2 * node + 1];
       const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
       const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      direct = __any_sync(kFull, active && !opening_passes<REL>(d2, t.ropen2[node],
-                                                               REL ? t.kmass[node] : 0.f, tol));
+      direct = __any_sync(kFull, active && !opening_passes<REL>(d2, o.x, o.y, tol));
     }
     if (direct) {
       const int j1 = info.y + info.z;
@@ -1232,11 +1320,10 @@ __device__ __forceinline__ void stackless_walk(const float4* __restrict__ pos, i
       pending += info.z;
       node = info.x;
     } else {
-      const float4 c = t.com[node];
+      const float4 c = t.dnode[2 * node], o = t.dnode[2 * node + 1];
       const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
       const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      const bool open =
-          active && !opening_passes<REL>(d2, t.ropen2[node], REL ? t.kmass[node] : 0.f, tol);
+      const bool open = active && !opening_passes<REL>(d2, o.x, o.y, tol);
       if (__any_sync(kFull, open)) {
         node = node + 1;
         continue;
@@ -1247,8 +1334,8 @@ __device__ __forceinline__ void stackless_walk(const float4* __restrict__ pos, i
       const float rinv3 = rinv * rinv2;
       float w = c.w * rinv3;
       if (ORDER == 2) {
-        const float4 qa = t.quad[2 * node];
-        const float qyz = t.quad[2 * node + 1].x;
+        const float4 qa = t.wquad[2 * info.w];
+        const float qyz = t.wquad[2 * info.w + 1].x;
         const float qzz = -qa.x - qa.w;
         // Q d and d.Q.d, d = com - target
         const float qdx = fmaf(qa.x, dx, fmaf(qa.y, dy, qa.z * dz));
@@ -1552,10 +1639,11 @@ __device__ __forceinline__ bool features_of(float4 c, float s, float4 qa, float 
   return true;
 }
 
-__device__ __forceinline__ bool cell_features(const Tree& t, int node, float4 c, float tx,
+// the same for the node of walk id w
+__device__ __forceinline__ bool cell_features(const Tree& t, int w, float4 c, float tx,
                                               float ty, float tz, float* f) {
-  return features_of(c, t.side[node], t.quad[2 * node], t.quad[2 * node + 1].x, t.spread[node],
-                     tx, ty, tz, f);
+  const float4 qb = t.wquad[2 * w + 1];
+  return features_of(c, qb.y, t.wquad[2 * w], qb.x, qb.z, tx, ty, tz, f);
 }
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
@@ -1623,11 +1711,12 @@ __global__ void mlp_pairs_kernel(const float4* __restrict__ pos, int n, Tree t, 
         node = info.x > node ? info.x : total;
         continue;
       }
-      const float4 c = t.com[node];
+      const float4 c = t.dnode[2 * node];
       const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
       const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      const float s = t.side[node];
-      const float ro = s / theta + t.shift[node];
+      const float4 qb = t.wquad[2 * info.w + 1];
+      const float s = qb.y;
+      const float ro = s / theta + qb.w;
       const bool pass = opening == NBSP_BH_OPENING_OFFSET ? d2 > ro * ro : s * s < th2 * d2;
       if (d2 > 0.f && pass && c.w > 0.f) {
         const float gdx = c.x - gx, gdy = c.y - gy, gdz = c.z - gz;
@@ -1701,9 +1790,9 @@ __global__ void mlp_labels_kernel(const float4* __restrict__ pos, int n, Tree t,
     az += __shfl_xor_sync(kFull, az, off);
   }
   if (lane != 0) return;
-  const float4 c = t.com[node];
+  const float4 c = t.dnode[2 * node];
   float f[nbsp_mlp::kIn];
-  if (!cell_features(t, node, c, p.x, p.y, p.z, f)) {
+  if (!cell_features(t, info.w, c, p.x, p.y, p.z, f)) {
     ok[k] = 0;
     return;
   }
@@ -1774,25 +1863,6 @@ __global__ void mlp_stats_kernel(const float* __restrict__ feat, const float* __
   }
 }
 
-// Particle index of slot f of the concatenated buckets: the last bucket e
-// with pref[e] <= f (pref: exclusive prefix of the counts, all counts >= 1).
-__device__ __forceinline__ int bucket_source(const int* pref, const int2* leaves, int nleaf,
-                                             int f) {
-  int lo = 0, hi = nleaf - 1;
-#pragma unroll
-  for (int it = 0; it < 6; ++it) {  // nleaf <= 64
-    const int mid = (lo + hi + 1) >> 1;
-    if (lo < hi) {
-      if (pref[mid] <= f) {
-        lo = mid;
-      } else {
-        hi = mid - 1;
-      }
-    }
-  }
-  return leaves[lo].x + (f - pref[lo]);
-}
-
 constexpr int kListThreads = 128;  // 4 warps, one traversal group each
 constexpr int kListCap = 64;       // cells / leaves gathered before a flush (>= 32 + 32)
 constexpr int kListStack = 1024;   // node ids per warp (4 KiB); overflow -> stackless walk
@@ -1825,8 +1895,8 @@ static_assert(kCtaStack + kFrontier <= 3 * kListStack, "frontier inside warp 2's
 // shared tile that every lane evaluates on its own target with paired f32x2
 // arithmetic whenever it is full.  Buckets that must be summed exactly are
 // listed (first particle, count); whenever 32 have gathered, their particles
-// are gathered into the same tile, one slot per lane located by binary search
-// over the counts' prefix sums, so all loads of a tile are in flight together.
+// are gathered into the same tile, one slot per lane and all loads of a tile in
+// flight together.
 // A quadrupole cell goes into a QuadTile with its moments when it is accepted.
 // A warp whose stack would overflow restarts with the stackless walk.
 //
@@ -1861,10 +1931,10 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
   __shared__ int s_stack[kListThreads / 32][STACK];
   __shared__ float s_probe_k[kListThreads / 32][REL ? 32 : 1];  // their M side^2
   // nodes awaiting per-target tests during a step; the same words hold the
-  // exclusive prefix of the bucket counts during a bucket flush (the two
-  // phases of an iteration never overlap: a __syncwarp ends each)
+  // buckets' particle offsets during a bucket flush (the two phases of an
+  // iteration never overlap: a __syncwarp ends each)
   __shared__ float4 s_probe[kListThreads / 32][32];
-  static_assert(sizeof(s_probe[0]) >= kListCap * sizeof(int), "prefix fits the probe words");
+  static_assert(sizeof(s_probe[0]) >= kListCap * sizeof(int), "offsets fit the probe words");
   __shared__ int2 s_leaves[kListThreads / 32][kListCap];  // (first particle, count)
   // ORDER 1: accepted cells are point masses in the source tile; ORDER 2:
   // cells fill a QuadTile
@@ -1979,13 +2049,7 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         all_open = all_open && (dmax2 <= ro || (REL && dmax2 * dmax2 * s_box[w][7] < km));
       }
       const bool to_front = ok && !all_accept && !all_open;
-      int4 ca = make_int4(-1, -1, -1, -1), cb = make_int4(-1, -1, -1, -1);
-      if (all_open) {
-        ca = reinterpret_cast<const int4*>(t.children)[2 * node];
-        cb = reinterpret_cast<const int4*>(t.children)[2 * node + 1];
-      }
-      const int kids = (ca.x >= 0) + (ca.y >= 0) + (ca.z >= 0) + (ca.w >= 0) + (cb.x >= 0) +
-                       (cb.y >= 0) + (cb.z >= 0) + (cb.w >= 0);
+      const int kids = all_open ? min(-info.z, 8) : 0;
       // block-wide exclusive prefixes of the three counts
       int ia = all_accept, ik = kids, ifr = to_front;
       for (int off = 1; off < 32; off <<= 1) {
@@ -2019,10 +2083,9 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       const int cbase = ctop - take, front0 = s_nfront;
       const bool abort = cbase + nk > kCtaStack || front0 + nf > kFrontier;  // block-uniform
       if (!abort) {
-        const int kid[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          if (k < kids) cstack[cbase + rk + k] = kid[k];
+          if (k < kids) cstack[cbase + rk + k] = info.y + k;
         if (to_front) front[front0 + rf] = node;
         // cells every group accepts: into every live warp's source tile, in
         // rounds of what fits before the tiles are evaluated
@@ -2091,7 +2154,6 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       int4 info = make_int4(0, 0, 0, 0);
       float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
       float ro = 0.f, km = 0.f;
-      int4 ca = make_int4(-1, -1, -1, -1), cb = make_int4(-1, -1, -1, -1);
       if (node >= total) {
         atomicOr(status, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
         node = -1;
@@ -2099,8 +2161,8 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       {  // every lane loads a node (idle lanes the root) so no branch diverges
         const bool valid = node >= 0;
         const int at = valid ? node : 0;
-        // one 32-byte record: the centre of mass and mass, the opening terms
-        // and the particle range (the node's next and parent links are not read)
+        // one 32-byte record: the centre of mass and mass, the opening terms,
+        // and a bucket's particles or an internal node's children
         const float4 w0 = __ldg(&t.wnode[2 * at]), w1 = __ldg(&t.wnode[2 * at + 1]);
         c = w0;
         ro = w1.x;
@@ -2141,24 +2203,10 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       }
       const bool open = (test || opened) && !accept;
       is_leaf = is_leaf || (open && info.z > 0);  // a failing bucket is summed exactly
-      if (open && info.z < 0) {                    // an opened cell pushes its -info.z children
-        ca = __ldg(reinterpret_cast<const int4*>(t.children) + 2 * node);
-        cb = __ldg(reinterpret_cast<const int4*>(t.children) + 2 * node + 1);
-        kids = min(-info.z, 8);
-      }
+      if (open && info.z < 0) kids = min(-info.z, 8);  // an opened cell pushes its children
       unsigned m = __ballot_sync(kFull, is_leaf);
       if (is_leaf) leaves[nleaf + __popc(m & lt)] = make_int2(info.y, info.z);
       nleaf += __popc(m);
-      {  // targets whose own particle is in one of these buckets: one term fewer
-        // (only the group's own buckets overlap its targets: a vote first)
-        const int lo = max(info.y - warp * 32, 0), hi = min(info.y + info.z - warp * 32, 32);
-        if (__any_sync(kFull, is_leaf && hi > lo)) {
-          const unsigned span = hi >= 32 ? kFull : (1u << max(hi, 0)) - 1u;
-          const unsigned own = __reduce_or_sync(
-              kFull, is_leaf && hi > lo ? span & ~((1u << min(lo, 31)) - 1u) : 0u);
-          if (active && ((own >> lane) & 1u)) exact -= 1u;
-        }
-      }
       m = __ballot_sync(kFull, accept);
       if (ORDER == 1) {
         // A monopole cell is a point mass at its centre of mass, already in
@@ -2168,7 +2216,7 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         if (CORR) {
           bool listme = false;
           if (accept) {
-            const float side = t.side[node];
+            const float side = t.wquad[2 * node + 1].y;
             const float gdx = c.x - gx, gdy = c.y - gy, gdz = c.z - gz;
             const float dg2 = fmaf(gdx, gdx, fmaf(gdy, gdy, gdz * gdz));
             const float lo = __ldg(&net->x_min[3]), hi = __ldg(&net->x_max[3]);
@@ -2197,8 +2245,8 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         float4 qa = make_float4(0.f, 0.f, 0.f, 0.f);
         float qyz = 0.f;
         if (accept) {
-          qa = t.quad[2 * node];
-          qyz = t.quad[2 * node + 1].x;
+          qa = t.wquad[2 * node];
+          qyz = t.wquad[2 * node + 1].x;
         }
         const int nacc = __popc(m), rank = __popc(m & lt), room = kStage - qstaged;
         if (accept && rank < room) stage_cell(qt, qstaged + rank, c, qa, qyz);
@@ -2224,23 +2272,25 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         break;
       }
       const int base = top + incl - kids;
-      const int kid[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        if (k < kids) stack[base + k] = kid[k];
+        if (k < kids) stack[base + k] = info.y + k;
       top += pushed;
       __syncwarp();
     }
     const bool drain = top == 0;
     if (nleaf >= 32 || (drain && nleaf > 0)) {
-      // The buckets' particles, concatenated, fill the tile: each lane finds
-      // the bucket of its slot by binary search over the exclusive prefix of
-      // the counts and loads its particles, all loads of a tile in flight at
-      // once.  The target's own particle adds exactly 0 (d = 0).
-      int* pref = reinterpret_cast<int*>(s_probe[wib]);
-      const int c0 = lane < nleaf ? leaves[lane].y : 0;
-      const int c1 = lane + 32 < nleaf ? leaves[lane + 32].y : 0;
-      int i0 = c0, i1 = c1;
+      // The buckets' particles, concatenated, fill the tile, all loads of a tile
+      // in flight at once.  A slot's bucket is the number of buckets that start
+      // at or before it: those before the tile's first slot, plus the bits up to
+      // it in the mask of the starts inside the tile (two words, one OR-reduction
+      // each; a binary search over the counts' prefix took three times the
+      // instructions and six dependent shared-memory loads).  The target's own
+      // particle adds exactly 0 (d = 0).
+      int* shift = reinterpret_cast<int*>(s_probe[wib]);  // first particle - first slot
+      const int2 l0 = lane < nleaf ? leaves[lane] : make_int2(0, 0);
+      const int2 l1 = lane + 32 < nleaf ? leaves[lane + 32] : make_int2(0, 0);
+      int i0 = l0.y, i1 = l1.y;
       for (int off = 1; off < 32; off <<= 1) {
         const int v0 = __shfl_up_sync(kFull, i0, off), v1 = __shfl_up_sync(kFull, i1, off);
         if (lane >= off) {
@@ -2250,16 +2300,38 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       }
       i1 += __shfl_sync(kFull, i0, 31);
       const int total_src = __shfl_sync(kFull, i1, 31);
-      if (lane < nleaf) pref[lane] = i0 - c0;
-      if (lane + 32 < nleaf) pref[lane + 32] = i1 - c1;
+      // first slot of each of this lane's buckets (none: past every slot)
+      const int b0 = lane < nleaf ? i0 - l0.y : INT_MAX, b1 = lane + 32 < nleaf ? i1 - l1.y : INT_MAX;
+      if (lane < nleaf) shift[lane] = l0.x - b0;
+      if (lane + 32 < nleaf) shift[lane + 32] = l1.x - b1;
+      {  // targets whose own particle is in one of these buckets: one term fewer
+        // (only the group's own buckets overlap its targets: a vote first)
+        const int g0 = warp * 32;
+        const int lo0 = max(l0.x - g0, 0), hi0 = min(l0.x + l0.y - g0, 32);
+        const int lo1 = max(l1.x - g0, 0), hi1 = min(l1.x + l1.y - g0, 32);
+        if (__any_sync(kFull, hi0 > lo0 || hi1 > lo1)) {
+          unsigned own = 0u;
+          if (hi0 > lo0) own |= (hi0 >= 32 ? kFull : (1u << hi0) - 1u) & ~((1u << lo0) - 1u);
+          if (hi1 > lo1) own |= (hi1 >= 32 ? kFull : (1u << hi1) - 1u) & ~((1u << lo1) - 1u);
+          own = __reduce_or_sync(kFull, own);
+          if (active && ((own >> lane) & 1u)) exact -= 1u;
+        }
+      }
       __syncwarp();
       exact += active ? (unsigned)total_src : 0u;  // own particles were taken off above
+      const unsigned le = 2u * lt + 1u;  // this lane's bit and those below
       for (int f0 = 0; f0 < total_src;) {
         const int take = min(total_src - f0, kStage - staged);
         const bool h0 = lane < take, h1 = lane + 32 < take;
+        const unsigned r0 = (unsigned)(b0 - f0), r1 = (unsigned)(b1 - f0);
+        const unsigned m0 = __reduce_or_sync(
+            kFull, (r0 < 32u ? 1u << r0 : 0u) | (r1 < 32u ? 1u << r1 : 0u));
+        const unsigned m1 = __reduce_or_sync(
+            kFull, (r0 - 32u < 32u ? 1u << (r0 - 32u) : 0u) | (r1 - 32u < 32u ? 1u << (r1 - 32u) : 0u));
+        const int before = __popc(__ballot_sync(kFull, b0 < f0)) + __popc(__ballot_sync(kFull, b1 < f0)) - 1;
         float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
-        if (h0) q0 = pos[bucket_source(pref, leaves, nleaf, f0 + lane)];
-        if (h1) q1 = pos[bucket_source(pref, leaves, nleaf, f0 + lane + 32)];
+        if (h0) q0 = pos[shift[before + __popc(m0 & le)] + f0 + lane];
+        if (h1) q1 = pos[shift[before + __popc(m0) + __popc(m1 & le)] + f0 + lane + 32];
         if (h0) stage_source(src, staged + lane, q0);
         if (h1) stage_source(src, staged + lane + 32, q1);
         staged += take;
@@ -2391,12 +2463,13 @@ __device__ __forceinline__ RowData load_row(const Tree& t, const float4* centre,
   RowData d;
   d.valid = valid;
   const int node = valid ? gn.y : 0, grp = valid ? gn.x : 0;
-  d.c = t.com[node];
+  d.c = t.wnode[2 * node];
   d.g = centre[grp];
-  d.qa = t.quad[2 * node];
-  d.qyz = t.quad[2 * node + 1].x;
-  d.side = t.side[node];
-  d.spread = t.spread[node];
+  d.qa = t.wquad[2 * node];
+  const float4 qb = t.wquad[2 * node + 1];
+  d.qyz = qb.x;
+  d.side = qb.y;
+  d.spread = qb.z;
   return d;
 }
 
@@ -2469,7 +2542,7 @@ __global__ void __launch_bounds__(128) corr_apply_kernel(const float4* __restric
     float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
     float yx = 0.f, yy = 0.f, yz = 0.f;
     if (k < cnt) {
-      c = t.com[lists.cells[(size_t)g * lists.capacity + k]];
+      c = t.wnode[2 * lists.cells[(size_t)g * lists.capacity + k]];
       const float* y = &lists.y[(size_t)(off + k) * 3];
       yx = c.w * y[0];
       yy = c.w * y[1];
@@ -2637,20 +2710,21 @@ void nbsp_bh_build(const uint64_t* keys, size_t n, int leaf_capacity, void* tree
                    cudaStream_t stream) {
   Tree t = tree_view(tree, n);
   cudaMemsetAsync(t.mask, 0, n * sizeof(uint32_t), stream);
-  cudaMemsetAsync(t.leaves, 0, sizeof(unsigned long long), stream);
+  cudaMemsetAsync(t.leaves, 0, 2 * sizeof(unsigned long long), stream);
   if (n >= 2)
     NBSP_COUNT_LAUNCH(1), radix_tree_kernel<<<(unsigned)((n - 1 + 255) / 256), 256, 0, stream>>>(keys, t, status);
-  // keep and place: one thread per internal binary node (n >= 2: the caller
-  // handles a lone particle without a tree)
-  const unsigned internal_blocks = (unsigned)((n - 1 + 255) / 256);
-  if (internal_blocks > 0)
-    NBSP_COUNT_LAUNCH(1), keep_kernel<<<internal_blocks, 256, 0, stream>>>(t, leaf_capacity, status);
+  // (n >= 2: the caller handles a lone particle without a tree)
+  const unsigned keep_blocks = (unsigned)((n - 1 + kKeepNodes - 1) / kKeepNodes);
+  if (keep_blocks > 0)
+    NBSP_COUNT_LAUNCH(1), keep_kernel<<<keep_blocks, kKeepThreads, 0, stream>>>(t, leaf_capacity, status);
   const int blocks = (int)((n + kScanItems - 1) / kScanItems);
   NBSP_COUNT_LAUNCH(1), scan_reduce_kernel<<<blocks, 256, 0, stream>>>(t);
   NBSP_COUNT_LAUNCH(1), scan_blocks_kernel<<<1, 1024, 0, stream>>>(t, blocks);
   NBSP_COUNT_LAUNCH(1), scan_apply_kernel<<<blocks, 256, 0, stream>>>(t);
-  if (internal_blocks > 0)
-    NBSP_COUNT_LAUNCH(1), place_kernel<<<internal_blocks, 256, 0, stream>>>(t, leaf_capacity, status);
+  // (at most a splitting cell per two particles: eight threads each)
+  const size_t place_blocks = (4 * n + 255) / 256;
+  NBSP_COUNT_LAUNCH(1), place_kernel<<<(unsigned)(place_blocks < kPlaceBlocks ? place_blocks : kPlaceBlocks), 256, 0, stream>>>(
+      t, leaf_capacity, status);
 }
 
 void nbsp_bh_moments(const void* pos4, const uint64_t* keys, size_t n, const double* geometry,
