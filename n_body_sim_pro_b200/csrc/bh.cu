@@ -40,21 +40,23 @@ constexpr int kBoundsThreads = 256;
 constexpr int kBoundsBlocks = 4 * 148;  // one wave at 4 blocks of 256 per SM (58 registers)
 constexpr int kBoundsVals = 11;  // min xyz, max xyz, m, mx, my, mz, |a|^2
 
-// The block's combined values in thread 0: each warp by shuffles, then the
-// warps' results by the first warp.
+// The combined values of the block's first kBoundsThreads threads in thread 0:
+// each warp by shuffles, then the warps' results by the first warp.
 __device__ __forceinline__ void bounds_block_reduce(double (&v)[kBoundsVals],
                                                     double (*sh)[kBoundsThreads / 32]) {
-  for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-    for (int q = 0; q < kBoundsVals; ++q) {
-      const double o = __shfl_xor_sync(0xffffffffu, v[q], off);
-      v[q] = q < 3 ? fmin(v[q], o) : q < 6 ? fmax(v[q], o) : v[q] + o;
-    }
-  }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0)
+  if (w < kBoundsThreads / 32) {
+    for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
-    for (int q = 0; q < kBoundsVals; ++q) sh[q][w] = v[q];
+      for (int q = 0; q < kBoundsVals; ++q) {
+        const double o = __shfl_xor_sync(0xffffffffu, v[q], off);
+        v[q] = q < 3 ? fmin(v[q], o) : q < 6 ? fmax(v[q], o) : v[q] + o;
+      }
+    }
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < kBoundsVals; ++q) sh[q][w] = v[q];
+  }
   __syncthreads();
   if (w != 0) return;
 #pragma unroll
@@ -124,17 +126,20 @@ __global__ void __launch_bounds__(kBoundsThreads) bounds_kernel(
     for (int q = 0; q < kBoundsVals; ++q) partial[blockIdx.x * kBoundsVals + q] = v[q];
 }
 
-// Root cube with the exact FP64 operation sequence of barnes_hut.c:471-483.
-__global__ void __launch_bounds__(kBoundsThreads) bounds_final_kernel(
-    const double* __restrict__ partial, int blocks, size_t n, double* __restrict__ geometry) {
-  __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
+// The blocks' partial results combined by a block's first kBoundsThreads threads
+// (the others only join the barrier), and in thread 0 the root cube with the
+// exact FP64 operation sequence of barnes_hut.c:471-483.
+__device__ __forceinline__ void root_geometry(const double* __restrict__ partial, int blocks,
+                                              size_t n, double (*sh)[kBoundsThreads / 32],
+                                              double* geometry) {
   double v[kBoundsVals] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY,
                            0.0,      0.0,      0.0,      0.0,       0.0};
-  for (int b = threadIdx.x; b < blocks; b += kBoundsThreads) {
-    for (int q = 0; q < 3; ++q) v[q] = fmin(v[q], partial[b * kBoundsVals + q]);
-    for (int q = 3; q < 6; ++q) v[q] = fmax(v[q], partial[b * kBoundsVals + q]);
-    for (int q = 6; q < kBoundsVals; ++q) v[q] += partial[b * kBoundsVals + q];
-  }
+  if (threadIdx.x < kBoundsThreads)
+    for (int b = threadIdx.x; b < blocks; b += kBoundsThreads) {
+      for (int q = 0; q < 3; ++q) v[q] = fmin(v[q], partial[b * kBoundsVals + q]);
+      for (int q = 3; q < 6; ++q) v[q] = fmax(v[q], partial[b * kBoundsVals + q]);
+      for (int q = 6; q < kBoundsVals; ++q) v[q] += partial[b * kBoundsVals + q];
+    }
   bounds_block_reduce(v, sh);
   if (threadIdx.x == 0) {
     const double lo[3] = {v[0], v[1], v[2]};
@@ -152,6 +157,12 @@ __global__ void __launch_bounds__(kBoundsThreads) bounds_final_kernel(
     for (int k = 0; k < 3; ++k) geometry[4 + k] = mt != 0.0 ? v[7 + k] / mt : 0.0;
     geometry[7] = n > 0 ? sqrt(v[10] / (double)n) : 0.0;  // rms |a| (when given)
   }
+}
+
+__global__ void __launch_bounds__(kBoundsThreads) bounds_final_kernel(
+    const double* __restrict__ partial, int blocks, size_t n, double* __restrict__ geometry) {
+  __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
+  root_geometry(partial, blocks, n, sh, geometry);
 }
 
 // ---------------------------------------------------------------------------
@@ -193,40 +204,71 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v) {
 // runs out.
 // ---------------------------------------------------------------------------
 
-// 512 threads of 8 keys: twice the warps of 256 x 16 at the same tile (the
-// ranking chain per warp is half as long); at 10M keys 0.92 ms for the 8
-// passes against 1.10 with 256 x 16 (and 1.17 with 1024 x 4, one block per SM)
-constexpr int kSortThreads = 512;
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096
+// A tile is THREADS x ITEMS keys.  Large systems: 512 threads of 8 keys (at 10M
+// keys 0.92 ms for the 8 passes against 1.10 with 256 x 16, whose ranking chain
+// per warp is twice as long, and 1.17 with 1024 x 4, one block per SM).  Below
+// kSortWide keys those tiles leave SMs idle and a pass is one tile's chain of
+// load, rank, look back and scatter: 512 threads of 4 keys take 78 us for the 8
+// passes at 100k-150k and 91 at 262k (wide tiles: 97 and 109; 256 x 4: 79 and
+// 95), the same as wide tiles at 500k and more beyond (1M: 185 against 154).
+struct SortWide {
+  static constexpr int kThreads = 512, kItems = 8, kBlocks = 2;
+};
+struct SortNarrow {
+  static constexpr int kThreads = 512, kItems = 4, kBlocks = 2;
+};
+constexpr size_t kSortWide = 450000;
 constexpr int kRadix = 256;
 constexpr int kLookback = 8;  // predecessors' flags read at once in the look-back
-static_assert(kSortThreads >= kRadix, "one thread per digit");
+template <class S>
+constexpr int sort_tile() {
+  static_assert(S::kThreads >= kRadix, "one thread per digit");
+  return S::kThreads * S::kItems;
+}
 constexpr int kSortPasses = 8;
 constexpr uint32_t kFlagA = 1u << 30, kFlagP = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr int kLookbackSpins = 1 << 22;  // ~ms per predecessor before the error flag
 constexpr int kKeysBlocks = 5 * 148;  // 40 warps per SM (48 registers): enough loads in flight
 
-// Sort scratch (32-bit words): hist[8][256] | base[8][256] | ticket[8] | status[8][tiles][256]
+// Sort scratch (32-bit words): hist[8][256] | ticket[8] | status[8][tiles][256]
 struct SortScratch {
   uint32_t* hist;
-  uint32_t* base;
   uint32_t* ticket;
   uint32_t* status;
 };
-__host__ __device__ inline size_t sort_tiles(size_t n) { return (n + kSortTile - 1) / kSortTile; }
-inline SortScratch sort_scratch(uint32_t* w, size_t n) {
+inline size_t sort_tiles(size_t n) {
+  const size_t tile = n < kSortWide ? sort_tile<SortNarrow>() : sort_tile<SortWide>();
+  return (n + tile - 1) / tile;
+}
+inline SortScratch sort_scratch(uint32_t* w) {
   SortScratch s;
   s.hist = w;
-  s.base = w + kSortPasses * kRadix;
-  s.ticket = s.base + kSortPasses * kRadix;
+  s.ticket = w + kSortPasses * kRadix;
   s.status = s.ticket + kSortPasses;
-  (void)n;
   return s;
 }
 inline size_t sort_scratch_words(size_t n) {
-  return 2 * kSortPasses * kRadix + kSortPasses + kSortPasses * sort_tiles(n) * kRadix;
+  return kSortPasses * kRadix + kSortPasses + kSortPasses * sort_tiles(n) * kRadix;
+}
+
+// Particle i's Morton key under root cube `geometry`, and its record for the
+// walk, still in input order: the float4 (relative to the centre of mass) and
+// with `unsorted_tol` the relative opening test's alpha max(|a_old|, rms) / G.
+__device__ __forceinline__ uint64_t particle_key(
+    size_t i, const double* __restrict__ x, const double* __restrict__ y,
+    const double* __restrict__ z, const double* __restrict__ m, const double (&geometry)[8],
+    const double* __restrict__ ax, const double* __restrict__ ay, const double* __restrict__ az,
+    double tol_scale, float4* __restrict__ unsorted, float* __restrict__ unsorted_tol) {
+  const double xi = x[i], yi = y[i], zi = z[i];
+  unsorted[i] = make_float4((float)__dsub_rn(xi, geometry[4]), (float)__dsub_rn(yi, geometry[5]),
+                            (float)__dsub_rn(zi, geometry[6]), (float)m[i]);
+  if (unsorted_tol != nullptr) {
+    const double a = fmax(sqrt(ax[i] * ax[i] + ay[i] * ay[i] + az[i] * az[i]), geometry[7]);
+    unsorted_tol[i] = a > 0.0 && isfinite(a) ? (float)(tol_scale * a) : INFINITY;
+  }
+  return spread3(axis_code(xi, geometry[0], geometry[3])) |
+         (spread3(axis_code(yi, geometry[1], geometry[3])) << 1) |
+         (spread3(axis_code(zi, geometry[2], geometry[3])) << 2);
 }
 
 __global__ void __launch_bounds__(256) keys_kernel(
@@ -238,9 +280,9 @@ __global__ void __launch_bounds__(256) keys_kernel(
   __shared__ uint32_t h[kSortPasses][kRadix];
   for (int k = threadIdx.x; k < kSortPasses * kRadix; k += blockDim.x) (&h[0][0])[k] = 0;
   __syncthreads();
-  const double cx = geometry[0], cy = geometry[1], cz = geometry[2], hs = geometry[3];
-  const double mx = geometry[4], my = geometry[5], mz = geometry[6];  // centre of mass
-  const double a_floor = geometry[7];  // rms |a_old|: the relative test's floor
+  double geo[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) geo[k] = geometry[k];
   const unsigned lane = threadIdx.x & 31;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -251,19 +293,9 @@ __global__ void __launch_bounds__(256) keys_kernel(
     const bool valid = i < n;
     uint64_t key = 0;
     if (valid) {
-      const double xi = x[i], yi = y[i], zi = z[i];
-      key = spread3(axis_code(xi, cx, hs)) | (spread3(axis_code(yi, cy, hs)) << 1) |
-            (spread3(axis_code(zi, cz, hs)) << 2);
+      key = particle_key(i, x, y, z, m, geo, ax, ay, az, tol_scale, unsorted, unsorted_tol);
       keys[i] = key;
       index[i] = (uint32_t)i;
-      // the walk's float4 (relative to the centre of mass), still in input
-      // order: the gather then moves one 16-byte record per particle
-      unsorted[i] = make_float4((float)__dsub_rn(xi, mx), (float)__dsub_rn(yi, my),
-                                (float)__dsub_rn(zi, mz), (float)m[i]);
-      if (unsorted_tol != nullptr) {  // relative opening test: alpha max(|a_old|, rms) / G
-        const double a = fmax(sqrt(ax[i] * ax[i] + ay[i] * ay[i] + az[i] * az[i]), a_floor);
-        unsorted_tol[i] = a > 0.0 && isfinite(a) ? (float)(tol_scale * a) : INFINITY;
-      }
     }
 #pragma unroll
     // digit counts: the low six bytes of the keys of one warp are spread over
@@ -286,35 +318,19 @@ __global__ void __launch_bounds__(256) keys_kernel(
   }
 }
 
-// One block of 256 threads: base[p][d] = number of keys whose digit p is < d.
-__global__ void __launch_bounds__(kRadix) sort_bases_kernel(const uint32_t* __restrict__ hist,
-                                                            uint32_t* __restrict__ base) {
-  __shared__ uint32_t sh[kRadix];
-  const int d = threadIdx.x;
-  for (int p = 0; p < kSortPasses; ++p) {
-    const uint32_t own = hist[p * kRadix + d];
-    uint32_t v = own;
-    sh[d] = v;
-    for (int off = 1; off < kRadix; off <<= 1) {
-      __syncthreads();
-      const uint32_t add = d >= off ? sh[d - off] : 0u;
-      __syncthreads();
-      v += add;
-      sh[d] = v;
-    }
-    base[p * kRadix + d] = v - own;
-    __syncthreads();
-  }
-}
-
 __device__ __forceinline__ uint32_t load_volatile(const uint32_t* p) {
   return *reinterpret_cast<const volatile uint32_t*>(p);
 }
 
-__global__ void __launch_bounds__(kSortThreads, 2) sort_pass_kernel(
+// hist: the pass's digit counts over all keys; every tile scans them for the
+// digits' first places (a launch of its own took 6 us).
+template <class S>
+__global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n, int shift,
-    const uint32_t* __restrict__ base, uint32_t* ticket, uint32_t* status, int* err) {
+    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* status, int* err) {
+  constexpr int kSortThreads = S::kThreads, kSortItems = S::kItems;
+  constexpr int kSortWarps = kSortThreads / 32, kSortTile = sort_tile<S>();
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t* sk = reinterpret_cast<uint64_t*>(smem);                     // kSortTile
   uint32_t* sv = reinterpret_cast<uint32_t*>(sk + kSortTile);           // kSortTile
@@ -322,9 +338,21 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_pass_kernel(
   uint32_t* start = wc + kSortWarps * kRadix;                           // 256
   uint32_t* gofs = start + kRadix;                                      // 256
   __shared__ int s_tile;
+  __shared__ uint32_t s_hsum[kRadix / 32];
 
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
   if (t == 0) s_tile = (int)atomicAdd(ticket, 1u);
+  uint32_t digit_base = 0;  // threads t < 256: keys of smaller digits
+  if (t < kRadix) {
+    const uint32_t own = hist[t];
+    uint32_t x = own;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t u = __shfl_up_sync(kFull, x, off);
+      if (lane >= off) x += u;
+    }
+    if (lane == 31) s_hsum[w] = x;
+    digit_base = x - own;
+  }
   for (int k = t; k < kSortWarps * kRadix; k += kSortThreads) wc[k] = 0;
   __syncthreads();
   const int tile = s_tile;
@@ -397,7 +425,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_pass_kernel(
       }
       atomicExch(st, kFlagP | ((prefix + count) & kCountMask));
     }
-    gofs[t] = base[t] + prefix;
+    for (int k = 0; k < w; ++k) digit_base += s_hsum[k];
+    gofs[t] = digit_base + prefix;
     uint32_t x = count;
     for (int off = 1; off < 32; off <<= 1) {
       const uint32_t u = __shfl_up_sync(kFull, x, off);
@@ -443,9 +472,137 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_pass_kernel(
   }
 }
 
-constexpr size_t kDownsweepSmem =
-    (size_t)kSortTile * (sizeof(uint64_t) + sizeof(uint32_t)) +
-    (size_t)(kSortWarps * kRadix + 2 * kRadix) * sizeof(uint32_t);
+template <class S>
+constexpr size_t sort_pass_smem() {
+  return (size_t)sort_tile<S>() * (sizeof(uint64_t) + sizeof(uint32_t)) +
+         (size_t)(S::kThreads / 32 * kRadix + 2 * kRadix) * sizeof(uint32_t);
+}
+
+// ---------------------------------------------------------------------------
+// the same sort for up to NBSP_BH_SMALL_SORT keys: two kernels
+//
+// Eight passes of the radix sort are eight chains of load, rank, look back and
+// scatter on a few tiles, about 10 us each however few keys there are.  Here
+// every CTA computes the keys of one tile of 1024 particles (and first, from the
+// bounds' partial results, the root cube) and sorts them in a bitonic network,
+// by (key, index), so that equal keys keep their order; then each key finds its
+// place by its rank among every other tile's keys, and the walk's records are
+// written there directly (no gather pass).  The ranks cost n / 1024 binary
+// searches per key, the radix passes none.  Sort and gather, small against
+// radix: 10 against 91 us at 10k, 11 against 88 at 20k, 35 against 95 at 65k, 70
+// against 82 at 100k, 132 against 82 at 150k: the line is where the two meet.
+// ---------------------------------------------------------------------------
+
+constexpr int kSmallTile = 1024;
+
+__global__ void __launch_bounds__(kSmallTile) small_keys_kernel(
+    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+    const double* __restrict__ m, size_t n, const double* __restrict__ partial, int blocks,
+    double* __restrict__ geometry, uint64_t* __restrict__ keys, uint32_t* __restrict__ index,
+    float4* __restrict__ unsorted, const double* __restrict__ ax, const double* __restrict__ ay,
+    const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol) {
+  __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
+  __shared__ double s_geo[8];
+  __shared__ uint64_t sk[kSmallTile];
+  __shared__ uint32_t sv[kSmallTile];
+  const int t = threadIdx.x;
+  root_geometry(partial, blocks, n, sh, s_geo);
+  __syncthreads();
+  double geo[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) geo[k] = s_geo[k];
+  if (blockIdx.x == 0 && t < 8) geometry[t] = s_geo[t];
+  const size_t i = (size_t)blockIdx.x * kSmallTile + t;
+  uint64_t key = ~0ull;  // past the end: behind every 63-bit key
+  if (i < n)
+    key = particle_key(i, x, y, z, m, geo, ax, ay, az, tol_scale, unsorted, unsorted_tol);
+  uint32_t val = (uint32_t)t;
+  for (int k = 2; k <= kSmallTile; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      uint64_t pk;
+      uint32_t pv;
+      if (j >= 32) {
+        __syncthreads();
+        sk[t] = key;
+        sv[t] = val;
+        __syncthreads();
+        pk = sk[t ^ j];
+        pv = sv[t ^ j];
+      } else {
+        pk = __shfl_xor_sync(kFull, (unsigned long long)key, j);
+        pv = __shfl_xor_sync(kFull, val, j);
+      }
+      const bool less = pk < key || (pk == key && pv < val);  // the partner belongs first
+      const bool first = ((t & j) == 0) == ((t & k) == 0);    // this slot takes the smaller
+      if (less == first) {
+        key = pk;
+        val = pv;
+      }
+    }
+  }
+  if (i < n) {
+    keys[i] = key;
+    index[i] = blockIdx.x * kSmallTile + val;
+  }
+}
+
+// 32 consecutive keys of one sorted tile per block; warp w ranks them among
+// tiles w, w + 8, ... (a warp's keys are neighbours, so its searches of a tile
+// run through nearly the same words), two tiles at a time.
+constexpr int kMergeWarps = 8;
+__global__ void __launch_bounds__(32 * kMergeWarps) small_merge_kernel(
+    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, int n,
+    uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+    const float4* __restrict__ unsorted, float4* __restrict__ pos,
+    const float* __restrict__ unsorted_tol, float* __restrict__ tol, int* err) {
+  __shared__ int s_rank[kMergeWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int s = blockIdx.x * 32 + lane;
+  const bool valid = s < n;
+  const uint64_t key = keys_in[valid ? s : n - 1];
+  const uint32_t i = w == 0 && valid ? vals_in[s] : 0u;
+  float4 record = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (w == 0 && valid && i < (uint32_t)n) record = unsorted[i];
+  const int tile = blockIdx.x * 32 / kSmallTile, tiles = (n + kSmallTile - 1) / kSmallTile;
+  int rank = 0;
+  for (int t0 = w; t0 < tiles; t0 += 2 * kMergeWarps) {
+    // keys of an earlier tile go before this one when not greater, keys of a
+    // later tile when smaller
+    int count[2], len[2];
+    uint64_t below[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int u = t0 + q * kMergeWarps;
+      count[q] = 0;
+      len[q] = u < tiles && u != tile ? min(kSmallTile, n - u * kSmallTile) : 0;
+      below[q] = key + (u < tile ? 1u : 0u);
+    }
+    const uint64_t* k0 = keys_in + (size_t)t0 * kSmallTile - 1;
+#pragma unroll
+    for (int step = kSmallTile; step > 0; step >>= 1) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int p = count[q] + step;
+        if (p <= len[q] && k0[q * kMergeWarps * kSmallTile + p] < below[q]) count[q] = p;
+      }
+    }
+    rank += count[0] + count[1];
+  }
+  s_rank[w][lane] = rank;
+  __syncthreads();
+  if (w != 0 || !valid) return;
+  rank = s % kSmallTile;
+#pragma unroll
+  for (int q = 0; q < kMergeWarps; ++q) rank += s_rank[q][lane];
+  if (rank >= n || i >= (uint32_t)n) {
+    atomicOr(err, NBSP_DEVICE_ERROR_TREE_INCONSISTENT);
+    return;
+  }
+  keys_out[rank] = key;
+  vals_out[rank] = i;
+  pos[rank] = record;
+  if (tol != nullptr) tol[rank] = unsorted_tol[i];
+}
 
 // The reference's insertion build fails with OVERFLOW when two particles share
 // a position (barnes_hut.c:149-153: more than 128 subdivisions).  Equal
@@ -2593,6 +2750,11 @@ int grid_for(size_t n, int threads) {
   return (int)b;
 }
 
+int bounds_blocks(size_t n) {
+  const size_t blocks = (n + kBoundsThreads - 1) / kBoundsThreads;
+  return blocks < 1 ? 1 : blocks > (size_t)kBoundsBlocks ? kBoundsBlocks : (int)blocks;
+}
+
 template <bool REL>
 void launch_walk(const float4* p, const float* tol, size_t n, Tree t, int order, int mode,
                  const nbsp_mlp::Net* net, const NbspCorrectionLists* lists, float eps2,
@@ -2635,30 +2797,54 @@ void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n, 
                     double* geometry, int* status, const double* ax, const double* ay,
                     const double* az, int rms_of_a, const NbspLeapfrogFusion* leapfrog,
                     cudaStream_t stream) {
-  size_t blocks = (n + kBoundsThreads - 1) / kBoundsThreads;
-  if (blocks < 1) blocks = 1;
-  if (blocks > (size_t)kBoundsBlocks) blocks = kBoundsBlocks;
+  const int blocks = bounds_blocks(n);
   if (leapfrog != nullptr && leapfrog->vx != nullptr) {
-    NBSP_COUNT_LAUNCH(1), bounds_kernel<true><<<(unsigned)blocks, kBoundsThreads, 0, stream>>>(
+    NBSP_COUNT_LAUNCH(1), bounds_kernel<true><<<blocks, kBoundsThreads, 0, stream>>>(
         x, y, z, m, n, partial, status, ax, ay, az, rms_of_a != 0, leapfrog->vx, leapfrog->vy,
         leapfrog->vz, leapfrog->half_dt, leapfrog->dt);
   } else {
-    NBSP_COUNT_LAUNCH(1), bounds_kernel<false><<<(unsigned)blocks, kBoundsThreads, 0, stream>>>(
+    NBSP_COUNT_LAUNCH(1), bounds_kernel<false><<<blocks, kBoundsThreads, 0, stream>>>(
         x, y, z, m, n, partial, status, ax, ay, az, rms_of_a != 0, nullptr, nullptr, nullptr,
         0.0, 0.0);
   }
-  NBSP_COUNT_LAUNCH(1), bounds_final_kernel<<<1, kBoundsThreads, 0, stream>>>(partial, (int)blocks,
-                                                                            n, geometry);
+  if (geometry != nullptr)
+    NBSP_COUNT_LAUNCH(1), bounds_final_kernel<<<1, kBoundsThreads, 0, stream>>>(partial, blocks, n,
+                                                                              geometry);
 }
 
-size_t nbsp_bh_sort_scratch_words(size_t n) { return sort_scratch_words(n); }
+void nbsp_bh_small_keys(const double* x, const double* y, const double* z, const double* m,
+                        size_t n, const double* partial, double* geometry, uint64_t* keys,
+                        uint32_t* index, void* unsorted, const double* ax, const double* ay,
+                        const double* az, double tol_scale, float* unsorted_tol,
+                        cudaStream_t stream) {
+  const unsigned tiles = (unsigned)((n + kSmallTile - 1) / kSmallTile);
+  NBSP_COUNT_LAUNCH(1), small_keys_kernel<<<tiles, kSmallTile, 0, stream>>>(
+      x, y, z, m, n, partial, bounds_blocks(n), geometry, keys, index, (float4*)unsorted, ax, ay,
+      az, tol_scale, unsorted_tol);
+}
+
+void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
+                         uint64_t* keys, uint32_t* index, const void* unsorted, void* pos4,
+                         const float* unsorted_tol, float* tol, int* status,
+                         cudaStream_t stream) {
+  NBSP_COUNT_LAUNCH(1), small_merge_kernel<<<(unsigned)((n + 31) / 32), 32 * kMergeWarps, 0, stream>>>(
+      keys_in, index_in, (int)n, keys, index, (const float4*)unsorted, (float4*)pos4,
+      unsorted_tol, tol, status);
+}
+
+// (buffers for n hold every smaller system too, whose narrow tiles may be more)
+size_t nbsp_bh_sort_scratch_words(size_t n) {
+  const size_t narrow = sort_scratch_words(n < kSortWide ? n : kSortWide - 1);
+  const size_t own = sort_scratch_words(n);
+  return own > narrow ? own : narrow;
+}
 
 void nbsp_bh_keys(const double* x, const double* y, const double* z, const double* m, size_t n,
                   const double* geometry, uint64_t* keys, uint32_t* index, void* unsorted,
                   uint32_t* scratch, const double* ax, const double* ay, const double* az,
                   double tol_scale, float* unsorted_tol, cudaStream_t stream) {
   cudaMemsetAsync(scratch, 0, sort_scratch_words(n) * sizeof(uint32_t), stream);
-  const SortScratch sc = sort_scratch(scratch, n);
+  const SortScratch sc = sort_scratch(scratch);
   size_t blocks = (n + 255) / 256;
   if (blocks < 1) blocks = 1;
   if (blocks > (size_t)kKeysBlocks) blocks = kKeysBlocks;
@@ -2669,18 +2855,20 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
 
 void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t* index_alt,
                   size_t n, uint32_t* scratch, int* status, cudaStream_t stream) {
-  cudaFuncSetAttribute(sort_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)kDownsweepSmem);
-  const SortScratch sc = sort_scratch(scratch, n);
+  const bool narrow = n < kSortWide;
+  const auto pass_kernel = narrow ? sort_pass_kernel<SortNarrow> : sort_pass_kernel<SortWide>;
+  const int threads = narrow ? SortNarrow::kThreads : SortWide::kThreads;
+  const size_t smem = narrow ? sort_pass_smem<SortNarrow>() : sort_pass_smem<SortWide>();
+  cudaFuncSetAttribute(pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const SortScratch sc = sort_scratch(scratch);
   const size_t tiles = sort_tiles(n);
-  NBSP_COUNT_LAUNCH(1), sort_bases_kernel<<<1, kRadix, 0, stream>>>(sc.hist, sc.base);
   uint64_t* kin = keys;
   uint32_t* vin = index;
   uint64_t* kout = keys_alt;
   uint32_t* vout = index_alt;
   for (int pass = 0; pass < kSortPasses; ++pass) {
-    NBSP_COUNT_LAUNCH(1), sort_pass_kernel<<<(unsigned)tiles, kSortThreads, kDownsweepSmem, stream>>>(
-        kin, vin, kout, vout, n, 8 * pass, sc.base + pass * kRadix, sc.ticket + pass,
+    NBSP_COUNT_LAUNCH(1), pass_kernel<<<(unsigned)tiles, threads, smem, stream>>>(
+        kin, vin, kout, vout, n, 8 * pass, sc.hist + pass * kRadix, sc.ticket + pass,
         sc.status + (size_t)pass * tiles * kRadix, status);
     uint64_t* tk = kin;
     kin = kout;

@@ -89,7 +89,12 @@ NBSP_HIDDEN void nbsp_bh_destroy(NbspBarnesHut* bh);
 
 /* ---- kernel launchers (bh.cu) -------------------------------------------- */
 
-/* bbox + centre of mass: geometry[0..3] = root centre xyz + half size (bit-exact
+/* Systems of up to this many particles are sorted by nbsp_bh_small_keys and
+ * nbsp_bh_small_merge (bh.cu says why). */
+#define NBSP_BH_SMALL_SORT ((size_t)98304)
+
+/* bbox + centre of mass (geometry NULL: only the blocks' partial results, which
+ * nbsp_bh_small_keys combines): geometry[0..3] = root centre xyz + half size (bit-exact
  * with the reference), geometry[4..6] = centre of mass.  partial >= 1024*10 doubles. */
 NBSP_HIDDEN void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n,
                                 double* partial, double* geometry, int* status, const double* ax,
@@ -111,8 +116,23 @@ NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z,
 /* (with unsorted_tol != NULL also the relative opening test's tolerance of each
  * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0) */
 
-/* 32-bit words of sort scratch for n keys (digit histograms, pass bases, tile
- * tickets and look-back status words). */
+/* For n <= NBSP_BH_SMALL_SORT, after nbsp_bh_bounds without geometry: geometry,
+ * `unsorted` and `unsorted_tol` as nbsp_bh_bounds and nbsp_bh_keys write them,
+ * and the keys and indices sorted tile by tile; then the whole order, as
+ * nbsp_bh_sort gives it, and the records in it, as nbsp_bh_gather does. */
+NBSP_HIDDEN void nbsp_bh_small_keys(const double* x, const double* y, const double* z,
+                                    const double* m, size_t n, const double* partial,
+                                    double* geometry, uint64_t* keys, uint32_t* index,
+                                    void* unsorted, const double* ax, const double* ay,
+                                    const double* az, double tol_scale, float* unsorted_tol,
+                                    cudaStream_t stream);
+NBSP_HIDDEN void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
+                                     uint64_t* keys, uint32_t* index, const void* unsorted,
+                                     void* pos4, const float* unsorted_tol, float* tol,
+                                     int* status, cudaStream_t stream);
+
+/* 32-bit words of sort scratch for n keys (digit histograms, tile
+ * tickets and look-back status words), enough for every smaller n too. */
 NBSP_HIDDEN size_t nbsp_bh_sort_scratch_words(size_t n);
 
 /* Stable LSD radix sort of (keys, index) by all 64 key bits, after nbsp_bh_keys

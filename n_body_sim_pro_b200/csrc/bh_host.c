@@ -153,21 +153,36 @@ static NBodySimProStatus ensure(NbspBarnesHut** handle, size_t n, NBodySimProErr
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
-/* tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
+/* The bounds, the sorted keys and permutation, and the walk's records in that
+ * order.  tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
 static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, double tol_scale,
                                 int* status, cudaStream_t stream) {
     const int rel = tol_scale > 0.0;
     const NbspLeapfrogFusion* lf = s->leapfrog.vx != NULL ? &s->leapfrog : NULL;
     const int with_a = rel || lf != NULL;
-    nbsp_bh_bounds(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, status,
+    const int small = s->n <= NBSP_BH_SMALL_SORT;
+    nbsp_bh_bounds(s->x, s->y, s->z, s->m, s->n, b->partial, small ? NULL : b->geometry, status,
                    with_a ? s->ax : NULL, with_a ? s->ay : NULL, with_a ? s->az : NULL, rel, lf,
                    stream);
     cudaEventRecord(b->events[1], stream);
+    if (small) {
+        nbsp_bh_small_keys(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, b->keys_alt,
+                           b->index_alt, b->unsorted, s->ax, s->ay, s->az, tol_scale,
+                           rel ? b->tol_unsorted : NULL, stream);
+        cudaEventRecord(b->events[2], stream);
+        nbsp_bh_small_merge(b->keys_alt, b->index_alt, s->n, b->keys, b->index, b->unsorted,
+                            b->pos4, rel ? b->tol_unsorted : NULL, rel ? b->tol : NULL, status,
+                            stream);
+        cudaEventRecord(b->events[3], stream);
+        return N_BODY_SIM_PRO_STATUS_OK;
+    }
     nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys, b->index, b->unsorted,
                  b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, stream);
     cudaEventRecord(b->events[2], stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status, stream);
     cudaEventRecord(b->events[3], stream);
+    nbsp_bh_gather(b->unsorted, b->index, s->n, b->pos4, rel ? b->tol_unsorted : NULL,
+                   rel ? b->tol : NULL, status, stream);
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
@@ -199,8 +214,6 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     const int rel = tol_scale > 0.0;
     morton(b, s, tol_scale, status, stream);
     nbsp_bh_duplicates(b->keys, b->index, s->x, s->y, s->z, n, status, stream);
-    nbsp_bh_gather(b->unsorted, b->index, n, b->pos4, rel ? b->tol_unsorted : NULL,
-                   rel ? b->tol : NULL, status, stream);
     nbsp_bh_build(b->keys, n, p->leaf_capacity, b->tree, status, stream);
     cudaEventRecord(b->events[4], stream);
     nbsp_bh_moments(b->pos4, b->keys, n, b->geometry, p->theta,
