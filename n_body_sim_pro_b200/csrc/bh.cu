@@ -166,6 +166,104 @@ __global__ void __launch_bounds__(kBoundsThreads) bounds_final_kernel(
 }
 
 // ---------------------------------------------------------------------------
+// the tree's arrays
+// ---------------------------------------------------------------------------
+
+// Scratch layout of one tree; binary ids: internal node i -> i (0..n-2),
+// particle leaf k -> (n-1) + k.
+struct Tree {
+  int n;
+  int2* range;        // [n-1] first, last of internal nodes
+  int2* child;        // [n-1] binary ids of the two children
+  int* cell;          // [2n-1] octree level of a cell node, -1 otherwise; keep_kernel
+                      // adds 32 times a kept cell's place among its siblings
+  int* oparent;       // [2n-1] octree parent (binary id) of a kept cell, from keep_kernel
+  int2* below;        // [n-1] splitting cells: walk id of the first child, children
+  int* split;         // [n-1] the splitting cells' binary ids
+  int* split_child;   // [8(n-1)] their octree children's binary ids, -1 behind the last
+  uint32_t* mask;     // [n]   levels of kept nodes starting at particle k
+  uint32_t* offset;   // [n+1] exclusive scan of popcounts; offset[n] = node count
+  uint32_t* block_sums;  // scan scratch
+  // Octree nodes carry two numberings, capacity 2n-1 each.  Depth-first (info,
+  // dnode) with skip links: the stackless walk and the training pairs.  Walk
+  // ids (everything else): the root is 0 and the children of every node are
+  // consecutive, in Morton order, so a node's record names them by the first
+  // one and a count, their records share cache lines, and neither the
+  // interaction-list walk nor the moments pass reads a list of children.
+  int4* info;         // depth-first: next, first particle, leaf count (0: internal), walk id
+  float4* dnode;      // depth-first, 2 per node: wnode's first six words
+  int4* link;         // parent, first child (or first particle), count as in wnode, depth-first id
+  int* level;
+  int* arrive;
+  int* height;
+  double4* mom;       // mass, com xyz (relative to the centre of mass)
+  double* quad64;     // 6 per node: xx xy xz yy yz zz (trace-free)
+  double* trace64;    // sum m |x - com|^2 per node (FP64)
+  // what the interaction-list walk reads of a node, in one 32-byte record: (com
+  // xyz, mass), (ropen2 = (2h / theta)^2, kmass = M (2h)^2 of the relative test,
+  // first particle of a bucket or first child, count as int bits: the particles
+  // of a bucket, minus the children of an internal node)
+  float4* wnode;      // 2 per node
+  // quadrupole walk and correction, 2 per node: (xx, xy, xz, yy), (yz, side =
+  // 2h, spread = sum m |x - com|^2 / (M side^2), shift = distance from the
+  // cell's geometric centre to its centre of mass)
+  float4* wquad;
+  unsigned long long* leaves;  // [2]: buckets; splitting cells << 32 | walk ids below the root
+};
+
+constexpr int kScanItems = 2048;
+
+// Sub-buffers of the tree scratch, each 256-byte aligned, carved from an
+// integer base address (tree_bytes() carves from 0 to measure the layout).
+template <typename T>
+__host__ __device__ inline T* carve(uintptr_t& p, size_t count) {
+  T* out = reinterpret_cast<T*>(p);
+  p += (count * sizeof(T) + 255) & ~(size_t)255;
+  return out;
+}
+
+__host__ __device__ inline Tree tree_layout(uintptr_t p, size_t n_, uintptr_t* end) {
+  Tree t;
+  const size_t n = n_ < 2 ? 2 : n_;
+  const size_t ni = n - 1, nb = 2 * n - 1;
+  t.n = (int)n_;
+  t.range = carve<int2>(p, ni);
+  t.child = carve<int2>(p, ni);
+  t.cell = carve<int>(p, nb);
+  t.oparent = carve<int>(p, nb);
+  t.below = carve<int2>(p, ni);
+  t.split = carve<int>(p, ni);
+  t.split_child = carve<int>(p, 8 * ni);
+  t.mask = carve<uint32_t>(p, n);
+  t.offset = carve<uint32_t>(p, n + 1);
+  t.block_sums = carve<uint32_t>(p, (n + kScanItems - 1) / kScanItems + 1);
+  t.info = carve<int4>(p, nb);
+  t.dnode = carve<float4>(p, 2 * nb);
+  t.link = carve<int4>(p, nb);
+  t.level = carve<int>(p, nb);
+  t.arrive = carve<int>(p, nb);
+  t.height = carve<int>(p, nb);
+  t.mom = carve<double4>(p, nb);
+  t.quad64 = carve<double>(p, 6 * nb);
+  t.trace64 = carve<double>(p, nb);
+  t.wnode = carve<float4>(p, 2 * nb);
+  t.wquad = carve<float4>(p, 2 * nb);
+  t.leaves = carve<unsigned long long>(p, 2);
+  if (end != nullptr) *end = p;
+  return t;
+}
+
+inline Tree tree_view(void* base, size_t n) {
+  return tree_layout(reinterpret_cast<uintptr_t>(base), n, nullptr);
+}
+
+size_t tree_bytes(size_t n) {
+  uintptr_t end = 0;
+  tree_layout(0, n, &end);
+  return (size_t)end;
+}
+
+// ---------------------------------------------------------------------------
 // Morton keys
 // ---------------------------------------------------------------------------
 
@@ -251,6 +349,17 @@ inline size_t sort_scratch_words(size_t n) {
   return kSortPasses * kRadix + kSortPasses + kSortPasses * sort_tiles(n) * kRadix;
 }
 
+// What the build and the walk count into starts at zero (with every particle's
+// mask, which the keys kernels clear beside its key; memsets took a place of
+// their own on the stream).
+constexpr int kCounters = 8;
+__device__ __forceinline__ void start_tree(const Tree& t, unsigned long long* counters) {
+  if (blockIdx.x == 0 && threadIdx.x < kCounters) {
+    counters[threadIdx.x] = 0;
+    if (threadIdx.x < 2) t.leaves[threadIdx.x] = 0;
+  }
+}
+
 // Particle i's Morton key under root cube `geometry`, and its record for the
 // walk, still in input order: the float4 (relative to the centre of mass) and
 // with `unsorted_tol` the relative opening test's alpha max(|a_old|, rms) / G.
@@ -276,8 +385,10 @@ __global__ void __launch_bounds__(256) keys_kernel(
     const double* __restrict__ m, size_t n, const double* __restrict__ geometry,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ index, float4* __restrict__ unsorted,
     uint32_t* __restrict__ hist, const double* __restrict__ ax, const double* __restrict__ ay,
-    const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol) {
+    const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol, Tree tree,
+    unsigned long long* counters) {
   __shared__ uint32_t h[kSortPasses][kRadix];
+  start_tree(tree, counters);
   for (int k = threadIdx.x; k < kSortPasses * kRadix; k += blockDim.x) (&h[0][0])[k] = 0;
   __syncthreads();
   double geo[8];
@@ -296,6 +407,7 @@ __global__ void __launch_bounds__(256) keys_kernel(
       key = particle_key(i, x, y, z, m, geo, ax, ay, az, tol_scale, unsorted, unsorted_tol);
       keys[i] = key;
       index[i] = (uint32_t)i;
+      tree.mask[i] = 0;
     }
 #pragma unroll
     // digit counts: the low six bytes of the keys of one warp are spread over
@@ -500,12 +612,14 @@ __global__ void __launch_bounds__(kSmallTile) small_keys_kernel(
     const double* __restrict__ m, size_t n, const double* __restrict__ partial, int blocks,
     double* __restrict__ geometry, uint64_t* __restrict__ keys, uint32_t* __restrict__ index,
     float4* __restrict__ unsorted, const double* __restrict__ ax, const double* __restrict__ ay,
-    const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol) {
+    const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol, Tree tree,
+    unsigned long long* counters) {
   __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
   __shared__ double s_geo[8];
   __shared__ uint64_t sk[kSmallTile];
   __shared__ uint32_t sv[kSmallTile];
   const int t = threadIdx.x;
+  start_tree(tree, counters);
   root_geometry(partial, blocks, n, sh, s_geo);
   __syncthreads();
   double geo[8];
@@ -514,8 +628,10 @@ __global__ void __launch_bounds__(kSmallTile) small_keys_kernel(
   if (blockIdx.x == 0 && t < 8) geometry[t] = s_geo[t];
   const size_t i = (size_t)blockIdx.x * kSmallTile + t;
   uint64_t key = ~0ull;  // past the end: behind every 63-bit key
-  if (i < n)
+  if (i < n) {
+    tree.mask[i] = 0;
     key = particle_key(i, x, y, z, m, geo, ax, ay, az, tol_scale, unsorted, unsorted_tol);
+  }
   uint32_t val = (uint32_t)t;
   for (int k = 2; k <= kSmallTile; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
@@ -610,23 +726,21 @@ __global__ void __launch_bounds__(32 * kMergeWarps) small_merge_kernel(
 // keys; each particle is compared with the next kDupWindow particles of its run
 // (runs of equal 63-bit keys are otherwise rare: cells of 2^-21 of the root).
 constexpr int kDupWindow = 32;
-__global__ void duplicates_kernel(const uint64_t* __restrict__ keys,
-                                  const uint32_t* __restrict__ perm, const double* __restrict__ x,
-                                  const double* __restrict__ y, const double* __restrict__ z,
-                                  size_t n, int* status) {
-  for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s + 1 < n;
-       s += (size_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[s];
-    if (keys[s + 1] != k) continue;
-    const uint32_t i = perm[s];
-    if (i >= n) continue;
-    const double px = x[i], py = y[i], pz = z[i];
-    for (size_t t = s + 1; t < n && t <= s + kDupWindow && keys[t] == k; ++t) {
-      const uint32_t j = perm[t];
-      if (j < n && x[j] == px && y[j] == py && z[j] == pz) {
-        atomicOr(status, NBSP_DEVICE_ERROR_DUPLICATE_POSITION);
-        return;
-      }
+__device__ __forceinline__ void flag_duplicates(size_t s, const uint64_t* __restrict__ keys,
+                                                const uint32_t* __restrict__ perm,
+                                                const double* __restrict__ x,
+                                                const double* __restrict__ y,
+                                                const double* __restrict__ z, size_t n,
+                                                int* status) {
+  const uint64_t k = keys[s];
+  const uint32_t i = perm[s];
+  if (i >= n) return;
+  const double px = x[i], py = y[i], pz = z[i];
+  for (size_t t = s + 1; t < n && t <= s + kDupWindow && keys[t] == k; ++t) {
+    const uint32_t j = perm[t];
+    if (j < n && x[j] == px && y[j] == py && z[j] == pz) {
+      atomicOr(status, NBSP_DEVICE_ERROR_DUPLICATE_POSITION);
+      return;
     }
   }
 }
@@ -658,11 +772,19 @@ __global__ void gather_kernel(const float4* __restrict__ unsorted,
 // (one aligned 32-byte record), so this pass is coalesced both ways.  KICK:
 // the closing kick of a device-resident leapfrog step, v += h a, with
 // kick_drift_kernel's arithmetic on the accelerations just written.
+// The first thread copies the tree's node count, leaf count and depth to
+// counters[2..4].
 template <bool KICK>
 __global__ void unsort_kernel(const double4* __restrict__ acc, size_t n, double g,
                               double* __restrict__ ax, double* __restrict__ ay,
                               double* __restrict__ az, double* __restrict__ vx,
-                              double* __restrict__ vy, double* __restrict__ vz, double h) {
+                              double* __restrict__ vy, double* __restrict__ vz, double h, Tree t,
+                              unsigned long long* counters) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    counters[2] = t.offset[t.n];
+    counters[3] = t.leaves[0];
+    counters[4] = (unsigned long long)t.height[0];
+  }
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const double4 a = acc[i];
@@ -682,100 +804,6 @@ __global__ void unsort_kernel(const double4* __restrict__ acc, size_t n, double 
 // tree
 // ---------------------------------------------------------------------------
 
-// Scratch layout of one tree; binary ids: internal node i -> i (0..n-2),
-// particle leaf k -> (n-1) + k.
-struct Tree {
-  int n;
-  int2* range;        // [n-1] first, last of internal nodes
-  int2* child;        // [n-1] binary ids of the two children
-  int* cell;          // [2n-1] octree level of a cell node, -1 otherwise; keep_kernel
-                      // adds 32 times a kept cell's place among its siblings
-  int* oparent;       // [2n-1] octree parent (binary id) of a kept cell, from keep_kernel
-  int2* below;        // [n-1] splitting cells: walk id of the first child, children
-  int* split;         // [n-1] the splitting cells' binary ids
-  int* split_child;   // [8(n-1)] their octree children's binary ids, -1 behind the last
-  uint32_t* mask;     // [n]   levels of kept nodes starting at particle k
-  uint32_t* offset;   // [n+1] exclusive scan of popcounts; offset[n] = node count
-  uint32_t* block_sums;  // scan scratch
-  // Octree nodes carry two numberings, capacity 2n-1 each.  Depth-first (info,
-  // dnode) with skip links: the stackless walk and the training pairs.  Walk
-  // ids (everything else): the root is 0 and the children of every node are
-  // consecutive, in Morton order, so a node's record names them by the first
-  // one and a count, their records share cache lines, and neither the
-  // interaction-list walk nor the moments pass reads a list of children.
-  int4* info;         // depth-first: next, first particle, leaf count (0: internal), walk id
-  float4* dnode;      // depth-first, 2 per node: wnode's first six words
-  int4* link;         // parent, first child (or first particle), count as in wnode, depth-first id
-  int* level;
-  int* arrive;
-  int* height;
-  double4* mom;       // mass, com xyz (relative to the centre of mass)
-  double* quad64;     // 6 per node: xx xy xz yy yz zz (trace-free)
-  double* trace64;    // sum m |x - com|^2 per node (FP64)
-  // what the interaction-list walk reads of a node, in one 32-byte record: (com
-  // xyz, mass), (ropen2 = (2h / theta)^2, kmass = M (2h)^2 of the relative test,
-  // first particle of a bucket or first child, count as int bits: the particles
-  // of a bucket, minus the children of an internal node)
-  float4* wnode;      // 2 per node
-  // quadrupole walk and correction, 2 per node: (xx, xy, xz, yy), (yz, side =
-  // 2h, spread = sum m |x - com|^2 / (M side^2), shift = distance from the
-  // cell's geometric centre to its centre of mass)
-  float4* wquad;
-  unsigned long long* leaves;  // [2]: buckets; splitting cells << 32 | walk ids below the root
-};
-
-constexpr int kScanItems = 2048;
-
-// Sub-buffers of the tree scratch, each 256-byte aligned, carved from an
-// integer base address (tree_bytes() carves from 0 to measure the layout).
-template <typename T>
-__host__ __device__ inline T* carve(uintptr_t& p, size_t count) {
-  T* out = reinterpret_cast<T*>(p);
-  p += (count * sizeof(T) + 255) & ~(size_t)255;
-  return out;
-}
-
-__host__ __device__ inline Tree tree_layout(uintptr_t p, size_t n_, uintptr_t* end) {
-  Tree t;
-  const size_t n = n_ < 2 ? 2 : n_;
-  const size_t ni = n - 1, nb = 2 * n - 1;
-  t.n = (int)n_;
-  t.range = carve<int2>(p, ni);
-  t.child = carve<int2>(p, ni);
-  t.cell = carve<int>(p, nb);
-  t.oparent = carve<int>(p, nb);
-  t.below = carve<int2>(p, ni);
-  t.split = carve<int>(p, ni);
-  t.split_child = carve<int>(p, 8 * ni);
-  t.mask = carve<uint32_t>(p, n);
-  t.offset = carve<uint32_t>(p, n + 1);
-  t.block_sums = carve<uint32_t>(p, (n + kScanItems - 1) / kScanItems + 1);
-  t.info = carve<int4>(p, nb);
-  t.dnode = carve<float4>(p, 2 * nb);
-  t.link = carve<int4>(p, nb);
-  t.level = carve<int>(p, nb);
-  t.arrive = carve<int>(p, nb);
-  t.height = carve<int>(p, nb);
-  t.mom = carve<double4>(p, nb);
-  t.quad64 = carve<double>(p, 6 * nb);
-  t.trace64 = carve<double>(p, nb);
-  t.wnode = carve<float4>(p, 2 * nb);
-  t.wquad = carve<float4>(p, 2 * nb);
-  t.leaves = carve<unsigned long long>(p, 2);
-  if (end != nullptr) *end = p;
-  return t;
-}
-
-inline Tree tree_view(void* base, size_t n) {
-  return tree_layout(reinterpret_cast<uintptr_t>(base), n, nullptr);
-}
-
-size_t tree_bytes(size_t n) {
-  uintptr_t end = 0;
-  tree_layout(0, n, &end);
-  return (size_t)end;
-}
-
 // Common prefix length of sorted keys i and j in bits (Karras 2012, with the
 // index as tie breaker); -1 outside [0, n).
 __device__ __forceinline__ int prefix(const uint64_t* __restrict__ keys, int n, int i, int j) {
@@ -793,11 +821,16 @@ __device__ __forceinline__ int level_of_delta(int delta) { return min(delta / 3,
 // The parent's prefix length is that of the node's range extended by one key
 // on the side with the longer common prefix, max(delta(first - 1, first),
 // delta(last, last + 1)), so each thread decides its own node and its leaf
-// children without reading another thread's results.
-__global__ void radix_tree_kernel(const uint64_t* __restrict__ keys, Tree t, int* status) {
+// children without reading another thread's results.  Thread i compares key i
+// with key i + 1 in any case, so it also looks for shared positions.
+__global__ void radix_tree_kernel(const uint64_t* __restrict__ keys,
+                                  const uint32_t* __restrict__ perm, const double* __restrict__ x,
+                                  const double* __restrict__ y, const double* __restrict__ z,
+                                  Tree t, int* status) {
   const int n = t.n;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
+  if (keys[i] == keys[i + 1]) flag_duplicates((size_t)i, keys, perm, x, y, z, (size_t)n, status);
   const int d = prefix(keys, n, i, i + 1) - prefix(keys, n, i, i - 1) >= 0 ? 1 : -1;
   const int dmin = prefix(keys, n, i, i - d);
   int lmax = 2;
@@ -1001,90 +1034,131 @@ __global__ void __launch_bounds__(kKeepThreads) keep_kernel(Tree t, int leaf_cap
   for (int e = tid; e < count; e += kKeepThreads) t.split[slot + e] = s_b[e];
   for (int e = tid; e < 8 * count; e += kKeepThreads) t.split_child[8 * slot + e] = s_child[e];
 }
-// Exclusive scan of popc(mask[k]) into offset[0..n].
-__global__ void scan_reduce_kernel(Tree t) {
-  __shared__ uint32_t sh[256];
+// Inclusive scan of v over a block of WARPS warps.
+template <int WARPS>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_sums) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t x = v;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t u = __shfl_up_sync(kFull, x, off);
+    if (lane >= off) x += u;
+  }
+  if (lane == 31) warp_sums[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    uint32_t y = lane < WARPS ? warp_sums[lane] : 0u;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t u = __shfl_up_sync(kFull, y, off);
+      if (lane >= off) y += u;
+    }
+    if (lane < WARPS) warp_sums[lane] = y;
+  }
+  __syncthreads();
+  x += w > 0 ? warp_sums[w - 1] : 0u;
+  __syncthreads();  // (warp_sums may be used again)
+  return x;
+}
+
+// Exclusive scan of popc(mask[k]) into offset[0..n].  Up to NBSP_BH_SMALL_SORT
+// particles in one kernel, whose blocks count what lies before them themselves
+// (at most 24 sixteen-byte loads a thread); then block sums first, scanned by a
+// kernel of their own only when they are many (at 1M 488).
+__device__ __forceinline__ uint32_t popc4(uint4 m) {
+  return __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+}
+
+constexpr int kSmallScanThreads = 1024;
+__global__ void __launch_bounds__(kSmallScanThreads) scan_small_kernel(Tree t) {
+  __shared__ uint32_t warp_sums[32];
+  __shared__ uint32_t s_before;
+  const int n = t.n, tid = threadIdx.x;
+  const int base = blockIdx.x * kScanItems;
+  const uint4* mask4 = reinterpret_cast<const uint4*>(t.mask);
+  uint32_t before = 0;
+#pragma unroll 8
+  for (int q = tid; q < base / 4; q += kSmallScanThreads) before += popc4(mask4[q]);
+  before = block_scan<32>(before, warp_sums);
+  if (tid == kSmallScanThreads - 1) s_before = before;
+  const int i0 = base + 2 * tid, i1 = i0 + 1;
+  const uint32_t v0 = i0 < n ? __popc(t.mask[i0]) : 0u, v1 = i1 < n ? __popc(t.mask[i1]) : 0u;
+  const uint32_t incl = block_scan<32>(v0 + v1, warp_sums) + s_before;
+  if (i0 < n) t.offset[i0] = incl - v0 - v1;
+  if (i1 < n) t.offset[i1] = incl - v1;
+  if (base + kScanItems >= n && tid == kSmallScanThreads - 1) t.offset[n] = incl;
+}
+
+constexpr int kScanThreads = 256;
+constexpr int kScanSums = 1024;  // block sums that every block adds up itself
+__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(Tree t) {
+  __shared__ uint32_t warp_sums[32];
   const int n = t.n;
   const size_t base = (size_t)blockIdx.x * kScanItems;
   uint32_t s = 0;
-  for (int k = threadIdx.x; k < kScanItems; k += 256) {
-    const size_t i = base + k;
+#pragma unroll
+  for (int k = 0; k < kScanItems / kScanThreads; ++k) {
+    const size_t i = base + k * kScanThreads + threadIdx.x;
     if (i < (size_t)n) s += __popc(t.mask[i]);
   }
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int stride = 128; stride > 0; stride >>= 1) {
-    if (threadIdx.x < stride) sh[threadIdx.x] += sh[threadIdx.x + stride];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) t.block_sums[blockIdx.x] = sh[0];
+  s = block_scan<kScanThreads / 32>(s, warp_sums);
+  if (threadIdx.x == kScanThreads - 1) t.block_sums[blockIdx.x] = s;
 }
 
 // Exclusive scan of the block sums in place (one block of 1024 threads, in
-// chunks of 1024), total into offset[n].
+// chunks of 1024).
 __global__ void __launch_bounds__(1024) scan_blocks_kernel(Tree t, int blocks) {
   __shared__ uint32_t warp_sums[32];
   __shared__ uint32_t carry;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   for (int base = 0; base < blocks; base += 1024) {
     const int b = base + threadIdx.x;
     const uint32_t v = b < blocks ? t.block_sums[b] : 0u;
-    uint32_t x = v;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t u = __shfl_up_sync(kFull, x, off);
-      if (lane >= off) x += u;
-    }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      uint32_t w = warp_sums[lane];
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t u = __shfl_up_sync(kFull, w, off);
-        if (lane >= off) w += u;
-      }
-      warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const uint32_t incl = x + (wid > 0 ? warp_sums[wid - 1] : 0u);
+    const uint32_t incl = block_scan<32>(v, warp_sums);
     const uint32_t c = carry;
     if (b < blocks) t.block_sums[b] = c + incl - v;
     __syncthreads();
     if (threadIdx.x == 1023) carry = c + incl;
     __syncthreads();
   }
-  if (threadIdx.x == 0) t.offset[t.n] = carry;
 }
 
-__global__ void scan_apply_kernel(Tree t) {
-  __shared__ uint32_t sh[256];
-  const int n = t.n;
+// SCANNED: the block sums hold what lies before each block.
+template <bool SCANNED>
+__global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(Tree t) {
+  __shared__ uint32_t warp_sums[32];
+  __shared__ uint32_t s_before;
+  const int n = t.n, tid = threadIdx.x;
+  if (SCANNED) {
+    if (tid == 0) s_before = t.block_sums[blockIdx.x];
+  } else {
+    uint32_t before = 0;
+#pragma unroll
+    for (int k = 0; k < kScanSums / kScanThreads; ++k) {
+      const unsigned b = k * kScanThreads + tid;
+      if (b < blockIdx.x) before += t.block_sums[b];
+    }
+    before = block_scan<kScanThreads / 32>(before, warp_sums);
+    if (tid == kScanThreads - 1) s_before = before;
+  }
   const size_t base = (size_t)blockIdx.x * kScanItems;
-  constexpr int per = kScanItems / 256;  // 8 contiguous items per thread
+  constexpr int per = kScanItems / kScanThreads;  // 8 contiguous items per thread
   uint32_t v[per];
   uint32_t s = 0;
+#pragma unroll
   for (int k = 0; k < per; ++k) {
-    const size_t i = base + (size_t)threadIdx.x * per + k;
+    const size_t i = base + (size_t)tid * per + k;
     v[k] = i < (size_t)n ? __popc(t.mask[i]) : 0u;
     s += v[k];
   }
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  uint32_t incl = s;
-  for (int off = 1; off < 256; off <<= 1) {
-    const uint32_t add = threadIdx.x >= off ? sh[threadIdx.x - off] : 0u;
-    __syncthreads();
-    incl += add;
-    sh[threadIdx.x] = incl;
-    __syncthreads();
-  }
-  uint32_t run = t.block_sums[blockIdx.x] + incl - s;
+  const uint32_t incl = block_scan<kScanThreads / 32>(s, warp_sums) + s_before;
+  uint32_t run = incl - s;
+#pragma unroll
   for (int k = 0; k < per; ++k) {
-    const size_t i = base + (size_t)threadIdx.x * per + k;
+    const size_t i = base + (size_t)tid * per + k;
     if (i < (size_t)n) t.offset[i] = run;
     run += v[k];
   }
+  if (base + kScanItems >= (size_t)n && tid == kScanThreads - 1) t.offset[n] = incl;
 }
 
 __device__ __forceinline__ int dfs_index(const Tree& t, int begin, int lvl) {
@@ -2736,13 +2810,6 @@ __global__ void __launch_bounds__(128) corr_apply_kernel(const float4* __restric
   }
 }
 
-__global__ void tree_counts_kernel(Tree t, unsigned long long* counters) {
-  if (threadIdx.x != 0) return;
-  counters[2] = t.offset[t.n];
-  counters[3] = *t.leaves;
-  counters[4] = (unsigned long long)t.height[0];
-}
-
 int grid_for(size_t n, int threads) {
   size_t b = (n + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -2815,12 +2882,12 @@ void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n, 
 void nbsp_bh_small_keys(const double* x, const double* y, const double* z, const double* m,
                         size_t n, const double* partial, double* geometry, uint64_t* keys,
                         uint32_t* index, void* unsorted, const double* ax, const double* ay,
-                        const double* az, double tol_scale, float* unsorted_tol,
-                        cudaStream_t stream) {
+                        const double* az, double tol_scale, float* unsorted_tol, void* tree,
+                        unsigned long long* counters, cudaStream_t stream) {
   const unsigned tiles = (unsigned)((n + kSmallTile - 1) / kSmallTile);
   NBSP_COUNT_LAUNCH(1), small_keys_kernel<<<tiles, kSmallTile, 0, stream>>>(
       x, y, z, m, n, partial, bounds_blocks(n), geometry, keys, index, (float4*)unsorted, ax, ay,
-      az, tol_scale, unsorted_tol);
+      az, tol_scale, unsorted_tol, tree_view(tree, n), counters);
 }
 
 void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
@@ -2842,7 +2909,8 @@ size_t nbsp_bh_sort_scratch_words(size_t n) {
 void nbsp_bh_keys(const double* x, const double* y, const double* z, const double* m, size_t n,
                   const double* geometry, uint64_t* keys, uint32_t* index, void* unsorted,
                   uint32_t* scratch, const double* ax, const double* ay, const double* az,
-                  double tol_scale, float* unsorted_tol, cudaStream_t stream) {
+                  double tol_scale, float* unsorted_tol, void* tree,
+                  unsigned long long* counters, cudaStream_t stream) {
   cudaMemsetAsync(scratch, 0, sort_scratch_words(n) * sizeof(uint32_t), stream);
   const SortScratch sc = sort_scratch(scratch);
   size_t blocks = (n + 255) / 256;
@@ -2850,7 +2918,7 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
   if (blocks > (size_t)kKeysBlocks) blocks = kKeysBlocks;
   NBSP_COUNT_LAUNCH(1), keys_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
       x, y, z, m, n, geometry, keys, index, (float4*)unsorted, sc.hist, ax, ay, az, tol_scale,
-      unsorted_tol);
+      unsorted_tol, tree_view(tree, n), counters);
 }
 
 void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t* index_alt,
@@ -2880,12 +2948,6 @@ void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t*
   // kSortPasses = 8 (even): the result is back in (keys, index)
 }
 
-void nbsp_bh_duplicates(const uint64_t* keys, const uint32_t* perm, const double* x,
-                        const double* y, const double* z, size_t n, int* status,
-                        cudaStream_t stream) {
-  NBSP_COUNT_LAUNCH(1), duplicates_kernel<<<grid_for(n, 256), 256, 0, stream>>>(keys, perm, x, y, z, n, status);
-}
-
 void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* pos4,
                     const float* unsorted_tol, float* tol, int* status, cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), gather_kernel<<<grid_for(n, 256), 256, 0, stream>>>(
@@ -2894,21 +2956,29 @@ void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* 
 
 size_t nbsp_bh_tree_bytes(size_t n) { return tree_bytes(n); }
 
-void nbsp_bh_build(const uint64_t* keys, size_t n, int leaf_capacity, void* tree, int* status,
+void nbsp_bh_build(const uint64_t* keys, const uint32_t* perm, const double* x, const double* y,
+                   const double* z, size_t n, int leaf_capacity, void* tree, int* status,
                    cudaStream_t stream) {
   Tree t = tree_view(tree, n);
-  cudaMemsetAsync(t.mask, 0, n * sizeof(uint32_t), stream);
-  cudaMemsetAsync(t.leaves, 0, 2 * sizeof(unsigned long long), stream);
   if (n >= 2)
-    NBSP_COUNT_LAUNCH(1), radix_tree_kernel<<<(unsigned)((n - 1 + 255) / 256), 256, 0, stream>>>(keys, t, status);
+    NBSP_COUNT_LAUNCH(1), radix_tree_kernel<<<(unsigned)((n - 1 + 255) / 256), 256, 0, stream>>>(
+        keys, perm, x, y, z, t, status);
   // (n >= 2: the caller handles a lone particle without a tree)
   const unsigned keep_blocks = (unsigned)((n - 1 + kKeepNodes - 1) / kKeepNodes);
   if (keep_blocks > 0)
     NBSP_COUNT_LAUNCH(1), keep_kernel<<<keep_blocks, kKeepThreads, 0, stream>>>(t, leaf_capacity, status);
   const int blocks = (int)((n + kScanItems - 1) / kScanItems);
-  NBSP_COUNT_LAUNCH(1), scan_reduce_kernel<<<blocks, 256, 0, stream>>>(t);
-  NBSP_COUNT_LAUNCH(1), scan_blocks_kernel<<<1, 1024, 0, stream>>>(t, blocks);
-  NBSP_COUNT_LAUNCH(1), scan_apply_kernel<<<blocks, 256, 0, stream>>>(t);
+  if (n <= NBSP_BH_SMALL_SORT) {
+    NBSP_COUNT_LAUNCH(1), scan_small_kernel<<<blocks, kSmallScanThreads, 0, stream>>>(t);
+  } else {
+    NBSP_COUNT_LAUNCH(1), scan_reduce_kernel<<<blocks, kScanThreads, 0, stream>>>(t);
+    if (blocks <= kScanSums) {
+      NBSP_COUNT_LAUNCH(1), scan_apply_kernel<false><<<blocks, kScanThreads, 0, stream>>>(t);
+    } else {
+      NBSP_COUNT_LAUNCH(1), scan_blocks_kernel<<<1, 1024, 0, stream>>>(t, blocks);
+      NBSP_COUNT_LAUNCH(1), scan_apply_kernel<true><<<blocks, kScanThreads, 0, stream>>>(t);
+    }
+  }
   // (at most a splitting cell per two particles: eight threads each)
   const size_t place_blocks = (4 * n + 255) / 256;
   NBSP_COUNT_LAUNCH(1), place_kernel<<<(unsigned)(place_blocks < kPlaceBlocks ? place_blocks : kPlaceBlocks), 256, 0, stream>>>(
@@ -2974,14 +3044,16 @@ void nbsp_bh_correct(const void* pos4, size_t n, const void* tree, const void* c
 }
 
 void nbsp_bh_unsort(const void* acc, size_t n, double g, double* ax, double* ay, double* az,
-                    const NbspLeapfrogFusion* leapfrog, cudaStream_t stream) {
+                    const NbspLeapfrogFusion* leapfrog, const void* tree,
+                    unsigned long long* counters, cudaStream_t stream) {
+  const Tree t = tree_view(const_cast<void*>(tree), n);
   if (leapfrog != nullptr && leapfrog->vx != nullptr) {
     NBSP_COUNT_LAUNCH(1), unsort_kernel<true><<<grid_for(n, 256), 256, 0, stream>>>(
         (const double4*)acc, n, g, ax, ay, az, leapfrog->vx, leapfrog->vy, leapfrog->vz,
-        leapfrog->half_dt);
+        leapfrog->half_dt, t, counters);
   } else {
     NBSP_COUNT_LAUNCH(1), unsort_kernel<false><<<grid_for(n, 256), 256, 0, stream>>>(
-        (const double4*)acc, n, g, ax, ay, az, nullptr, nullptr, nullptr, 0.0);
+        (const double4*)acc, n, g, ax, ay, az, nullptr, nullptr, nullptr, 0.0, t, counters);
   }
 }
 
@@ -3006,12 +3078,6 @@ void nbsp_bh_mlp_stats(const float* feat, const float* lab, const int* ok, int r
                        cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), mlp_stats_kernel<<<nbsp_mlp::kIn + nbsp_mlp::kOut, 256, 0, stream>>>(
       feat, lab, ok, rows, (nbsp_mlp::Net*)net);
-}
-
-void nbsp_bh_tree_counts(const void* tree, size_t n, unsigned long long* counters,
-                         cudaStream_t stream) {
-  Tree t = tree_view(const_cast<void*>(tree), n);
-  NBSP_COUNT_LAUNCH(1), tree_counts_kernel<<<1, 32, 0, stream>>>(t, counters);
 }
 
 }  // extern "C"

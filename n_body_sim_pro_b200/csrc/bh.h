@@ -112,9 +112,11 @@ NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z,
                               size_t n, const double* geometry, uint64_t* keys, uint32_t* index,
                               void* unsorted, uint32_t* sort_scratch, const double* ax,
                               const double* ay, const double* az, double tol_scale,
-                              float* unsorted_tol, cudaStream_t stream);
+                              float* unsorted_tol, void* tree, unsigned long long* counters,
+                              cudaStream_t stream);
 /* (with unsorted_tol != NULL also the relative opening test's tolerance of each
- * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0) */
+ * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0;
+ * the tree's masks and leaf counts and the 8 counters are set to zero) */
 
 /* For n <= NBSP_BH_SMALL_SORT, after nbsp_bh_bounds without geometry: geometry,
  * `unsorted` and `unsorted_tol` as nbsp_bh_bounds and nbsp_bh_keys write them,
@@ -125,6 +127,7 @@ NBSP_HIDDEN void nbsp_bh_small_keys(const double* x, const double* y, const doub
                                     double* geometry, uint64_t* keys, uint32_t* index,
                                     void* unsorted, const double* ax, const double* ay,
                                     const double* az, double tol_scale, float* unsorted_tol,
+                                    void* tree, unsigned long long* counters,
                                     cudaStream_t stream);
 NBSP_HIDDEN void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
                                      uint64_t* keys, uint32_t* index, const void* unsorted,
@@ -143,11 +146,6 @@ NBSP_HIDDEN void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_al
                               uint32_t* index_alt, size_t n, uint32_t* sort_scratch, int* status,
                               cudaStream_t stream);
 
-/* Flag NBSP_DEVICE_ERROR_DUPLICATE_POSITION when two particles share a position. */
-NBSP_HIDDEN void nbsp_bh_duplicates(const uint64_t* keys, const uint32_t* perm, const double* x,
-                                    const double* y, const double* z, size_t n, int* status,
-                                    cudaStream_t stream);
-
 /* pos4[s] = unsorted[perm[s]] (Morton order), tol[s] = unsorted_tol[perm[s]]. */
 NBSP_HIDDEN void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* pos4,
                                 const float* unsorted_tol, float* tol, int* status,
@@ -156,9 +154,12 @@ NBSP_HIDDEN void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size
 /* Device-side layout of the tree build scratch; sized by nbsp_bh_tree_bytes. */
 NBSP_HIDDEN size_t nbsp_bh_tree_bytes(size_t n);
 
-/* Build the octree from the sorted keys. `tree` is nbsp_bh_tree_bytes(n) bytes. */
-NBSP_HIDDEN void nbsp_bh_build(const uint64_t* keys, size_t n, int leaf_capacity, void* tree,
-                               int* status, cudaStream_t stream);
+/* Build the octree from the sorted keys; flag NBSP_DEVICE_ERROR_DUPLICATE_POSITION
+ * when two particles share a position.  `tree` is nbsp_bh_tree_bytes(n) bytes,
+ * started by nbsp_bh_keys or nbsp_bh_small_keys. */
+NBSP_HIDDEN void nbsp_bh_build(const uint64_t* keys, const uint32_t* perm, const double* x,
+                               const double* y, const double* z, size_t n, int leaf_capacity,
+                               void* tree, int* status, cudaStream_t stream);
 
 /* Moments + walk-format node records.  order 1 or 2. */
 /* Opening tests: the reference's (2h)^2 < theta^2 d^2 (barnes_hut.c:596-599), or
@@ -254,12 +255,10 @@ NBSP_HIDDEN const void* nbsp_bh_tree(const NbspBarnesHut* bh);
  * stores it) */
 NBSP_HIDDEN void nbsp_bh_unsort(const void* acc, size_t n, double gravitational_constant,
                                 double* ax, double* ay, double* az,
-                                const NbspLeapfrogFusion* leapfrog, cudaStream_t stream);
-/* (with a leapfrog fusion, NULL: none, v is then kicked by half_dt * a) */
-
-/* Copy node_count, leaf_count and depth of the tree to counters[2..4]. */
-NBSP_HIDDEN void nbsp_bh_tree_counts(const void* tree, size_t n, unsigned long long* counters,
-                                     cudaStream_t stream);
+                                const NbspLeapfrogFusion* leapfrog, const void* tree,
+                                unsigned long long* counters, cudaStream_t stream);
+/* (with a leapfrog fusion, NULL: none, v is then kicked by half_dt * a; the
+ * tree's node_count, leaf_count and depth go to counters[2..4]) */
 
 #ifdef __cplusplus
 }

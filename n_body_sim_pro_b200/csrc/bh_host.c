@@ -168,7 +168,7 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
     if (small) {
         nbsp_bh_small_keys(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, b->keys_alt,
                            b->index_alt, b->unsorted, s->ax, s->ay, s->az, tol_scale,
-                           rel ? b->tol_unsorted : NULL, stream);
+                           rel ? b->tol_unsorted : NULL, b->tree, b->counters, stream);
         cudaEventRecord(b->events[2], stream);
         nbsp_bh_small_merge(b->keys_alt, b->index_alt, s->n, b->keys, b->index, b->unsorted,
                             b->pos4, rel ? b->tol_unsorted : NULL, rel ? b->tol : NULL, status,
@@ -177,7 +177,8 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
         return N_BODY_SIM_PRO_STATUS_OK;
     }
     nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys, b->index, b->unsorted,
-                 b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, stream);
+                 b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, b->tree,
+                 b->counters, stream);
     cudaEventRecord(b->events[2], stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status, stream);
     cudaEventRecord(b->events[3], stream);
@@ -204,7 +205,6 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
         b->timed = 0;
         return N_BODY_SIM_PRO_STATUS_OK;
     }
-    BH_TRY(cudaMemsetAsync(b->counters, 0, BH_COUNTERS * sizeof(unsigned long long), stream));
     cudaEventRecord(b->events[0], stream);
     /* relative opening test: tolerance alpha |a_old| / G */
     const double g = fabs(p->gravitational_constant);
@@ -213,8 +213,8 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
         return st;
     const int rel = tol_scale > 0.0;
     morton(b, s, tol_scale, status, stream);
-    nbsp_bh_duplicates(b->keys, b->index, s->x, s->y, s->z, n, status, stream);
-    nbsp_bh_build(b->keys, n, p->leaf_capacity, b->tree, status, stream);
+    nbsp_bh_build(b->keys, b->index, s->x, s->y, s->z, n, p->leaf_capacity, b->tree, status,
+                  stream);
     cudaEventRecord(b->events[4], stream);
     nbsp_bh_moments(b->pos4, b->keys, n, b->geometry, p->theta,
                     rel ? fmin(p->theta, NBSP_BH_START_THETA) : 0.0, p->opening,
@@ -229,8 +229,7 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
                         b->counters, status, stream);
     cudaEventRecord(b->events[6], stream);
     nbsp_bh_unsort(b->acc, n, p->gravitational_constant, s->ax, s->ay, s->az,
-                   s->leapfrog.vx != NULL ? &s->leapfrog : NULL, stream);
-    nbsp_bh_tree_counts(b->tree, n, b->counters, stream);
+                   s->leapfrog.vx != NULL ? &s->leapfrog : NULL, b->tree, b->counters, stream);
     cudaEventRecord(b->events[7], stream);
     BH_TRY(cudaGetLastError());
     BH_TRY(cudaMemcpyAsync(b->host_counters, b->counters, BH_COUNTERS * sizeof(unsigned long long),
