@@ -2103,9 +2103,14 @@ constexpr int kListStackRel = 960;
 // blocks per SM of the monopole list walks (at most 56 registers at 9): 9
 // where shared memory allows (the plain and the corrected walk's block at
 // 1024 ids is 24,576 B)
-template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED>
+// LATENCY, the walk of systems whose blocks all fit at once at 4 (quadrupole 3)
+// per SM: there a warp has its scheduler nearly to itself, and what counts is
+// the length of its own chain
+template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED, bool LATENCY>
 constexpr int list_walk_blocks() {
-  return ORDER != 1 ? 5 : (!SHARED && (REL ? STACK == kListStackRel : true)) ? 9 : 8;
+  return LATENCY      ? (ORDER != 1 ? 3 : 4)
+         : ORDER != 1 ? 5
+         : (!SHARED && (REL ? STACK == kListStackRel : true)) ? 9 : 8;
 }
 // SHARED walk: the block's top-of-tree traversal keeps its stack and frontier
 // in the warps' stack space (it ends before any warp walks)
@@ -2152,8 +2157,14 @@ static_assert(kCtaStack + kFrontier <= 3 * kListStack, "frontier inside warp 2's
 // would alone (the same interactions; only the order of the FP32 sums moves).
 // A block whose shared stack or frontier would overflow starts every group
 // from the root instead.
-template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED = false>
-__global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, CORR, REL, SHARED>())) walk_lists_kernel(
+//
+// LATENCY (small systems): the same steps with registers to spare, so that the
+// terms of a tile overlap (a lone warp waited about 2,800 cycles for a tile that
+// is 600 instructions at 56 registers); the records of the next step's nodes are
+// loaded before this step's tiles are evaluated, and four nodes at a time take
+// the per-target test.  LATENCY_MEASURED
+template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED = false, bool LATENCY = false>
+__global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, CORR, REL, SHARED, LATENCY>())) walk_lists_kernel(
     const float4* __restrict__ pos, const float* __restrict__ tol, int n, Tree t, float eps2,
     const uint32_t* __restrict__ perm, double4* __restrict__ acc,
     unsigned long long* __restrict__ counters, int* status,
@@ -2368,6 +2379,16 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
     stack[0] = 0;
   }
   __syncwarp();
+  // the next step's nodes (a lane without one: -1) and with LATENCY their
+  // records; idle lanes load the root's, so that no branch diverges
+  int next = lane < top ? stack[top - 1 - lane] : -1;
+  float4 next0 = make_float4(0.f, 0.f, 0.f, 0.f), next1 = next0;
+  auto load_next = [&]() {
+    const int at = next >= 0 && next < total ? next : 0;
+    next0 = __ldg(&t.wnode[2 * at]);
+    next1 = __ldg(&t.wnode[2 * at + 1]);
+  };
+  if (LATENCY) load_next();
   // (staged > 0 with nothing left to walk: cells the shared phase staged; the
   // draining iteration evaluates them)
   for (;;) {  // until the stack, the bucket list and the tiles are drained
@@ -2376,10 +2397,8 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         if (lane == 0) atomicOr(status, NBSP_DEVICE_ERROR_WALK_LIMIT);
         break;
       }
-      const int take = min(32, top);
-      int node = lane < take ? stack[top - 1 - lane] : -1;
-      top -= take;
-      __syncwarp();
+      int node = next;
+      top -= min(32, top);
       bool is_leaf = false, accept = false, test = false;
       int kids = 0;
       int4 info = make_int4(0, 0, 0, 0);
@@ -2394,7 +2413,8 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         const int at = valid ? node : 0;
         // one 32-byte record: the centre of mass and mass, the opening terms,
         // and a bucket's particles or an internal node's children
-        const float4 w0 = __ldg(&t.wnode[2 * at]), w1 = __ldg(&t.wnode[2 * at + 1]);
+        const float4 w0 = LATENCY ? next0 : __ldg(&t.wnode[2 * at]);
+        const float4 w1 = LATENCY ? next1 : __ldg(&t.wnode[2 * at + 1]);
         c = w0;
         ro = w1.x;
         if (REL) km = w1.y;
@@ -2423,14 +2443,27 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       if (test) probe[lane] = make_float4(c.x, c.y, c.z, ro);
       if (REL && test) s_probe_k[wib][lane] = km;
       __syncwarp();
-      for (unsigned pend = __ballot_sync(kFull, test); pend != 0u; pend &= pend - 1u) {
-        const int from = __ffs(pend) - 1;
-        const float4 q = probe[from];
-        const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-        const bool fail = active && !opening_passes<REL>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q.w,
-                                                         REL ? s_probe_k[wib][from] : 0.f, tl);
-        const bool any = __any_sync(kFull, fail);
-        if (lane == from) accept = !any;
+      constexpr int kProbes = LATENCY ? 4 : 1;
+      for (unsigned pend = __ballot_sync(kFull, test); pend != 0u;) {
+        int from[kProbes];
+        bool fail[kProbes];
+#pragma unroll
+        for (int k = 0; k < kProbes; ++k) {  // (none left: the first one again)
+          from[k] = k == 0 || pend != 0u ? __ffs(pend) - 1 : from[0];
+          pend &= pend - 1u;
+        }
+#pragma unroll
+        for (int k = 0; k < kProbes; ++k) {
+          const float4 q = probe[from[k]];
+          const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+          fail[k] = active && !opening_passes<REL>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q.w,
+                                                   REL ? s_probe_k[wib][from[k]] : 0.f, tl);
+        }
+#pragma unroll
+        for (int k = 0; k < kProbes; ++k) {
+          const bool any = __any_sync(kFull, fail[k]);
+          if (lane == from[k]) accept = !any;
+        }
       }
       const bool open = (test || opened) && !accept;
       is_leaf = is_leaf || (open && info.z > 0);  // a failing bucket is summed exactly
@@ -2438,6 +2471,26 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       unsigned m = __ballot_sync(kFull, is_leaf);
       if (is_leaf) leaves[nleaf + __popc(m & lt)] = make_int2(info.y, info.z);
       nleaf += __popc(m);
+      // the children go onto the stack before the accepted cells are staged: the
+      // next step's nodes are then known while tiles are evaluated
+      int incl = kids;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, off);
+        if (lane >= off) incl += v;
+      }
+      const int pushed = __shfl_sync(kFull, incl, 31);
+      if (top + pushed > STACK) {
+        overflow = true;
+        break;
+      }
+      const int base = top + incl - kids;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < kids) stack[base + k] = info.y + k;
+      top += pushed;
+      __syncwarp();
+      next = lane < top ? stack[top - 1 - lane] : -1;
+      if (LATENCY) load_next();
       m = __ballot_sync(kFull, accept);
       if (ORDER == 1) {
         // A monopole cell is a point mass at its centre of mass, already in
@@ -2492,22 +2545,6 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         }
         approx += (unsigned)nacc;  // (warp-uniform; an idle lane's is dropped at the end)
       }
-      int incl = kids;
-      for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += v;
-      }
-      const int pushed = __shfl_sync(kFull, incl, 31);
-      if (top + pushed > STACK) {
-        overflow = true;
-        break;
-      }
-      const int base = top + incl - kids;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k < kids) stack[base + k] = info.y + k;
-      top += pushed;
-      __syncwarp();
     }
     const bool drain = top == 0;
     if (nleaf >= 32 || (drain && nleaf > 0)) {
@@ -2837,12 +2874,18 @@ void launch_walk(const float4* p, const float* tol, size_t n, Tree t, int order,
       NBSP_COUNT_LAUNCH(1), walk_lists_kernel<1, kListStack, false, REL, true><<<blocks, kListThreads, 0, stream>>>(
           p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none);
     } else if (order == 2) {
-      NBSP_COUNT_LAUNCH(1), walk_lists_kernel<2, kListStack, false, REL><<<blocks, kListThreads, 0, stream>>>(
-          p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none);
+      constexpr unsigned kAtOnce = 148 * list_walk_blocks<2, kListStack, false, REL, false, true>();
+      NBSP_COUNT_LAUNCH(1), (blocks <= kAtOnce ? walk_lists_kernel<2, kListStack, false, REL, false, true>
+                                               : walk_lists_kernel<2, kListStack, false, REL>)
+          <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
+                                                status, nullptr, none);
     } else {
       constexpr int kStack = REL ? kListStackRel : kListStack;
-      NBSP_COUNT_LAUNCH(1), walk_lists_kernel<1, kStack, false, REL><<<blocks, kListThreads, 0, stream>>>(
-          p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none);
+      constexpr unsigned kAtOnce = 148 * list_walk_blocks<1, kStack, false, REL, false, true>();
+      NBSP_COUNT_LAUNCH(1), (blocks <= kAtOnce ? walk_lists_kernel<1, kStack, false, REL, false, true>
+                                               : walk_lists_kernel<1, kStack, false, REL>)
+          <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
+                                                status, nullptr, none);
     }
     return;
   }
