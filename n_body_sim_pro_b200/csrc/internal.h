@@ -84,6 +84,19 @@ NBSP_HIDDEN void nbsp_allpairs_finalize(const void* partial_hi, const void* part
                                         int chunks, double gravitational_constant, double* ax,
                                         double* ay, double* az, cudaStream_t stream);
 
+/* Systems of fewer than this many particles (the autotuner's range starts here)
+ * have nbsp_allpairs_small: accelerations of the positions and masses at x, y,
+ * z, m (device addresses, also of mapped page-locked host memory) into ax, ay,
+ * az and into out_x, out_y, out_z, with the arithmetic of nbsp_allpairs_force in
+ * chunks of 256 sources.  `packed` >= n rounded up to 256 float4; *report
+ * receives the status bits.  Returns a cudaError_t. */
+#define NBSP_ALLPAIRS_SMALL 2048
+NBSP_HIDDEN int nbsp_allpairs_small(const double* x, const double* y, const double* z,
+                                    const double* m, size_t n, float softening_squared,
+                                    double gravitational_constant, void* packed, double* ax,
+                                    double* ay, double* az, double* out_x, double* out_y,
+                                    double* out_z, int* report, cudaStream_t stream);
+
 /* Kick (v += a*h) and, when `drift` is set, drift (x += v*dt) in FP64, then
  * repack the relative float4 positions.  The leapfrog/Verlet opening half. */
 NBSP_HIDDEN void nbsp_kick_drift(double* x, double* y, double* z, double* vx, double* vy,
