@@ -1,13 +1,18 @@
 // Training of the far-field correction MLP on BF16 tensor cores.
 //
-// One train-step launch processes one minibatch: every CTA owns 128 rows
-// (8 warps x 16 rows).  Forward and the activation gradients (dH2 = dY W3^T,
-// dH1 = dZ2 W2^T) run on mma.sync m16n8k16 straight from register fragments;
-// the weight gradients (dW = dZ^T H, a contraction over the 128 rows) run on
-// mma.sync as well, from BF16 copies of the activations staged in shared
-// memory.  Each CTA writes its gradient to its own slot; the Adam kernel sums
-// the slots in a fixed order (deterministic), updates the FP32 master weights
-// and a second kernel rebuilds the BF16 fragments.
+// Every CTA owns 128 rows of a minibatch (8 warps x 16 rows).  Forward and the
+// activation gradients (dH2 = dY W3^T, dH1 = dZ2 W2^T) run on mma.sync m16n8k16
+// straight from register fragments; the weight gradients (dW = dZ^T H, a
+// contraction over the 128 rows) run on mma.sync as well, from BF16 copies of
+// the activations staged in shared memory, read back as transposed fragments by
+// ldmatrix.  Each CTA writes its gradient to its own slot; the slots are summed
+// in a fixed order (deterministic) for the Adam update of the FP32 master
+// weights and of the BF16 fragments.
+//
+// A step of a small minibatch is bound by latency (1024 rows: 8 CTAs, 3e7 flop),
+// so an epoch is one cooperative launch instead of three a step: with it, the
+// ldmatrix fragments and the forward-only losses an epoch of 245,760 rows in
+// steps of 1024, its shuffle and losses included, takes 4.9 ms instead of 8.7.
 //
 // Loss: mean squared error over the 3 outputs of the standardised labels,
 // L = 1 / (3 B) sum_r sum_c (y_rc - t_rc)^2.
@@ -39,248 +44,455 @@ __device__ __forceinline__ unsigned short bf16_bits(float v) {
   return *reinterpret_cast<const unsigned short*>(&b);
 }
 
-// A fragment of the transpose of a row-major [rows][cols] BF16 matrix M:
-// A[i][k] = M[row0 + k][col0 + i]  (16 x 16 tile).
-__device__ __forceinline__ void load_at(const unsigned short* m, int cols, int row0, int col0,
+// Row strides of the staged BF16 matrices: odd multiples of 16 bytes, so that the
+// eight rows of an ldmatrix tile (and store_c's words) lie in different banks.
+constexpr int kStrideX = kInPad + 8, kStrideH = kHidden + 8, kStrideY = kOutPad;
+
+__device__ __forceinline__ uint32_t smem_address(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// A fragment of the transpose of a staged row-major matrix m, A[i][k] =
+// m[row0 + k][col0 + i] (16 x 16 tile).
+__device__ __forceinline__ void load_at(const unsigned short* m, int stride, int row0, int col0,
                                         int lane, uint32_t* a) {
-  const int g = lane >> 2, t = lane & 3;
-  auto pair = [&](int i, int k) -> uint32_t {
-    const uint32_t lo = m[(row0 + k) * cols + col0 + i];
-    const uint32_t hi = m[(row0 + k + 1) * cols + col0 + i];
-    return lo | (hi << 16);
-  };
-  a[0] = pair(g, 2 * t);
-  a[1] = pair(g + 8, 2 * t);
-  a[2] = pair(g, 2 * t + 8);
-  a[3] = pair(g + 8, 2 * t + 8);
+  // tiles in register order: (k 0-7, i 0-7), (k 0-7, i 8-15), (k 8-15, i 0-7), (k 8-15, i 8-15)
+  const int row = row0 + (lane & 7) + ((lane >> 4) << 3), col = col0 + (lane & 8);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+               : "r"(smem_address(m + row * stride + col))
+               : "memory");
 }
 
-// B fragment of a row-major [rows][cols] BF16 matrix N: B[k][n] = N[row0 + k][col0 + n].
-__device__ __forceinline__ uint2 load_b(const unsigned short* m, int cols, int row0, int col0,
+// B fragment of a staged row-major matrix m: B[k][n] = m[row0 + k][col0 + n]; for
+// an 8-column matrix also the nonzero half (i < 8) of its transpose's A fragment.
+__device__ __forceinline__ uint2 load_b(const unsigned short* m, int stride, int row0, int col0,
                                         int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  const uint32_t b0 = (uint32_t)m[(row0 + 2 * t) * cols + col0 + g] |
-                      ((uint32_t)m[(row0 + 2 * t + 1) * cols + col0 + g] << 16);
-  const uint32_t b1 = (uint32_t)m[(row0 + 2 * t + 8) * cols + col0 + g] |
-                      ((uint32_t)m[(row0 + 2 * t + 9) * cols + col0 + g] << 16);
-  return make_uint2(b0, b1);
+  uint2 b;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(b.x), "=r"(b.y)
+               : "r"(smem_address(m + (row0 + (lane & 15)) * stride + col0))
+               : "memory");
+  return b;
 }
 
-// Store a 16 x 8 C fragment (rows row0.., cols col0..) as BF16 into [rows][cols].
-__device__ __forceinline__ void store_c(unsigned short* m, int cols, int row0, int col0, int lane,
-                                        const float* c) {
+// Store a 16 x 8 C fragment (rows row0.., cols col0..) as BF16.
+__device__ __forceinline__ void store_c(unsigned short* m, int stride, int row0, int col0,
+                                        int lane, const float* c) {
   const int g = lane >> 2, t = lane & 3;
-  m[(row0 + g) * cols + col0 + 2 * t] = bf16_bits(c[0]);
-  m[(row0 + g) * cols + col0 + 2 * t + 1] = bf16_bits(c[1]);
-  m[(row0 + g + 8) * cols + col0 + 2 * t] = bf16_bits(c[2]);
-  m[(row0 + g + 8) * cols + col0 + 2 * t + 1] = bf16_bits(c[3]);
+  *reinterpret_cast<uint32_t*>(&m[(row0 + g) * stride + col0 + 2 * t]) = pack_bf16(c[0], c[1]);
+  *reinterpret_cast<uint32_t*>(&m[(row0 + g + 8) * stride + col0 + 2 * t]) = pack_bf16(c[2], c[3]);
 }
 
-struct Stage {
-  unsigned short x[kRows * kInPad];
-  unsigned short h1[kRows * kHidden];
-  unsigned short h2[kRows * kHidden];
-  unsigned short dz1[kRows * kHidden];
-  unsigned short dz2[kRows * kHidden];
-  unsigned short dy[kRows * kOutPad];
-  float db[kWarps][kHidden * 2 + kOutPad];
+struct __align__(16) Stage {
+  TrainFrags f;
+  unsigned short x[kRows * kStrideX];
+  unsigned short h1[kRows * kStrideH];
+  unsigned short h2[kRows * kStrideH];
+  unsigned short dz1[kRows * kStrideH];
+  unsigned short dz2[kRows * kStrideH];
+  unsigned short dy[kRows * kStrideY];
   float loss[kWarps];
 };
 
-// grad: [kParams] slot of this CTA.  rows_valid: rows of this CTA that exist.
-__global__ void __launch_bounds__(kRows * 2) train_step_kernel(
-    const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
-    int first_row, int rows_total, float inv_batch3, const TrainFrags* __restrict__ f,
-    float* __restrict__ grad, float* __restrict__ loss_out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Stage& st = *reinterpret_cast<Stage*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Threads of a training CTA: warps 0..7 carry the rows through the network (166
+// registers: four more warps leave them without spills, eight more do not) and
+// share the weight gradients; the last four sum the bias gradients meanwhile.
+constexpr int kTrainThreads = 384;
+// Floats per gradient slot (whole float4s).
+constexpr int kSlot = (kParams + 3) / 4 * 4;
+
+// What a lane feeds the network of its two rows: features and the standardised
+// labels of the outputs its C fragment holds.
+struct RowInputs {
+  uint32_t x[4];
+  float label[4];
+  bool v0, v1;
+};
+
+// order NULL: rows in place.
+__device__ __forceinline__ RowInputs load_rows(const uint32_t* __restrict__ x_bf16,
+                                               const float* __restrict__ y,
+                                               const int* __restrict__ order, int r0,
+                                               int rows_total, int lane) {
+  const int t = lane & 3, r1 = r0 + 8;
+  RowInputs in;
+  in.v0 = r0 < rows_total;
+  in.v1 = r1 < rows_total;
+  const int s0 = in.v0 ? (order != nullptr ? order[r0] : r0) : 0;
+  const int s1 = in.v1 ? (order != nullptr ? order[r1] : r1) : 0;
+  in.x[0] = in.v0 ? x_bf16[s0 * 8 + t] : 0u;
+  in.x[1] = in.v1 ? x_bf16[s1 * 8 + t] : 0u;
+  in.x[2] = in.v0 ? x_bf16[s0 * 8 + t + 4] : 0u;
+  in.x[3] = in.v1 ? x_bf16[s1 * 8 + t + 4] : 0u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int col = 2 * t + (q & 1);
+    in.label[q] = (q < 2 ? in.v0 : in.v1) && col < kOut ? y[(q < 2 ? s0 : s1) * 3 + col] : 0.f;
+  }
+  return in;
+}
+
+// The 16 rows of one warp through the network and, unless LOSS_ONLY, back: the
+// activations and their gradients staged for the weight gradients.  lane 0
+// leaves the rows' summed squared error in st.loss[warp].
+template <bool LOSS_ONLY>
+__device__ __forceinline__ void rows_pass(Stage& st, const RowInputs& in, int warp, int lane,
+                                          float inv_batch3) {
+  const TrainFrags& f = st.f;
   const int g = lane >> 2, t = lane & 3;
-  // rows of this warp: 16 consecutive rows of the CTA
-  const int r0 = first_row + blockIdx.x * kRows + warp * 16 + g;
-  const int r1 = r0 + 8;
-  const bool v0 = r0 < rows_total, v1 = r1 < rows_total;
-  const int s0 = v0 ? order[r0] : 0, s1 = v1 ? order[r1] : 0;
-
-  if (warp < kWarps) {
-    uint32_t xa[4];
-    xa[0] = v0 ? x_bf16[s0 * 8 + t] : 0u;
-    xa[1] = v1 ? x_bf16[s1 * 8 + t] : 0u;
-    xa[2] = v0 ? x_bf16[s0 * 8 + t + 4] : 0u;
-    xa[3] = v1 ? x_bf16[s1 * 8 + t + 4] : 0u;
-    const int lr = warp * 16;  // local row base
-    // stage X (BF16) for dW1
-    {
-      const uint32_t* xw = xa;
-      unsigned int* xs = reinterpret_cast<unsigned int*>(st.x);
-      xs[(lr + g) * 8 + t] = xw[0];
-      xs[(lr + g + 8) * 8 + t] = xw[1];
-      xs[(lr + g) * 8 + t + 4] = xw[2];
-      xs[(lr + g + 8) * 8 + t + 4] = xw[3];
-    }
-    // forward, keeping pre-activations
-    float z1[8][4], z2[8][4];
-    uint32_t h1[16], h2[16];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16(c, xa, f->w1[nt * 32 + lane]);
-      const float bb0 = f->b1[8 * nt + 2 * t], bb1 = f->b1[8 * nt + 2 * t + 1];
-      z1[nt][0] = c[0] + bb0;
-      z1[nt][1] = c[1] + bb1;
-      z1[nt][2] = c[2] + bb0;
-      z1[nt][3] = c[3] + bb1;
-      float a[4] = {gelu(z1[nt][0]), gelu(z1[nt][1]), gelu(z1[nt][2]), gelu(z1[nt][3])};
-      store_c(st.h1, kHidden, lr, 8 * nt, lane, a);
-      const int ks = nt >> 1, hi = (nt & 1) * 2;
-      h1[4 * ks + hi] = pack_bf16(a[0], a[1]);
-      h1[4 * ks + hi + 1] = pack_bf16(a[2], a[3]);
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &h1[4 * ks], f->w2[(ks * 8 + nt) * 32 + lane]);
-      const float bb0 = f->b2[8 * nt + 2 * t], bb1 = f->b2[8 * nt + 2 * t + 1];
-      z2[nt][0] = c[0] + bb0;
-      z2[nt][1] = c[1] + bb1;
-      z2[nt][2] = c[2] + bb0;
-      z2[nt][3] = c[3] + bb1;
-      float a[4] = {gelu(z2[nt][0]), gelu(z2[nt][1]), gelu(z2[nt][2]), gelu(z2[nt][3])};
-      store_c(st.h2, kHidden, lr, 8 * nt, lane, a);
-      const int ks = nt >> 1, hi = (nt & 1) * 2;
-      h2[4 * ks + hi] = pack_bf16(a[0], a[1]);
-      h2[4 * ks + hi + 1] = pack_bf16(a[2], a[3]);
-    }
-    float out[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) mma_bf16(out, &h2[4 * ks], f->w3[ks * 32 + lane]);
-    // dY = 2 (y - t) / (3 B) on the 3 real outputs of valid rows
-    float dy[4];
-    float lsum = 0.f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int col = 2 * t + (q & 1);
-      const bool row_ok = q < 2 ? v0 : v1;
-      const int s = q < 2 ? s0 : s1;
-      float d = 0.f;
-      if (row_ok && col < kOut) {
-        const float e = out[q] + f->b3[col] - y[s * 3 + col];
-        lsum += e * e;
-        d = 2.f * e * inv_batch3;
-      }
-      dy[q] = d;
-    }
-    store_c(st.dy, kOutPad, lr, 0, lane, dy);
-    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-    if (lane == 0) st.loss[warp] = lsum;
-    // dH2 = dY W3^T  (K 16 with columns 8..15 zero)
-    uint32_t dya[4] = {pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], dy[3]), 0u, 0u};
-    uint32_t dz2a[16];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16(c, dya, f->w3t[nt * 32 + lane]);
-      float d[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z2[nt][q]);
-      store_c(st.dz2, kHidden, lr, 8 * nt, lane, d);
-      const int ks = nt >> 1, hi = (nt & 1) * 2;
-      dz2a[4 * ks + hi] = pack_bf16(d[0], d[1]);
-      dz2a[4 * ks + hi + 1] = pack_bf16(d[2], d[3]);
-    }
-    // dH1 = dZ2 W2^T
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &dz2a[4 * ks], f->w2t[(ks * 8 + nt) * 32 + lane]);
-      float d[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z1[nt][q]);
-      store_c(st.dz1, kHidden, lr, 8 * nt, lane, d);
-    }
+  const int lr = warp * 16;  // local row base
+  if (!LOSS_ONLY) {  // stage X (BF16) for dW1
+    unsigned int* xs = reinterpret_cast<unsigned int*>(st.x);
+    xs[(lr + g) * (kStrideX / 2) + t] = in.x[0];
+    xs[(lr + g + 8) * (kStrideX / 2) + t] = in.x[1];
+    xs[(lr + g) * (kStrideX / 2) + t + 4] = in.x[2];
+    xs[(lr + g + 8) * (kStrideX / 2) + t + 4] = in.x[3];
   }
-  __syncthreads();
-
-  // bias gradients: column sums over the CTA's rows (threads 0..135)
-  const int tid = threadIdx.x;
-  if (tid < kHidden) {
-    float s1 = 0.f, s2 = 0.f;
-    for (int r = 0; r < kRows; ++r) {
-      __nv_bfloat16 a = *reinterpret_cast<const __nv_bfloat16*>(&st.dz1[r * kHidden + tid]);
-      __nv_bfloat16 b = *reinterpret_cast<const __nv_bfloat16*>(&st.dz2[r * kHidden + tid]);
-      s1 += __bfloat162float(a);
-      s2 += __bfloat162float(b);
-    }
-    grad[(size_t)blockIdx.x * kParams + kOffB1 + tid] = s1;
-    grad[(size_t)blockIdx.x * kParams + kOffB2 + tid] = s2;
-  } else if (tid < kHidden + kOut) {
-    const int c = tid - kHidden;
-    float s = 0.f;
-    for (int r = 0; r < kRows; ++r)
-      s += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(&st.dy[r * kOutPad + c]));
-    grad[(size_t)blockIdx.x * kParams + kOffB3 + c] = s;
-  } else if (tid == kHidden + kOut) {
-    float s = 0.f;
-    for (int w = 0; w < kWarps; ++w) s += st.loss[w];
-    loss_out[blockIdx.x] = s;
+  // forward, keeping pre-activations
+  float z1[8][4], z2[8][4];
+  uint32_t h1[16], h2[16];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(c, in.x, f.w1[nt * 32 + lane]);
+    const float bb0 = f.b1[8 * nt + 2 * t], bb1 = f.b1[8 * nt + 2 * t + 1];
+    z1[nt][0] = c[0] + bb0;
+    z1[nt][1] = c[1] + bb1;
+    z1[nt][2] = c[2] + bb0;
+    z1[nt][3] = c[3] + bb1;
+    float a[4] = {gelu(z1[nt][0]), gelu(z1[nt][1]), gelu(z1[nt][2]), gelu(z1[nt][3])};
+    if (!LOSS_ONLY) store_c(st.h1, kStrideH, lr, 8 * nt, lane, a);
+    const int ks = nt >> 1, hi = (nt & 1) * 2;
+    h1[4 * ks + hi] = pack_bf16(a[0], a[1]);
+    h1[4 * ks + hi + 1] = pack_bf16(a[2], a[3]);
   }
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &h1[4 * ks], f.w2[(ks * 8 + nt) * 32 + lane]);
+    const float bb0 = f.b2[8 * nt + 2 * t], bb1 = f.b2[8 * nt + 2 * t + 1];
+    z2[nt][0] = c[0] + bb0;
+    z2[nt][1] = c[1] + bb1;
+    z2[nt][2] = c[2] + bb0;
+    z2[nt][3] = c[3] + bb1;
+    float a[4] = {gelu(z2[nt][0]), gelu(z2[nt][1]), gelu(z2[nt][2]), gelu(z2[nt][3])};
+    if (!LOSS_ONLY) store_c(st.h2, kStrideH, lr, 8 * nt, lane, a);
+    const int ks = nt >> 1, hi = (nt & 1) * 2;
+    h2[4 * ks + hi] = pack_bf16(a[0], a[1]);
+    h2[4 * ks + hi + 1] = pack_bf16(a[2], a[3]);
+  }
+  float out[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) mma_bf16(out, &h2[4 * ks], f.w3[ks * 32 + lane]);
+  // dY = 2 (y - t) / (3 B) on the 3 real outputs of valid rows
+  float dy[4];
+  float lsum = 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int col = 2 * t + (q & 1);
+    const bool row_ok = q < 2 ? in.v0 : in.v1;
+    float d = 0.f;
+    if (row_ok && col < kOut) {
+      const float e = out[q] + f.b3[col] - in.label[q];
+      lsum += e * e;
+      d = 2.f * e * inv_batch3;
+    }
+    dy[q] = d;
+  }
+  for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+  if (lane == 0) st.loss[warp] = lsum;
+  if (LOSS_ONLY) return;
+  store_c(st.dy, kStrideY, lr, 0, lane, dy);
+  // dH2 = dY W3^T  (K 16 with columns 8..15 zero)
+  uint32_t dya[4] = {pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], dy[3]), 0u, 0u};
+  uint32_t dz2a[16];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(c, dya, f.w3t[nt * 32 + lane]);
+    float d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z2[nt][q]);
+    store_c(st.dz2, kStrideH, lr, 8 * nt, lane, d);
+    const int ks = nt >> 1, hi = (nt & 1) * 2;
+    dz2a[4 * ks + hi] = pack_bf16(d[0], d[1]);
+    dz2a[4 * ks + hi + 1] = pack_bf16(d[2], d[3]);
+  }
+  // dH1 = dZ2 W2^T
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &dz2a[4 * ks], f.w2t[(ks * 8 + nt) * 32 + lane]);
+    float d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z1[nt][q]);
+    store_c(st.dz1, kStrideH, lr, 8 * nt, lane, d);
+  }
+}
 
-  // weight gradients on tensor cores: dW = dZ^T H over the 128 rows (8 k-steps)
-  // output tiles: dW2 4 x 8 (32), dW1 4 x 2 (8), dW3 1 x 8 (8), shared by the CTA's warps
-  const int nwarps = blockDim.x >> 5;
-  for (int tile = warp; tile < 32 + 8 + 8; tile += nwarps) {
+__device__ __forceinline__ float bf16_value(unsigned short b) {
+  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(&b));
+}
+
+// After rows_pass of all 128 rows and a barrier: the CTA's gradient into its slot
+// `grad`.  Weight gradients on tensor cores, dW = dZ^T H over the 128 rows (8
+// k-steps): output tiles dW2 4 x 8 (32), dW1 4 x 2 (8), dW3 1 x 8 (8), six for
+// each of the first eight warps; the last four sum the bias columns meanwhile.
+__device__ __forceinline__ void weight_gradients(const Stage& st, int warp, int lane, int tid,
+                                                 float* __restrict__ grad) {
+  const int g = lane >> 2, t = lane & 3;
+  if (warp >= kWarps) {
+    const int c = tid - kWarps * 32;  // 0..127: columns of dZ1, then of dZ2
+    const unsigned short* m = (c < kHidden ? st.dz1 : st.dz2) + (c & (kHidden - 1));
+    float s = 0.f;
+#pragma unroll 16
+    for (int r = 0; r < kRows; ++r) s += bf16_value(m[r * kStrideH]);
+    grad[(c < kHidden ? kOffB1 : kOffB2) + (c & (kHidden - 1))] = s;
+    if (c < kOut) {
+      float sy = 0.f;
+#pragma unroll 16
+      for (int r = 0; r < kRows; ++r) sy += bf16_value(st.dy[r * kStrideY + c]);
+      grad[kOffB3 + c] = sy;
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int q = 0; q < 6; ++q) {
+    const int tile = warp + kWarps * q;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     if (tile < 32) {  // dW2[out][in] = sum_r dZ2[r][out] H1[r][in]
       const int mi = tile >> 3, nj = tile & 7;
+#pragma unroll
       for (int ks = 0; ks < kRows / 16; ++ks) {
         uint32_t a[4];
-        load_at(st.dz2, kHidden, ks * 16, mi * 16, lane, a);
-        mma_bf16(c, a, load_b(st.h1, kHidden, ks * 16, nj * 8, lane));
+        load_at(st.dz2, kStrideH, ks * 16, mi * 16, lane, a);
+        mma_bf16(c, a, load_b(st.h1, kStrideH, ks * 16, nj * 8, lane));
       }
       const int o0 = mi * 16 + g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + (size_t)blockIdx.x * kParams + kOffW2;
-      gw[o0 * kHidden + i0] = c[0];
-      gw[o0 * kHidden + i0 + 1] = c[1];
-      gw[(o0 + 8) * kHidden + i0] = c[2];
-      gw[(o0 + 8) * kHidden + i0 + 1] = c[3];
+      float* gw = grad + kOffW2;
+      *reinterpret_cast<float2*>(&gw[o0 * kHidden + i0]) = make_float2(c[0], c[1]);
+      *reinterpret_cast<float2*>(&gw[(o0 + 8) * kHidden + i0]) = make_float2(c[2], c[3]);
     } else if (tile < 40) {  // dW1[out][in] = sum_r dZ1[r][out] X[r][in], in < 10
       const int mi = (tile - 32) >> 1, nj = (tile - 32) & 1;
+#pragma unroll
       for (int ks = 0; ks < kRows / 16; ++ks) {
         uint32_t a[4];
-        load_at(st.dz1, kHidden, ks * 16, mi * 16, lane, a);
-        mma_bf16(c, a, load_b(st.x, kInPad, ks * 16, nj * 8, lane));
+        load_at(st.dz1, kStrideH, ks * 16, mi * 16, lane, a);
+        mma_bf16(c, a, load_b(st.x, kStrideX, ks * 16, nj * 8, lane));
       }
       const int o0 = mi * 16 + g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + (size_t)blockIdx.x * kParams + kOffW1;
+      float* gw = grad + kOffW1;
       if (i0 < kIn) gw[o0 * kIn + i0] = c[0], gw[(o0 + 8) * kIn + i0] = c[2];
       if (i0 + 1 < kIn) gw[o0 * kIn + i0 + 1] = c[1], gw[(o0 + 8) * kIn + i0 + 1] = c[3];
     } else {  // dW3[out][in] = sum_r dY[r][out] H2[r][in], out < 3 (M 16 from 8 padded)
       const int nj = tile - 40;
+#pragma unroll
       for (int ks = 0; ks < kRows / 16; ++ks) {
-        uint32_t a[4];
-        // A[i][k] = dY[k][i] for i < 8, zero for i >= 8
-        const int gg = lane >> 2, tt = lane & 3;
-        auto pair = [&](int i, int k) -> uint32_t {
-          if (i >= kOutPad) return 0u;
-          const uint32_t lo = st.dy[(ks * 16 + k) * kOutPad + i];
-          const uint32_t hi = st.dy[(ks * 16 + k + 1) * kOutPad + i];
-          return lo | (hi << 16);
-        };
-        a[0] = pair(gg, 2 * tt);
-        a[1] = pair(gg + 8, 2 * tt);
-        a[2] = pair(gg, 2 * tt + 8);
-        a[3] = pair(gg + 8, 2 * tt + 8);
-        mma_bf16(c, a, load_b(st.h2, kHidden, ks * 16, nj * 8, lane));
+        const uint2 y = load_b(st.dy, kStrideY, ks * 16, 0, lane);
+        const uint32_t a[4] = {y.x, 0u, y.y, 0u};  // A[i][k] = dY[k][i], zero for i >= 8
+        mma_bf16(c, a, load_b(st.h2, kStrideH, ks * 16, nj * 8, lane));
       }
       const int o0 = g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + (size_t)blockIdx.x * kParams + kOffW3;
+      float* gw = grad + kOffW3;
       if (o0 < kOut) {
         gw[o0 * kHidden + i0] = c[0];
         gw[o0 * kHidden + i0 + 1] = c[1];
       }
     }
+  }
+}
+
+__device__ __forceinline__ void copy_frags(Stage& st, const TrainFrags* f) {
+  static_assert(sizeof(TrainFrags) % 16 == 0, "copied as uint4");
+  const uint4* src = reinterpret_cast<const uint4*>(f);
+  uint4* dst = reinterpret_cast<uint4*>(&st.f);
+  for (int k = threadIdx.x; k < (int)(sizeof(TrainFrags) / 16); k += blockDim.x) dst[k] = src[k];
+}
+
+// One forward/backward: CTA c's rows first_row + 128 c .. of `order` (NULL: rows
+// in place), its gradient into slot c of grad, its loss sum into loss_out[c].
+__global__ void __launch_bounds__(kTrainThreads, 1) train_step_kernel(
+    const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
+    int first_row, int rows_total, float inv_batch3, const TrainFrags* __restrict__ f,
+    float* __restrict__ grad, float* __restrict__ loss_out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Stage& st = *reinterpret_cast<Stage*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  copy_frags(st, f);
+  RowInputs in = {};
+  if (warp < kWarps)
+    in = load_rows(x_bf16, y, order, first_row + blockIdx.x * kRows + warp * 16 + (lane >> 2),
+                   rows_total, lane);
+  __syncthreads();
+  if (warp < kWarps) rows_pass<false>(st, in, warp, lane, inv_batch3);
+  __syncthreads();
+  weight_gradients(st, warp, lane, tid, grad + (size_t)blockIdx.x * kSlot);
+  if (tid == 0) {
+    float s = 0.f;
+    for (int w = 0; w < kWarps; ++w) s += st.loss[w];
+    loss_out[blockIdx.x] = s;
+  }
+}
+
+// Summed squared errors of 128-row tiles of rows first_row.. (in place), one value
+// per tile: the forward half alone.
+__global__ void __launch_bounds__(kRows * 2) loss_kernel(
+    const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, int first_row, int tiles,
+    const TrainFrags* __restrict__ f, float* __restrict__ loss_out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Stage& st = *reinterpret_cast<Stage*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  copy_frags(st, f);
+  __syncthreads();
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const RowInputs in =
+        load_rows(x_bf16, y, nullptr, first_row + tile * kRows + warp * 16 + (lane >> 2),
+                  first_row + tiles * kRows, lane);
+    rows_pass<true>(st, in, warp, lane, 0.f);
+    __syncthreads();
+    if (tid == 0) {
+      float s = 0.f;
+      for (int w = 0; w < kWarps; ++w) s += st.loss[w];
+      loss_out[tile] = s;
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ void adam(float gsum, float& param, float& m, float& v, float lr,
+                                     float beta1, float beta2, float eps, float bias1,
+                                     float bias2) {
+  // (the fused forms are written out, so that every kernel rounds alike)
+  const float mm = __fmaf_rn(1.f - beta1, gsum, __fmul_rn(beta1, m));
+  const float vv = __fmaf_rn(__fmul_rn(1.f - beta2, gsum), gsum, __fmul_rn(beta2, v));
+  m = mm;
+  v = vv;
+  param -= lr * (mm / bias1) / (sqrtf(vv / bias2) + eps);
+}
+
+// Parameter p = value in the BF16 fragments (build_fwd and build_bwd place the
+// same elements) or the FP32 biases.
+__device__ __forceinline__ void put_fragment(uint2* frag, int ntiles, int n, int k,
+                                             unsigned short bits) {
+  const int kk = k & 15;
+  const int e = ((k >> 4) * ntiles + (n >> 3)) * 32 + (n & 7) * 4 + ((kk & 7) >> 1);
+  reinterpret_cast<unsigned short*>(&frag[e])[(kk >> 3) * 2 + (kk & 1)] = bits;
+}
+__device__ __forceinline__ void put_parameter(TrainFrags& f, int p, float value) {
+  const unsigned short bits = bf16_bits(value);
+  if (p < kOffB1) {
+    put_fragment(f.w1, 8, p / kIn, p % kIn, bits);
+  } else if (p < kOffW2) {
+    f.b1[p - kOffB1] = value;
+  } else if (p < kOffB2) {
+    const int o = (p - kOffW2) / kHidden, i = (p - kOffW2) % kHidden;
+    put_fragment(f.w2, 8, o, i, bits);
+    put_fragment(f.w2t, 8, i, o, bits);
+  } else if (p < kOffW3) {
+    f.b2[p - kOffB2] = value;
+  } else if (p < kOffB3) {
+    const int o = (p - kOffW3) / kHidden, i = (p - kOffW3) % kHidden;
+    put_fragment(f.w3, 1, o, i, bits);
+    put_fragment(f.w3t, 8, i, o, bits);
+  } else if (p < kParams) {
+    f.b3[p - kOffB3] = value;
+  }
+}
+
+// Wait until all CTAs of the launch have arrived `round` times (their writes
+// before are visible after); false when the wait ran out of its polls, and from
+// then on at once.
+constexpr int kBarrierPolls = 1 << 22;
+__device__ __forceinline__ bool grid_arrive_wait(int* arrivals, int* failed, int round, int* s_ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int seen;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(arrivals) : "memory");
+    const int target = round * (int)gridDim.x;
+    int polls = 0;
+    ++seen;
+    while (seen < target && ++polls < kBarrierPolls)
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(arrivals) : "memory");
+    if (seen < target) atomicExch(failed, 1);
+    *s_ok = seen >= target;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// All the steps of an epoch in one cooperative launch, a CTA per 128 rows of the
+// minibatch.  A step ends with every CTA summing all slots (two sets of them, by
+// the step's parity, so that one barrier a step is enough) and updating its own
+// copy of the parameters, moments and fragments — the same arithmetic on the same
+// numbers, so the copies stay equal; the first CTA stores them at the end.
+// bias: the step's 1 - beta^t for both moments.
+constexpr int kEpochCtas = 32;
+__global__ void __launch_bounds__(kTrainThreads, 1) train_epoch_kernel(
+    const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
+    int rows_total, int steps, float inv_batch3, const TrainFrags* __restrict__ f,
+    float* __restrict__ slots, float* __restrict__ params, float* __restrict__ m,
+    float* __restrict__ v, float lr, float beta1, float beta2, float eps,
+    const float2* __restrict__ bias, int* arrivals, int* failed) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Stage& st = *reinterpret_cast<Stage*>(smem_raw);
+  __shared__ int s_ok;
+  // this CTA's parameters and moments
+  float* own = reinterpret_cast<float*>(smem_raw + sizeof(Stage));
+  float *pp = own, *mm = own + kSlot, *vv = own + 2 * kSlot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ctas = gridDim.x, batch = ctas * kRows;
+  copy_frags(st, f);
+  for (int p = tid; p < kSlot; p += kTrainThreads) {
+    pp[p] = p < kParams ? params[p] : 0.f;
+    mm[p] = p < kParams ? m[p] : 0.f;
+    vv[p] = p < kParams ? v[p] : 0.f;
+  }
+  const int row = blockIdx.x * kRows + warp * 16 + (lane >> 2);
+  RowInputs in = {};
+  if (warp < kWarps) in = load_rows(x_bf16, y, order, row, rows_total, lane);
+  __syncthreads();
+  for (int step = 0; step < steps; ++step) {
+    float* set = slots + (size_t)(step & 1) * ctas * kSlot;
+    if (warp < kWarps) rows_pass<false>(st, in, warp, lane, inv_batch3);
+    __syncthreads();
+    weight_gradients(st, warp, lane, tid, set + (size_t)blockIdx.x * kSlot);
+    // the next step's rows are on their way while the CTAs wait for each other
+    if (warp < kWarps && step + 1 < steps)
+      in = load_rows(x_bf16, y, order, (step + 1) * batch + row, rows_total, lane);
+    const float2 b = bias[step];
+    if (!grid_arrive_wait(arrivals, failed, step + 1, &s_ok)) return;
+    for (int group = tid; group < kSlot / 4; group += kTrainThreads) {
+      float gsum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+      for (int s = 0; s < ctas; ++s) {
+        const float4 d = __ldcg(reinterpret_cast<const float4*>(set + (size_t)s * kSlot) + group);
+        gsum[0] += d.x;
+        gsum[1] += d.y;
+        gsum[2] += d.z;
+        gsum[3] += d.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int p = 4 * group + e;
+        if (p >= kParams) continue;
+        float value = pp[p], mp = mm[p], vp = vv[p];
+        adam(gsum[e], value, mp, vp, lr, beta1, beta2, eps, b.x, b.y);
+        pp[p] = value;
+        mm[p] = mp;
+        vv[p] = vp;
+        put_parameter(st.f, p, value);
+      }
+    }
+    __syncthreads();
+  }
+  if (blockIdx.x != 0) return;
+  for (int p = tid; p < kParams; p += kTrainThreads) {
+    params[p] = pp[p];
+    m[p] = mm[p];
+    v[p] = vv[p];
   }
 }
 
@@ -293,14 +505,10 @@ __global__ void reduce_adam_kernel(const float* __restrict__ partial, int slots,
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kParams) return;
   float gsum = 0.f;
-  for (int s = 0; s < slots; ++s) gsum += partial[(size_t)s * kParams + p];
+  for (int s = 0; s < slots; ++s) gsum += partial[(size_t)s * kSlot + p];
   if (grad_out != nullptr) grad_out[p] = gsum;
   if (!apply) return;
-  const float mm = beta1 * m[p] + (1.f - beta1) * gsum;
-  const float vv = beta2 * v[p] + (1.f - beta2) * gsum * gsum;
-  m[p] = mm;
-  v[p] = vv;
-  params[p] -= lr * (mm / bias1) / (sqrtf(vv / bias2) + eps);
+  adam(gsum, params[p], m[p], v[p], lr, beta1, beta2, eps, bias1, bias2);
 }
 
 __device__ __forceinline__ float w_at(const float* w, int out, int in, int outs, int ins) {
@@ -454,6 +662,8 @@ void nbsp_mlp_get_scaling(const void* net, float* table, cudaStream_t stream) {
 size_t nbsp_mlp_frags_bytes(void) { return sizeof(TrainFrags); }
 int nbsp_mlp_param_count(void) { return kParams; }
 int nbsp_mlp_rows_per_cta(void) { return kRows; }
+int nbsp_mlp_slot_floats(void) { return kSlot; }
+int nbsp_mlp_epoch_ctas(void) { return kEpochCtas; }
 
 void nbsp_mlp_build_frags(const float* params, void* frags, void* net, cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), build_frags_kernel<<<1, 256, 0, stream>>>(params, (TrainFrags*)frags,
@@ -466,15 +676,56 @@ void nbsp_mlp_standardise(const float* feat, const float* lab, int rows, const v
       feat, lab, rows, (const Net*)net, x, y);
 }
 
-// One forward/backward over rows [first_row, first_row + ctas * 128) of `order`;
-// per-CTA gradients into partial[ctas][params], per-CTA loss sums into loss.
+// One forward/backward over rows [first_row, first_row + ctas * 128) of `order`
+// (NULL: rows in place); per-CTA gradients into partial[ctas][slot floats],
+// per-CTA loss sums into loss.
 void nbsp_mlp_train_step(const uint32_t* x, const float* y, const int* order, int first_row,
                          int rows_total, int ctas, float inv_batch3, const void* frags,
                          float* partial, float* loss, cudaStream_t stream) {
   const int smem = (int)sizeof(Stage);
   cudaFuncSetAttribute(train_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  NBSP_COUNT_LAUNCH(1), train_step_kernel<<<ctas, kRows * 2, smem, stream>>>(
+  NBSP_COUNT_LAUNCH(1), train_step_kernel<<<ctas, kTrainThreads, smem, stream>>>(
       x, y, order, first_row, rows_total, inv_batch3, (const TrainFrags*)frags, partial, loss);
+}
+
+// The loss sums of `tiles` 128-row tiles from first_row on, in place.
+void nbsp_mlp_loss(const uint32_t* x, const float* y, int first_row, int tiles, const void* frags,
+                   float* loss, cudaStream_t stream) {
+  const int smem = (int)sizeof(Stage);
+  cudaFuncSetAttribute(loss_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int grid = tiles < 2 * 148 ? tiles : 2 * 148;  // two CTAs of ~105 KB per SM
+  NBSP_COUNT_LAUNCH(1), loss_kernel<<<grid, kRows * 2, smem, stream>>>(
+      x, y, first_row, tiles, (const TrainFrags*)frags, loss);
+}
+
+static const float kBeta1 = 0.9f, kBeta2 = 0.999f, kAdamEps = 1e-8f;
+
+// 1 - beta^step of both moments.
+void nbsp_mlp_adam_bias(int step, float* bias) {
+  bias[0] = 1.f - powf(kBeta1, (float)step);
+  bias[1] = 1.f - powf(kBeta2, (float)step);
+}
+
+// `steps` minibatches of ctas * 128 rows of `order` from its start, forward,
+// backward and Adam, in one launch (ctas <= nbsp_mlp_epoch_ctas()); slots: two
+// sets of ctas gradient slots; bias: steps pairs of nbsp_mlp_adam_bias on the
+// device; sync: two zeroed ints, the second nonzero when a wait ran out.  The
+// fragments in `frags` and the inference network are not touched.
+int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order, int rows_total,
+                         int steps, int ctas, float inv_batch3, const void* frags, float* slots,
+                         float* params, float* m, float* v, float lr, const void* bias, int* sync,
+                         cudaStream_t stream) {
+  const int smem = (int)(sizeof(Stage) + 3 * kSlot * sizeof(float));
+  cudaFuncSetAttribute(train_epoch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const TrainFrags* f = (const TrainFrags*)frags;
+  const float2* b = (const float2*)bias;
+  float beta1 = kBeta1, beta2 = kBeta2, eps = kAdamEps;
+  int* failed = sync + 1;
+  void* args[] = {&x, &y, &order, &rows_total, &steps, &inv_batch3, &f, &slots, &params, &m, &v,
+                  &lr, &beta1, &beta2, &eps, &b, &sync, &failed};
+  NBSP_COUNT_LAUNCH(1);
+  return (int)cudaLaunchCooperativeKernel((const void*)train_epoch_kernel, dim3((unsigned)ctas),
+                                          dim3(kTrainThreads), args, (size_t)smem, stream);
 }
 
 void nbsp_mlp_evaluate(const void* net, const float* feat, int rows, float* out, int tcgen05,
@@ -497,10 +748,10 @@ void nbsp_mlp_evaluate(const void* net, const float* feat, int rows, float* out,
 
 void nbsp_mlp_reduce_adam(const float* partial, int slots, float* grad_out, float* params, float* m,
                           float* v, float lr, int step, int apply, cudaStream_t stream) {
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float bias1 = 1.f - powf(b1, (float)step), bias2 = 1.f - powf(b2, (float)step);
+  float bias[2];
+  nbsp_mlp_adam_bias(step, bias);
   NBSP_COUNT_LAUNCH(1), reduce_adam_kernel<<<(kParams + 255) / 256, 256, 0, stream>>>(
-      partial, slots, grad_out, params, m, v, lr, b1, b2, 1e-8f, bias1, bias2, apply);
+      partial, slots, grad_out, params, m, v, lr, kBeta1, kBeta2, kAdamEps, bias[0], bias[1], apply);
 }
 
 }  // extern "C"

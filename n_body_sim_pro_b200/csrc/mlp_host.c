@@ -32,6 +32,16 @@ NBSP_HIDDEN void nbsp_mlp_train_step(const uint32_t* x, const float* y, const in
                                      int first_row, int rows_total, int ctas, float inv_batch3,
                                      const void* frags, float* partial, float* loss,
                                      cudaStream_t stream);
+NBSP_HIDDEN int nbsp_mlp_slot_floats(void);
+NBSP_HIDDEN int nbsp_mlp_epoch_ctas(void);
+NBSP_HIDDEN void nbsp_mlp_loss(const uint32_t* x, const float* y, int first_row, int tiles,
+                               const void* frags, float* loss, cudaStream_t stream);
+NBSP_HIDDEN void nbsp_mlp_adam_bias(int step, float* bias);
+NBSP_HIDDEN int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order,
+                                     int rows_total, int steps, int ctas, float inv_batch3,
+                                     const void* frags, float* slots, float* params, float* m,
+                                     float* v, float lr, const void* bias, int* sync,
+                                     cudaStream_t stream);
 NBSP_HIDDEN void nbsp_mlp_reduce_adam(const float* partial, int slots, float* grad_out,
                                       float* params, float* m, float* v, float lr, int step,
                                       int apply, cudaStream_t stream);
@@ -52,6 +62,9 @@ struct NBodySimProCudaCorrection {
     float* loss;            /* per-CTA loss sums */
     float* grad;            /* reduced gradient */
     int slots;
+    float* bias;            /* per step of an epoch, 1 - beta^t of both moments */
+    int* sync;              /* the epoch kernel's arrivals and failure flag */
+    int bias_steps;
     uint32_t* x;            /* standardised BF16 features, 8 words per row */
     float* y;               /* standardised labels */
     float* feat;            /* raw features of the kept rows */
@@ -117,7 +130,8 @@ void n_body_sim_pro_cuda_correction_destroy(NBodySimProCudaCorrection* c) {
     cudaSetDevice(c->device);
     if (c->stream != NULL) cudaStreamSynchronize(c->stream);
     free_data(c);
-    void* p[] = {c->params, c->m, c->v, c->frags, c->net, c->partial, c->loss, c->grad};
+    void* p[] = {c->params, c->m, c->v, c->frags, c->net, c->partial, c->loss, c->grad,
+                 c->bias, c->sync};
     for (size_t k = 0; k < sizeof(p) / sizeof(p[0]); ++k) cudaFree(p[k]);
     cudaFreeHost(c->host_loss);
     if (c->stream != NULL) cudaStreamDestroy(c->stream);
@@ -185,6 +199,7 @@ NBodySimProCudaCorrection* n_body_sim_pro_cuda_correction_create(uint64_t seed,
     if (code == cudaSuccess) code = cudaMalloc((void**)&c->grad, np * sizeof(float));
     if (code == cudaSuccess) code = cudaMalloc(&c->frags, nbsp_mlp_frags_bytes());
     if (code == cudaSuccess) code = cudaMalloc(&c->net, nbsp_mlp_net_bytes());
+    if (code == cudaSuccess) code = cudaMalloc((void**)&c->sync, 2 * sizeof(int));
     if (code == cudaSuccess) code = cudaMallocHost((void**)&c->host_loss, 1 << 20);
     if (code != cudaSuccess) {
         mcuda(error, code, __LINE__, "correction set-up");
@@ -210,7 +225,7 @@ static NBodySimProStatus ensure_slots(NBodySimProCudaCorrection* c, int slots,
     c->partial = NULL;
     c->loss = NULL;
     c->slots = 0;
-    MTRY(cudaMalloc((void**)&c->partial, (size_t)slots * nbsp_mlp_param_count() * sizeof(float)));
+    MTRY(cudaMalloc((void**)&c->partial, (size_t)slots * nbsp_mlp_slot_floats() * sizeof(float)));
     MTRY(cudaMalloc((void**)&c->loss, (size_t)slots * sizeof(float)));
     c->slots = slots;
     return N_BODY_SIM_PRO_STATUS_OK;
@@ -309,7 +324,7 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_generate(NBodySimProCudaCorrect
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
-/* Mean loss over rows [first, first + count) in identity order (no update). */
+/* Mean loss over rows [first, first + count), in place (no update). */
 static NBodySimProStatus evaluate(NBodySimProCudaCorrection* c, size_t first, size_t count,
                                   double* loss, NBodySimProError* error) {
     const int per = nbsp_mlp_rows_per_cta();
@@ -320,19 +335,12 @@ static NBodySimProStatus evaluate(NBodySimProCudaCorrection* c, size_t first, si
     }
     NBodySimProStatus st = ensure_slots(c, ctas, error);
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
-    int* ident = (int*)malloc(count * sizeof(int));
-    if (ident == NULL) return mfail(error, N_BODY_SIM_PRO_STATUS_OUT_OF_MEMORY, __LINE__, "order");
-    for (size_t r = 0; r < count; ++r) ident[r] = (int)(first + r);
-    cudaError_t code = cudaMemcpyAsync(c->order, ident, count * sizeof(int), cudaMemcpyHostToDevice,
-                                       c->stream);
-    if (code == cudaSuccess) {
-        nbsp_mlp_train_step(c->x, c->y, c->order, 0, (int)count, ctas, 1.f / (3.f * (float)count),
-                            c->frags, c->partial, c->loss, c->stream);
+    nbsp_mlp_loss(c->x, c->y, (int)first, ctas, c->frags, c->loss, c->stream);
+    cudaError_t code = cudaGetLastError();
+    if (code == cudaSuccess)
         code = cudaMemcpyAsync(c->host_loss, c->loss, (size_t)ctas * sizeof(float),
                                cudaMemcpyDeviceToHost, c->stream);
-    }
     if (code == cudaSuccess) code = cudaStreamSynchronize(c->stream);
-    free(ident);
     if (code != cudaSuccess) return mcuda(error, code, __LINE__, "evaluation");
     double s = 0.0;
     for (int k = 0; k < ctas; ++k) s += c->host_loss[k];
@@ -353,11 +361,26 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
                      "no training set: call n_body_sim_pro_cuda_correction_generate first");
     MTRY(cudaSetDevice(c->device));
     const int ctas = batch / per;
-    NBodySimProStatus st = ensure_slots(c, ctas, error);
-    if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     const size_t n = c->train_rows;
+    const int steps = (int)(n / (size_t)batch);
+    /* an epoch in one cooperative launch, up to the minibatch its blocks sum */
+    const int one_launch = ctas <= nbsp_mlp_epoch_ctas() && steps > 0;
+    NBodySimProStatus st = ensure_slots(c, one_launch ? 2 * ctas : ctas, error);
+    if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
+    if (one_launch && steps > c->bias_steps) {
+        cudaFree(c->bias);
+        c->bias = NULL;
+        c->bias_steps = 0;
+        MTRY(cudaMalloc((void**)&c->bias, 2 * (size_t)steps * sizeof(float)));
+        c->bias_steps = steps;
+    }
     int* order = (int*)malloc(n * sizeof(int));
-    if (order == NULL) return mfail(error, N_BODY_SIM_PRO_STATUS_OUT_OF_MEMORY, __LINE__, "order");
+    float* bias = (float*)malloc((2 * (size_t)steps + 1) * sizeof(float));
+    if (order == NULL || bias == NULL) {
+        free(order);
+        free(bias);
+        return mfail(error, N_BODY_SIM_PRO_STATUS_OUT_OF_MEMORY, __LINE__, "order");
+    }
     uint64_t s = c->seed ^ 0x5DEECE66Dull;
     for (int epoch = 0; epoch < epochs; ++epoch) {
         for (size_t r = 0; r < n; ++r) order[r] = (int)r;
@@ -369,18 +392,47 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
         }
         cudaError_t code = cudaMemcpyAsync(c->order, order, n * sizeof(int), cudaMemcpyHostToDevice,
                                            c->stream);
-        for (size_t first = 0; code == cudaSuccess && first + (size_t)batch <= n; first += batch) {
-            nbsp_mlp_train_step(c->x, c->y, c->order, (int)first, (int)n, ctas,
-                                1.f / (3.f * (float)batch), c->frags, c->partial, c->loss,
-                                c->stream);
+        const float inv_batch3 = 1.f / (3.f * (float)batch);
+        int failed = 0;
+        if (one_launch) {
+            for (int k = 0; k < steps; ++k) nbsp_mlp_adam_bias(c->adam_step + 1 + k, bias + 2 * k);
+            if (code == cudaSuccess)
+                code = cudaMemcpyAsync(c->bias, bias, 2 * (size_t)steps * sizeof(float),
+                                       cudaMemcpyHostToDevice, c->stream);
+            if (code == cudaSuccess) code = cudaMemsetAsync(c->sync, 0, 2 * sizeof(int), c->stream);
+            if (code == cudaSuccess)
+                code = (cudaError_t)nbsp_mlp_train_epoch(
+                    c->x, c->y, c->order, (int)n, steps, ctas, inv_batch3, c->frags, c->partial,
+                    c->params, c->m, c->v, (float)learning_rate, c->bias, c->sync, c->stream);
+            if (code == cudaSuccess) {
+                c->adam_step += steps;
+                nbsp_mlp_build_frags(c->params, c->frags, c->net, c->stream);
+                code = cudaGetLastError();
+            }
+            if (code == cudaSuccess)
+                code = cudaMemcpyAsync(c->host_loss, c->sync + 1, sizeof(int),
+                                       cudaMemcpyDeviceToHost, c->stream);
+        }
+        for (size_t first = 0; !one_launch && code == cudaSuccess && first + (size_t)batch <= n;
+             first += batch) {
+            nbsp_mlp_train_step(c->x, c->y, c->order, (int)first, (int)n, ctas, inv_batch3,
+                                c->frags, c->partial, c->loss, c->stream);
             nbsp_mlp_reduce_adam(c->partial, ctas, NULL, c->params, c->m, c->v,
                                  (float)learning_rate, ++c->adam_step, 1, c->stream);
             nbsp_mlp_build_frags(c->params, c->frags, c->net, c->stream);
             code = cudaGetLastError();
         }
         if (code == cudaSuccess) code = cudaStreamSynchronize(c->stream);
+        if (code == cudaSuccess && one_launch) memcpy(&failed, c->host_loss, sizeof(failed));
+        if (failed) {
+            free(order);
+            free(bias);
+            return mfail(error, N_BODY_SIM_PRO_STATUS_INVALID_STATE, __LINE__,
+                         "training: the thread blocks' wait for one another ran out");
+        }
         if (code != cudaSuccess) {
             free(order);
+            free(bias);
             return mcuda(error, code, __LINE__, "training step");
         }
         double tl = 0.0, vl = 0.0;
@@ -392,6 +444,7 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
         if (validation_loss != NULL) validation_loss[epoch] = vl;
     }
     free(order);
+    free(bias);
     return st;
 }
 
