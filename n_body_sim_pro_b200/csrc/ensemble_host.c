@@ -21,25 +21,27 @@
 #include <string.h>
 
 /* ensemble.cu launchers */
-NBSP_HIDDEN int nbsp_ensemble_shape_supported(int block, int per_thread);
-NBSP_HIDDEN int nbsp_ensemble_resident_ctas(int block, int per_thread);
-NBSP_HIDDEN void nbsp_ensemble_advance(int block, int per_thread, int grid, double* x, double* y,
-                                       double* z, double* vx, double* vy, double* vz, double* ax,
-                                       double* ay, double* az, const double* m,
-                                       const long long* offset, const double* centre,
-                                       const int* item_start, const int* item_systems,
-                                       const int* item_group, int items, int* counter,
+NBSP_HIDDEN int nbsp_ensemble_resident_ctas(int block);
+NBSP_HIDDEN void nbsp_ensemble_advance(int block, int grid, double* x, double* y, double* z,
+                                       double* vx, double* vy, double* vz, double* ax, double* ay,
+                                       double* az, const double* m, const long long* offset,
+                                       const double* centre, const int* item_start,
+                                       const int* item_systems, const int* item_slot,
+                                       const int* item_warps, int items, int* counter,
                                        int* status, double g, float eps2, double dt, int steps,
                                        int guard, cudaStream_t stream);
 
-enum { ENS_MAX_SYSTEM = 4096, ENS_SHAPES = 3, ENS_TILE = 64 /* = kTile in ensemble.cu */ };
+enum { ENS_MAX_SYSTEM = 4096, ENS_SHAPES = 3, ENS_TILE = 64 /* = kTile in ensemble.cu */,
+       ENS_TILES = ENS_MAX_SYSTEM / ENS_TILE /* tiles of a CTA's particle slots */ };
 
-static const int kEnsShapes[ENS_SHAPES][2] = {{512, 8}, {1024, 4}, {256, 16}};
+/* threads per CTA; targets per thread of a system that fills the CTA's slots */
+static const int kEnsShapes[ENS_SHAPES][2] = {{1024, 4}, {768, 6}, {512, 8}};
 
 typedef struct Items {
     int* start;    /* host [items + 1] */
     int* systems;  /* host [systems] */
-    int* group;    /* host [items] */
+    int* slot;     /* host [systems], parallel to systems */
+    int* warps;    /* host [items] */
     int count;
 } Items;
 
@@ -52,7 +54,7 @@ struct NBodySimProCudaEnsemble {
     double max_mass; /* largest |m|: decides whether the self pair needs a guard */
     long long* offset;      /* device */
     long long* host_offset; /* host */
-    int *d_item_start, *d_item_systems, *d_item_group;
+    int *d_item_start, *d_item_systems, *d_item_slot, *d_item_warps;
     int items;
     int *counter, *status, *host_status;
     int block, per_thread, grid, tuned;
@@ -104,12 +106,13 @@ static void release_graph(NBodySimProCudaEnsemble* e) {
 
 static void release_data(NBodySimProCudaEnsemble* e) {
     void* p[] = {e->x, e->y, e->z, e->vx, e->vy, e->vz, e->ax, e->ay, e->az, e->m, e->centre,
-                 e->offset, e->d_item_start, e->d_item_systems, e->d_item_group, e->packed,
+                 e->offset, e->d_item_start, e->d_item_systems, e->d_item_slot, e->d_item_warps,
+                 e->packed,
                  e->hi, e->lo};
     for (size_t k = 0; k < sizeof(p) / sizeof(p[0]); ++k) cudaFree(p[k]);
     e->x = e->y = e->z = e->vx = e->vy = e->vz = e->ax = e->ay = e->az = e->m = e->centre = NULL;
     e->offset = NULL;
-    e->d_item_start = e->d_item_systems = e->d_item_group = NULL;
+    e->d_item_start = e->d_item_systems = e->d_item_slot = e->d_item_warps = NULL;
     e->packed = e->hi = e->lo = NULL;
     free(e->host_offset);
     e->host_offset = NULL;
@@ -175,12 +178,6 @@ void n_body_sim_pro_cuda_ensemble_destroy(NBodySimProCudaEnsemble* e) {
     free(e);
 }
 
-static unsigned next_pow2(unsigned v) {
-    unsigned p = 32;
-    while (p < v) p <<= 1;
-    return p;
-}
-
 typedef struct SortKey {
     long long cost;
     int index;
@@ -193,32 +190,23 @@ static int by_cost_desc(const void* a, const void* b) {
     return x->index - y->index;
 }
 
-/* Threads of the subgroup that owns a system of n particles: the kernel pads
- * each system to whole tiles of ENS_TILE sources (ensemble.cu kTile), and the
- * subgroup's G * k shared-memory slots must hold the padded system.  G is the
- * smallest whole number of warps that does (a power of two below one warp, so
- * subgroups never straddle a warp boundary): every thread slot beyond the
- * system's particles still runs the force loop, so a power-of-two G would
- * waste up to half of the work of the largest systems. */
-static int group_threads(long long n, int k) {
-    const long long padded = (n + ENS_TILE - 1) / ENS_TILE * ENS_TILE;
-    const long long need = (padded + k - 1) / k;
-    if (need < 32) return (int)next_pow2((unsigned)need);
-    return (int)((need + 31) / 32 * 32);
-}
+static int tiles_of(long long n) { return (int)((n + ENS_TILE - 1) / ENS_TILE); }
 
-/* Bundle systems into work items for threads-per-CTA `block` and `k` targets
- * per thread; items ordered by cost (sum n^2), largest first. */
-static int build_items(const long long* off, size_t systems, int block, int k, Items* out) {
+/* Bundle systems into work items for CTAs of `block` threads, on `sm_count` SMs;
+ * items ordered by their time, longest first. */
+static int build_items(const long long* off, size_t systems, int block, int sm_count, Items* out) {
+    const int cta_warps = block / 32;
     SortKey* order = (SortKey*)malloc(systems * sizeof(SortKey));
+    SortKey* io = (SortKey*)malloc(systems * sizeof(SortKey)); /* at most one item a system */
+    int* tmp_start = (int*)malloc((systems + 1) * sizeof(int));
+    int* tmp_warps = (int*)malloc(systems * sizeof(int));
     int* start = (int*)malloc((systems + 1) * sizeof(int));
     int* list = (int*)malloc(systems * sizeof(int));
-    int* group = (int*)malloc(systems * sizeof(int));
-    long long* cost = (long long*)malloc(systems * sizeof(long long));
-    int* tmp_start = (int*)malloc((systems + 1) * sizeof(int));
-    int* tmp_group = (int*)malloc(systems * sizeof(int));
-    if (!order || !start || !list || !group || !cost || !tmp_start || !tmp_group) {
-        free(order); free(start); free(list); free(group); free(cost); free(tmp_start); free(tmp_group);
+    int* slot = (int*)malloc(systems * sizeof(int));
+    int* warps = (int*)malloc(systems * sizeof(int));
+    if (!order || !io || !tmp_start || !tmp_warps || !start || !list || !slot || !warps) {
+        free(order); free(io); free(tmp_start); free(tmp_warps);
+        free(start); free(list); free(slot); free(warps);
         return 1;
     }
     for (size_t s = 0; s < systems; ++s) {
@@ -226,55 +214,53 @@ static int build_items(const long long* off, size_t systems, int block, int k, I
         order[s].index = (int)s;
     }
     qsort(order, systems, sizeof(SortKey), by_cost_desc); /* largest systems first */
-    /* greedy bundling: consecutive systems of one size class share an item */
+    /* Greedy bundling of consecutive systems: as many as the CTA has slots and
+     * warps for, no more than leave every SM an item, and none smaller than 7/8
+     * of the first (an item's step lasts as long as its largest system's).  Each
+     * gets an equal share of the warps, no more than it has tiles. */
+    const size_t share = (systems + (size_t)sm_count - 1) / (size_t)sm_count;
     int items = 0;
-    size_t s = 0;
-    int* cursor = list;
-    while (s < systems) {
-        const long long n = order[s].cost;
-        const int g = group_threads(n, k);
-        const int per_item = block / g;
-        tmp_start[items] = (int)(cursor - list);
-        tmp_group[items] = g;
-        long long c = 0;
-        int taken = 0;
-        while (s < systems && taken < per_item) {
-            const long long m = order[s].cost;
-            if (group_threads(m, k) != g) break;
-            *cursor++ = order[s].index;
-            c += m * m;
+    for (size_t s = 0; s < systems;) {
+        const int largest = tiles_of(order[s].cost);
+        size_t taken = 0;
+        int smallest = largest, used = 0;
+        tmp_start[items] = (int)s;
+        while (s < systems && taken < (size_t)cta_warps && taken < share) {
+            const int t = tiles_of(order[s].cost);
+            if (used + t > ENS_TILES || 8 * t < 7 * largest) break;
+            used += t;
+            smallest = t;
             ++taken;
             ++s;
         }
-        cost[items] = c;
+        int w = cta_warps / (int)taken;
+        if (w > smallest) w = smallest;
+        tmp_warps[items] = w;
+        io[items].cost = (long long)largest * largest * ENS_TILE / w;
+        io[items].index = items;
         ++items;
     }
-    tmp_start[items] = (int)(cursor - list);
-    /* order items by cost (longest processing time first) */
-    SortKey* io = (SortKey*)malloc((size_t)items * sizeof(SortKey));
-    int* list2 = (int*)malloc(systems * sizeof(int));
-    if (!io || !list2) {
-        free(io); free(list2); free(order); free(start); free(list); free(group); free(cost);
-        free(tmp_start); free(tmp_group);
-        return 1;
-    }
-    for (int i = 0; i < items; ++i) {
-        io[i].cost = cost[i];
-        io[i].index = i;
-    }
+    tmp_start[items] = (int)systems;
+    /* order items by time (longest processing time first) */
     qsort(io, (size_t)items, sizeof(SortKey), by_cost_desc);
-    int pos = 0;
+    int at = 0;
     for (int i = 0; i < items; ++i) {
         const int src = io[i].index;
-        start[i] = pos;
-        group[i] = tmp_group[src];
-        for (int q = tmp_start[src]; q < tmp_start[src + 1]; ++q) list2[pos++] = list[q];
+        start[i] = at;
+        warps[i] = tmp_warps[src];
+        int used = 0;
+        for (int q = tmp_start[src]; q < tmp_start[src + 1]; ++q) {
+            list[at] = order[q].index;
+            slot[at++] = used * ENS_TILE;
+            used += tiles_of(order[q].cost);
+        }
     }
-    start[items] = pos;
-    free(io); free(order); free(list); free(cost); free(tmp_start); free(tmp_group);
+    start[items] = at;
+    free(order); free(io); free(tmp_start); free(tmp_warps);
     out->start = start;
-    out->systems = list2;
-    out->group = group;
+    out->systems = list;
+    out->slot = slot;
+    out->warps = warps;
     out->count = items;
     return 0;
 }
@@ -282,22 +268,25 @@ static int build_items(const long long* off, size_t systems, int block, int k, I
 static void free_items(Items* it) {
     free(it->start);
     free(it->systems);
-    free(it->group);
+    free(it->slot);
+    free(it->warps);
     memset(it, 0, sizeof(*it));
 }
 
 static NBodySimProStatus load_items(NBodySimProCudaEnsemble* e, int block, int k,
                                     NBodySimProError* error) {
     Items it;
-    if (build_items(e->host_offset, e->systems, block, k, &it))
+    if (build_items(e->host_offset, e->systems, block, e->sm_count, &it))
         return efail(error, N_BODY_SIM_PRO_STATUS_OUT_OF_MEMORY, __LINE__, "work items");
     cudaFree(e->d_item_start);
     cudaFree(e->d_item_systems);
-    cudaFree(e->d_item_group);
-    e->d_item_start = e->d_item_systems = e->d_item_group = NULL;
+    cudaFree(e->d_item_slot);
+    cudaFree(e->d_item_warps);
+    e->d_item_start = e->d_item_systems = e->d_item_slot = e->d_item_warps = NULL;
     cudaError_t code = cudaMalloc((void**)&e->d_item_start, (size_t)(it.count + 1) * sizeof(int));
     if (code == cudaSuccess) code = cudaMalloc((void**)&e->d_item_systems, e->systems * sizeof(int));
-    if (code == cudaSuccess) code = cudaMalloc((void**)&e->d_item_group, (size_t)it.count * sizeof(int));
+    if (code == cudaSuccess) code = cudaMalloc((void**)&e->d_item_slot, e->systems * sizeof(int));
+    if (code == cudaSuccess) code = cudaMalloc((void**)&e->d_item_warps, (size_t)it.count * sizeof(int));
     if (code == cudaSuccess)
         code = cudaMemcpy(e->d_item_start, it.start, (size_t)(it.count + 1) * sizeof(int),
                           cudaMemcpyHostToDevice);
@@ -305,12 +294,15 @@ static NBodySimProStatus load_items(NBodySimProCudaEnsemble* e, int block, int k
         code = cudaMemcpy(e->d_item_systems, it.systems, e->systems * sizeof(int),
                           cudaMemcpyHostToDevice);
     if (code == cudaSuccess)
-        code = cudaMemcpy(e->d_item_group, it.group, (size_t)it.count * sizeof(int),
+        code = cudaMemcpy(e->d_item_slot, it.slot, e->systems * sizeof(int),
+                          cudaMemcpyHostToDevice);
+    if (code == cudaSuccess)
+        code = cudaMemcpy(e->d_item_warps, it.warps, (size_t)it.count * sizeof(int),
                           cudaMemcpyHostToDevice);
     e->items = it.count;
     free_items(&it);
     if (code != cudaSuccess) return ecuda(error, code, __LINE__, "work item upload");
-    const int resident = nbsp_ensemble_resident_ctas(block, k);
+    const int resident = nbsp_ensemble_resident_ctas(block);
     e->block = block;
     e->per_thread = k;
     e->grid = e->sm_count * (resident > 0 ? resident : 1);
@@ -425,9 +417,9 @@ static int self_pair_needs_guard(const NBodySimProCudaEnsemble* e, float eps2) {
 static void enqueue_persistent(NBodySimProCudaEnsemble* e, double g, float eps2, double dt,
                                int steps) {
     cudaMemsetAsync(e->counter, 0, sizeof(int), e->stream);
-    nbsp_ensemble_advance(e->block, e->per_thread, e->grid, e->x, e->y, e->z, e->vx, e->vy, e->vz,
-                          e->ax, e->ay, e->az, e->m, e->offset, e->centre, e->d_item_start,
-                          e->d_item_systems, e->d_item_group, e->items, e->counter, e->status, g,
+    nbsp_ensemble_advance(e->block, e->grid, e->x, e->y, e->z, e->vx, e->vy, e->vz, e->ax, e->ay,
+                          e->az, e->m, e->offset, e->centre, e->d_item_start, e->d_item_systems,
+                          e->d_item_slot, e->d_item_warps, e->items, e->counter, e->status, g,
                           eps2, dt, steps, self_pair_needs_guard(e, eps2), e->stream);
 }
 
@@ -498,7 +490,6 @@ NBodySimProStatus n_body_sim_pro_cuda_ensemble_autotune(NBodySimProCudaEnsemble*
     float best_ms = 0.f;
     NBodySimProStatus st = N_BODY_SIM_PRO_STATUS_OK;
     for (int s = 0; s < ENS_SHAPES && st == N_BODY_SIM_PRO_STATUS_OK; ++s) {
-        if (!nbsp_ensemble_shape_supported(kEnsShapes[s][0], kEnsShapes[s][1])) continue;
         st = load_items(e, kEnsShapes[s][0], kEnsShapes[s][1], error);
         if (st != N_BODY_SIM_PRO_STATUS_OK) break;
         cudaEventRecord(e->ev[0], e->stream);
