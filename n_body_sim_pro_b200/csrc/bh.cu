@@ -1264,19 +1264,35 @@ struct Opening {
   int criterion;         // NBSP_BH_OPENING_*
 };
 
+// The same once a thread has read the geometry: the climb's acquires would have
+// every node read it again.
+struct OpeningTerms {
+  double root_side;
+  double it, it2;  // 1 / theta and its square, at the angle in force
+};
+__device__ __forceinline__ OpeningTerms opening_terms(const Opening& o) {
+  // Without previous accelerations every target's relative test passes (its
+  // tolerance is +inf), so the geometric test alone decides: at the start
+  // angle, not at the loose bound the relative test runs under.
+  const double a_rms = o.geometry[7];
+  const bool start = o.relative && !(a_rms > 0.0 && a_rms < INFINITY);
+  return {2.0 * o.geometry[3], start ? o.start_inv_theta : o.inv_theta,
+          start ? o.start_inv_theta2 : o.inv_theta2};
+}
+
 // The records of node `w` from its moments; `first` and `count` as its link has
 // them, `particle` its first particle.
 template <bool QUAD>
 __device__ __forceinline__ void finish_node(const Tree& t, int w, const Moments& mo, int first,
                                             int count, int dfs, int particle, int lvl,
-                                            const Opening& o) {
+                                            const Opening& o, const OpeningTerms& terms) {
   t.mom[w] = make_double4(mo.m, mo.cx, mo.cy, mo.cz);
   // cell side 2h = root side / 2^lvl
   const int l = min(lvl, 21);
-  const double half = o.geometry[3];
-  const double side = ldexp(2.0 * half, -l);
+  const double side = terms.root_side * __hiloint2double((1023 - l) << 20, 0);
   double shift = 0.0;
   if (o.criterion == NBSP_BH_OPENING_OFFSET) {
+    const double half = o.geometry[3];
     // the cell's centre from the first key's top 3 lvl bits, in the particles'
     // frame (relative to the centre of mass)
     const uint64_t key = o.keys[particle];
@@ -1289,17 +1305,10 @@ __device__ __forceinline__ void finish_node(const Tree& t, int w, const Moments&
     }
     shift = sqrt(shift2);
   }
-  // Without previous accelerations every target's relative test passes (its
-  // tolerance is +inf), so the geometric test alone decides: at the start
-  // angle, not at the loose bound the relative test runs under.
-  const double a_rms = o.geometry[7];
-  const bool start = o.relative && !(a_rms > 0.0 && a_rms < INFINITY);
-  const double it = start ? o.start_inv_theta : o.inv_theta;
-  const double it2 = start ? o.start_inv_theta2 : o.inv_theta2;
   // reference: accept when (2h)^2 < theta^2 d^2; offset: when 2h / theta + shift < d
   const double r2 = o.criterion == NBSP_BH_OPENING_OFFSET
-                        ? (side * it + shift) * (side * it + shift)
-                        : side * side * it2;
+                        ? (side * terms.it + shift) * (side * terms.it + shift)
+                        : side * side * terms.it2;
   const float4 a = make_float4((float)mo.cx, (float)mo.cy, (float)mo.cz, (float)mo.m);
   const float4 b = make_float4((float)r2, (float)(mo.m * side * side), __int_as_float(first),
                                __int_as_float(count));
@@ -1316,6 +1325,8 @@ __device__ __forceinline__ void finish_node(const Tree& t, int w, const Moments&
                     mo.m > 0.0 ? (float)(mo.t2 / (mo.m * side * side)) : 0.f, (float)shift);
   }
 }
+
+constexpr size_t kMomentsWide = 1500000;  // particles from which occupancy counts
 
 // L2-coherent load of a double4 written by another thread of this grid.
 __device__ __forceinline__ double4 ldcg_d4(const double4* p) {
@@ -1342,14 +1353,17 @@ __device__ __forceinline__ int arrive_acq_rel(int* p) {
 // moments.  The parent's link does not depend on the arrival, so it is loaded
 // beside the atomic (and the grandparent's beside the moments); with lists of
 // children and per-node arrays the climb waited for two more loads a level.
-// Monopole pass at 6 blocks per SM (40 registers, a few spilled to L1): the
-// extra warps hide more of it (0.246 -> 0.228 ms at 10M); the quadrupole pass
-// is left to the compiler (its moments would spill hundreds of bytes per thread
-// at 40 or 64)
-template <bool QUAD>
-__global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4* __restrict__ pos, Tree t,
-                                                      Opening open, int* status) {
+// Every acquire makes what a thread reads afterwards come from L2 again, so the
+// opening terms are read once before the climb and nothing is spilled in it:
+// 37 -> 25 us at 10k particles, 49 -> 31 at 150k.  From kMomentsWide particles
+// on the leaves' loads are the larger part and the monopole pass runs 6 blocks
+// per SM (40 registers, a few spilled): 152 -> 123 us at 4M, but 55 -> 61 at 1M;
+// the quadrupole pass would spill hundreds of bytes per thread at 40 or 64.
+template <bool QUAD, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) moments_kernel(const float4* __restrict__ pos, Tree t,
+                                                              Opening open, int* status) {
   const int total = (int)t.offset[t.n];
+  const OpeningTerms terms = opening_terms(open);
   for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < total;
        node += gridDim.x * blockDim.x) {
     const int4 info = t.link[node];
@@ -1401,7 +1415,7 @@ __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4
       }
     }
     const int particle = info.y;
-    finish_node<QUAD>(t, node, mo, info.y, info.z, info.w, particle, t.level[node], open);
+    finish_node<QUAD>(t, node, mo, info.y, info.z, info.w, particle, t.level[node], open, terms);
     for (int climb = 0; parent >= 0; ++climb) {
       const int nc = -up.z, first = up.y;
       if (climb > 64 || parent >= total || nc < 1 || nc > 8 || first < 1 ||
@@ -1458,7 +1472,7 @@ __global__ void __launch_bounds__(256, QUAD ? 1 : 6) moments_kernel(const float4
       t.height[parent] = hmax + 1;
       // (the particle that names the cell's corner: any of the node's will do,
       // its key's top bits are the cell's)
-      finish_node<QUAD>(t, parent, pm, first, -nc, up.w, particle, level, open);
+      finish_node<QUAD>(t, parent, pm, first, -nc, up.w, particle, level, open, terms);
       parent = up.x;
       up = next;
     }
@@ -3045,11 +3059,11 @@ void nbsp_bh_moments(const void* pos4, const uint64_t* keys, size_t n, const dou
   size_t blocks = (nb + 255) / 256;  // grid-stride over the octree nodes (<= 2n - 1)
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (quadrupoles)
-    NBSP_COUNT_LAUNCH(1), moments_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(
+    NBSP_COUNT_LAUNCH(1), moments_kernel<true, 1><<<(unsigned)blocks, 256, 0, stream>>>(
                               (const float4*)pos4, t, o, status);
   else
-    NBSP_COUNT_LAUNCH(1), moments_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(
-                              (const float4*)pos4, t, o, status);
+    NBSP_COUNT_LAUNCH(1), (n < kMomentsWide ? moments_kernel<false, 1> : moments_kernel<false, 6>)
+        <<<(unsigned)blocks, 256, 0, stream>>>((const float4*)pos4, t, o, status);
 }
 
 void nbsp_bh_walk(const void* pos4, const float* tol, size_t n, const void* tree, int order,
