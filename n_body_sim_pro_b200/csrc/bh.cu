@@ -2130,15 +2130,24 @@ constexpr int kListStackRel = 960;
 // blocks per SM of the monopole list walks (at most 56 registers at 9): 9
 // where shared memory allows (the plain and the corrected walk's block at
 // 1024 ids is 24,576 B)
-// LATENCY, the walk of systems whose blocks all fit at once at 4 (quadrupole 3)
-// per SM: there a warp has its scheduler nearly to itself, and what counts is
-// the length of its own chain
-template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED, bool LATENCY>
+// LATENCY > 0: blocks per SM of the walk of small systems, whose warps have their
+// schedulers nearly to themselves, so that what counts is the length of their own
+// chains.  Four blocks while all fit at once (75,776 particles); then six
+// (quadrupole four) up to kLatencyBlocks blocks, which is two (three) times what
+// fits: walk at 113k 204 -> 180 us, 170k 284 -> 257, 200k 321 -> 293, the same at
+// 300k; quadrupole at 76k 212 -> 191, 150k 363 -> 356, 300k 680 -> 684
+constexpr unsigned kLatencyBlocks = 148 * 12;
+template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED, int LATENCY>
 constexpr int list_walk_blocks() {
-  return LATENCY      ? (ORDER != 1 ? 3 : 4)
+  return LATENCY > 0  ? LATENCY
          : ORDER != 1 ? 5
          : (!SHARED && (REL ? STACK == kListStackRel : true)) ? 9 : 8;
 }
+// LATENCY: pending nodes of a step beyond which each lane tests its own against
+// the 32 targets, rather than the lanes their targets against one node after
+// another: 32 independent tests take as long as four to eight of the others (turns
+// of 3, 6, 10, 16: walk at 10k 59, 59, 64, 67 us; at 56 registers it spills)
+constexpr int kProbeTurn = 4;
 // SHARED walk: the block's top-of-tree traversal keeps its stack and frontier
 // in the warps' stack space (it ends before any warp walks)
 constexpr int kCtaStack = 2048;    // warps 0 and 1's stacks
@@ -2185,12 +2194,13 @@ static_assert(kCtaStack + kFrontier <= 3 * kListStack, "frontier inside warp 2's
 // A block whose shared stack or frontier would overflow starts every group
 // from the root instead.
 //
-// LATENCY (small systems): the same steps with registers to spare, so that the
-// terms of a tile overlap (a lone warp waited about 2,800 cycles for a tile that
-// is 600 instructions at 56 registers); the records of the next step's nodes are
-// loaded before this step's tiles are evaluated, and four nodes at a time take
-// the per-target test.  LATENCY_MEASURED
-template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED = false, bool LATENCY = false>
+// LATENCY (small systems): the same steps with registers to spare; the records of
+// the next step's nodes are loaded before this step's tiles are evaluated, four
+// nodes at a time take the per-target test, and when more are pending each lane
+// tests its own node against all targets (groups on a system's outskirts have
+// wide boxes that decide little, and their steps set the walk's time): walk 106
+// -> 59 us at 10k, 107 -> 65 at 20k, 152 -> 115 at 65k.
+template <int ORDER, int STACK, bool CORR, bool REL, bool SHARED = false, int LATENCY = 0>
 __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, CORR, REL, SHARED, LATENCY>())) walk_lists_kernel(
     const float4* __restrict__ pos, const float* __restrict__ tol, int n, Tree t, float eps2,
     const uint32_t* __restrict__ perm, double4* __restrict__ acc,
@@ -2415,7 +2425,7 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
     next0 = __ldg(&t.wnode[2 * at]);
     next1 = __ldg(&t.wnode[2 * at + 1]);
   };
-  if (LATENCY) load_next();
+  if (LATENCY > 0) load_next();
   // (staged > 0 with nothing left to walk: cells the shared phase staged; the
   // draining iteration evaluates them)
   for (;;) {  // until the stack, the bucket list and the tiles are drained
@@ -2440,8 +2450,8 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
         const int at = valid ? node : 0;
         // one 32-byte record: the centre of mass and mass, the opening terms,
         // and a bucket's particles or an internal node's children
-        const float4 w0 = LATENCY ? next0 : __ldg(&t.wnode[2 * at]);
-        const float4 w1 = LATENCY ? next1 : __ldg(&t.wnode[2 * at + 1]);
+        const float4 w0 = LATENCY > 0 ? next0 : __ldg(&t.wnode[2 * at]);
+        const float4 w1 = LATENCY > 0 ? next1 : __ldg(&t.wnode[2 * at + 1]);
         c = w0;
         ro = w1.x;
         if (REL) km = w1.y;
@@ -2467,11 +2477,28 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       const bool opened = test && active && !opening_passes<REL>(d2own, ro, km, tl);
       test = test && !opened;
       float4* probe = s_probe[wib];
-      if (test) probe[lane] = make_float4(c.x, c.y, c.z, ro);
-      if (REL && test) s_probe_k[wib][lane] = km;
+      unsigned pend = __ballot_sync(kFull, test);
+      if (LATENCY > 0 && __popc(pend) > kProbeTurn) {
+        // many: each lane its own node against every target (an idle lane of the
+        // last group repeats the last particle and tolerates everything)
+        probe[lane] = make_float4(p.x, p.y, p.z, tl);
+        __syncwarp();
+        bool all = test;
+#pragma unroll 8
+        for (int q = 0; q < 32; ++q) {
+          const float4 u = probe[q];
+          const float dx = c.x - u.x, dy = c.y - u.y, dz = c.z - u.z;
+          all = opening_passes<REL>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), ro, km, u.w) && all;
+        }
+        accept = accept || all;
+        pend = 0u;
+      } else if (test) {
+        probe[lane] = make_float4(c.x, c.y, c.z, ro);
+        if (REL) s_probe_k[wib][lane] = km;
+      }
       __syncwarp();
-      constexpr int kProbes = LATENCY ? 4 : 1;
-      for (unsigned pend = __ballot_sync(kFull, test); pend != 0u;) {
+      constexpr int kProbes = LATENCY > 0 ? 4 : 1;
+      while (pend != 0u) {
         int from[kProbes];
         bool fail[kProbes];
 #pragma unroll
@@ -2517,7 +2544,7 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
       top += pushed;
       __syncwarp();
       next = lane < top ? stack[top - 1 - lane] : -1;
-      if (LATENCY) load_next();
+      if (LATENCY > 0) load_next();
       m = __ballot_sync(kFull, accept);
       if (ORDER == 1) {
         // A monopole cell is a point mass at its centre of mass, already in
@@ -2901,16 +2928,15 @@ void launch_walk(const float4* p, const float* tol, size_t n, Tree t, int order,
       NBSP_COUNT_LAUNCH(1), walk_lists_kernel<1, kListStack, false, REL, true><<<blocks, kListThreads, 0, stream>>>(
           p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none);
     } else if (order == 2) {
-      constexpr unsigned kAtOnce = 148 * list_walk_blocks<2, kListStack, false, REL, false, true>();
-      NBSP_COUNT_LAUNCH(1), (blocks <= kAtOnce ? walk_lists_kernel<2, kListStack, false, REL, false, true>
+      NBSP_COUNT_LAUNCH(1), (blocks <= kLatencyBlocks ? walk_lists_kernel<2, kListStack, false, REL, false, 4>
                                                : walk_lists_kernel<2, kListStack, false, REL>)
           <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
                                                 status, nullptr, none);
     } else {
       constexpr int kStack = REL ? kListStackRel : kListStack;
-      constexpr unsigned kAtOnce = 148 * list_walk_blocks<1, kStack, false, REL, false, true>();
-      NBSP_COUNT_LAUNCH(1), (blocks <= kAtOnce ? walk_lists_kernel<1, kStack, false, REL, false, true>
-                                               : walk_lists_kernel<1, kStack, false, REL>)
+      NBSP_COUNT_LAUNCH(1), (blocks <= 148 * 4   ? walk_lists_kernel<1, kStack, false, REL, false, 4>
+                             : blocks <= kLatencyBlocks ? walk_lists_kernel<1, kStack, false, REL, false, 6>
+                                                 : walk_lists_kernel<1, kStack, false, REL>)
           <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
                                                 status, nullptr, none);
     }

@@ -38,3 +38,29 @@ def test_walks_agree_on_the_tree(cuda, n, leaf, order):
         c.upload(s)
         exact = c.reference_acceleration(g, np.arange(n))
     assert np.sqrt(np.sum((results[1] - exact) ** 2) / np.sum(exact ** 2)) < 1e-2
+
+
+@pytest.mark.parametrize("n", [75776, 75777, 227328, 227329])
+@pytest.mark.parametrize("order, alpha", [(1, 0.0), (1, 0.005), (2, 0.0)])
+def test_walk_forms_take_the_same_decisions(cuda, n, order, alpha):
+    """Either side of the lines between the list walk's register forms: the same
+    cells and particles as the stackless walk, the same sums to FP32 rounding."""
+    s = to_system(cuda, O.preset_parallel("globular_cluster", n, 3))
+    g = cuda.gravity_init(1.0, 0.01)
+    results, counts = [], []
+    for walk in (0, 1):
+        with cuda.CudaContext(theta=0.7, multipole_order=order, relative_opening=alpha) as c:
+            c.set_walk(walk)
+            c.upload(s)
+            for _ in range(2 if alpha > 0.0 else 1):
+                c.compute_acceleration(g, cuda.Algorithm.BARNES_HUT)
+            results.append(c.download_accelerations())
+            st = c.stats()
+            counts.append([st["accepted_approximations"], st["exact_interactions"]])
+    if alpha == 0.0:
+        assert counts[0] == counts[1]
+    else:  # the first evaluations' roundings move the second's tolerances
+        assert abs(counts[0][0] - counts[1][0]) <= 1e-6 * counts[1][0]
+    rms = np.sqrt(np.mean(results[0] ** 2))
+    bar = 2e-6 if alpha == 0.0 else 2e-5
+    assert np.sqrt(np.mean((results[0] - results[1]) ** 2)) <= bar * rms
