@@ -534,12 +534,13 @@ static NBodySimProStatus pack_state(NBodySimProCudaContext* c, NBodySimProError*
 
 /* One force evaluation of the resident state with `algorithm`; with a
  * leapfrog fusion (Barnes-Hut only; NULL: none) the step's opening kick and
- * drift and its closing kick run inside the evaluation's first and last passes. */
+ * drift and its closing kick run inside the evaluation's first and last passes.
+ * unread: its statistics and phase timings will be those of a later one. */
 static NBodySimProStatus resident_accelerations_fused(NBodySimProCudaContext* c,
                                                       const NBodySimProGravity* g,
                                                       NBodySimProCudaAlgorithm algorithm,
                                                       const NbspLeapfrogFusion* leapfrog,
-                                                      NBodySimProError* error) {
+                                                      int unread, NBodySimProError* error) {
     if (c->n == 0) return N_BODY_SIM_PRO_STATUS_OK;
     if (algorithm == N_BODY_SIM_PRO_CUDA_ALGORITHM_BARNES_HUT) {
         NbspBarnesHutParams p;
@@ -553,6 +554,7 @@ static NBodySimProStatus resident_accelerations_fused(NBodySimProCudaContext* c,
         p.tolerance = c->tolerance;
         p.correction = c->correction;
         p.quadrupoles = c->tree_quadrupoles;
+        p.unread = unread;
         NbspBarnesHutState s = {c->x, c->y, c->z, c->m, c->ax, c->ay, c->az, c->n,
                                 {NULL, NULL, NULL, 0.0, 0.0}};
         if (leapfrog != NULL) s.leapfrog = *leapfrog;
@@ -570,7 +572,7 @@ static NBodySimProStatus resident_accelerations(NBodySimProCudaContext* c,
                                                 const NBodySimProGravity* g,
                                                 NBodySimProCudaAlgorithm algorithm,
                                                 NBodySimProError* error) {
-    return resident_accelerations_fused(c, g, algorithm, NULL, error);
+    return resident_accelerations_fused(c, g, algorithm, NULL, 0, error);
 }
 
 /* ------------------------------------------------------------------------- */
@@ -1070,8 +1072,8 @@ NBodySimProStatus n_body_sim_pro_cuda_advance(NBodySimProCudaContext* c,
         const NbspLeapfrogFusion lf = {c->vx, c->vy, c->vz, h, dt};
         for (int step = 0; step < steps; ++step) {
             if (n >= 2) {
-                if ((st = resident_accelerations_fused(c, gravity, algorithm, &lf, error)) !=
-                    N_BODY_SIM_PRO_STATUS_OK)
+                if ((st = resident_accelerations_fused(c, gravity, algorithm, &lf, step + 1 < steps,
+                                                       error)) != N_BODY_SIM_PRO_STATUS_OK)
                     return st;
                 continue;
             }

@@ -40,6 +40,8 @@ typedef struct NbspBarnesHutParams {
     int opening;            /* NBSP_BH_OPENING_* */
     double tolerance;       /* alpha of the relative opening test; 0: geometric test alone */
     const void* correction; /* device network (mlp.cuh Net) or NULL */
+    int unread;             /* an evaluation whose statistics and timings nobody will read
+                               (a step before an advance's last): none are taken */
     int quadrupoles;        /* the cells' quadrupoles and spread even for the monopole walk
                                (the correction's training reads them) */
 } NbspBarnesHutParams;

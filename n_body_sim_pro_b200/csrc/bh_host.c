@@ -38,6 +38,7 @@ struct NbspBarnesHut {
     unsigned long long* host_counters;  /* pinned */
     cudaEvent_t events[BH_EVENTS];
     int timed;                          /* events hold a full evaluation */
+    int unread;                         /* NbspBarnesHutParams.unread of this evaluation */
 };
 
 static NBodySimProStatus bh_fail(NBodySimProError* error, NBodySimProStatus status,
@@ -153,6 +154,13 @@ static NBodySimProStatus ensure(NbspBarnesHut** handle, size_t n, NBodySimProErr
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
+/* A phase boundary of an evaluation whose timings are read.  (An event between
+ * two kernels holds the second one back; eight of them were a tenth of a step at
+ * 10k particles.) */
+static void mark(NbspBarnesHut* b, int event, cudaStream_t stream) {
+    if (!b->unread) cudaEventRecord(b->events[event], stream);
+}
+
 /* The bounds, the sorted keys and permutation, and the walk's records in that
  * order.  tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
 static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, double tol_scale,
@@ -164,24 +172,24 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
     nbsp_bh_bounds(s->x, s->y, s->z, s->m, s->n, b->partial, small ? NULL : b->geometry, status,
                    with_a ? s->ax : NULL, with_a ? s->ay : NULL, with_a ? s->az : NULL, rel, lf,
                    stream);
-    cudaEventRecord(b->events[1], stream);
+    mark(b, 1, stream);
     if (small) {
         nbsp_bh_small_keys(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, b->keys_alt,
                            b->index_alt, b->unsorted, s->ax, s->ay, s->az, tol_scale,
                            rel ? b->tol_unsorted : NULL, b->tree, b->counters, stream);
-        cudaEventRecord(b->events[2], stream);
+        mark(b, 2, stream);
         nbsp_bh_small_merge(b->keys_alt, b->index_alt, s->n, b->keys, b->index, b->unsorted,
                             b->pos4, rel ? b->tol_unsorted : NULL, rel ? b->tol : NULL, status,
                             stream);
-        cudaEventRecord(b->events[3], stream);
+        mark(b, 3, stream);
         return N_BODY_SIM_PRO_STATUS_OK;
     }
     nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys, b->index, b->unsorted,
                  b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, b->tree,
                  b->counters, stream);
-    cudaEventRecord(b->events[2], stream);
+    mark(b, 2, stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status, stream);
-    cudaEventRecord(b->events[3], stream);
+    mark(b, 3, stream);
     nbsp_bh_gather(b->unsorted, b->index, s->n, b->pos4, rel ? b->tol_unsorted : NULL,
                    rel ? b->tol : NULL, status, stream);
     return N_BODY_SIM_PRO_STATUS_OK;
@@ -196,6 +204,7 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     NbspBarnesHut* b = *handle;
     const size_t n = s->n;
+    b->unread = p->unread;
     if (n == 1) { /* a lone particle feels nothing; no tree to walk */
         BH_TRY(cudaMemsetAsync(s->ax, 0, sizeof(double), stream));
         BH_TRY(cudaMemsetAsync(s->ay, 0, sizeof(double), stream));
@@ -205,7 +214,7 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
         b->timed = 0;
         return N_BODY_SIM_PRO_STATUS_OK;
     }
-    cudaEventRecord(b->events[0], stream);
+    mark(b, 0, stream);
     /* relative opening test: tolerance alpha |a_old| / G */
     const double g = fabs(p->gravitational_constant);
     const double tol_scale = p->tolerance > 0.0 ? (g > 0.0 ? p->tolerance / g : INFINITY) : 0.0;
@@ -215,23 +224,24 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     morton(b, s, tol_scale, status, stream);
     nbsp_bh_build(b->keys, b->index, s->x, s->y, s->z, n, p->leaf_capacity, b->tree, status,
                   stream);
-    cudaEventRecord(b->events[4], stream);
+    mark(b, 4, stream);
     nbsp_bh_moments(b->pos4, b->keys, n, b->geometry, p->theta,
                     rel ? fmin(p->theta, NBSP_BH_START_THETA) : 0.0, p->opening,
                     p->multipole_order == 2 || p->correction != NULL || p->quadrupoles, b->tree,
                     status, stream);
-    cudaEventRecord(b->events[5], stream);
+    mark(b, 5, stream);
     nbsp_bh_walk(b->pos4, rel ? b->tol : NULL, n, b->tree, p->multipole_order, p->walk_mode,
                  p->correction, p->correction != NULL ? &b->lists : NULL,
                  (float)p->softening_squared, b->index, b->acc, b->counters, status, stream);
     if (p->correction != NULL)
         nbsp_bh_correct(b->pos4, n, b->tree, p->correction, &b->lists, b->index, b->acc,
                         b->counters, status, stream);
-    cudaEventRecord(b->events[6], stream);
+    mark(b, 6, stream);
     nbsp_bh_unsort(b->acc, n, p->gravitational_constant, s->ax, s->ay, s->az,
                    s->leapfrog.vx != NULL ? &s->leapfrog : NULL, b->tree, b->counters, stream);
-    cudaEventRecord(b->events[7], stream);
+    mark(b, 7, stream);
     BH_TRY(cudaGetLastError());
+    if (p->unread) return N_BODY_SIM_PRO_STATUS_OK;
     BH_TRY(cudaMemcpyAsync(b->host_counters, b->counters, BH_COUNTERS * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, stream));
     b->timed = 1;
@@ -282,7 +292,8 @@ NBodySimProStatus nbsp_bh_morton(NbspBarnesHut** handle, const NbspBarnesHutStat
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     NbspBarnesHut* b = *handle;
     const size_t n = s->n;
-    cudaEventRecord(b->events[0], stream);
+    b->unread = 0;
+    mark(b, 0, stream);
     morton(b, s, 0.0, status, stream);
     BH_TRY(cudaGetLastError());
     uint32_t* perm32 = NULL;
