@@ -194,7 +194,8 @@ typedef enum NBodySimProCudaAlgorithm {
     N_BODY_SIM_PRO_CUDA_ALGORITHM_BARNES_HUT = 1
 } NBodySimProCudaAlgorithm;
 
-/* Per-phase device time of the most recent evaluation, milliseconds (CUDA events). */
+/* Per-phase device time of the most recent evaluation, milliseconds: Barnes-Hut
+ * phases from the GPU's clock at each phase's start, the rest from CUDA events. */
 typedef struct NBodySimProCudaTimings {
     double bounds_ms;      /* bbox + centre-of-mass reduction */
     double keys_ms;        /* Morton keys */
@@ -311,7 +312,7 @@ N_BODY_SIM_PRO_CUDA_API NBodySimProStatus n_body_sim_pro_cuda_context_set_relati
 N_BODY_SIM_PRO_CUDA_API int n_body_sim_pro_cuda_context_stats(
     const NBodySimProCudaContext* context, NBodySimProBarnesHutStats* stats);
 
-/* Device-event phase timings of the last evaluation or advance. 0 on success. */
+/* Phase timings of the last evaluation or advance. 0 on success. */
 N_BODY_SIM_PRO_CUDA_API int n_body_sim_pro_cuda_context_timings(
     const NBodySimProCudaContext* context, NBodySimProCudaTimings* timings);
 

@@ -74,6 +74,18 @@ __device__ __forceinline__ void bounds_block_reduce(double (&v)[kBoundsVals],
   }
 }
 
+// Phase boundaries of an evaluation are read from the GPU's clock by the first
+// thread of each phase's first kernel (stamp NULL: not timed).  A timing event
+// between two kernels held the second one back by about 3.5 us.
+__device__ __forceinline__ unsigned long long gpu_clock() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void stamp_start(unsigned long long* stamp) {
+  if (stamp != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *stamp = gpu_clock();
+}
+
 // KICK: the opening kick and drift of a device-resident leapfrog step first
 // (kick_drift_kernel's arithmetic), the reductions then of the drifted state.
 template <bool KICK>
@@ -82,7 +94,9 @@ __global__ void __launch_bounds__(kBoundsThreads) bounds_kernel(
     const double* __restrict__ m, size_t n, double* __restrict__ partial, int* status,
     const double* __restrict__ ax, const double* __restrict__ ay,
     const double* __restrict__ az, bool rms_of_a, double* __restrict__ vx,
-    double* __restrict__ vy, double* __restrict__ vz, double h, double dt) {
+    double* __restrict__ vy, double* __restrict__ vz, double h, double dt,
+    unsigned long long* stamp) {
+  stamp_start(stamp);
   __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
   double v[kBoundsVals] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY,
                            0.0,      0.0,      0.0,      0.0,       0.0};
@@ -352,10 +366,13 @@ inline size_t sort_scratch_words(size_t n) {
 // What the build and the walk count into starts at zero (with every particle's
 // mask, which the keys kernels clear beside its key; memsets took a place of
 // their own on the stream).
-constexpr int kCounters = 8;
-__device__ __forceinline__ void start_tree(const Tree& t, unsigned long long* counters) {
+constexpr int kCounters = NBSP_BH_COUNTERS;
+__device__ __forceinline__ void start_tree(const Tree& t, unsigned long long* counters,
+                                           unsigned long long* stamp) {
+  stamp_start(stamp);
   if (blockIdx.x == 0 && threadIdx.x < kCounters) {
     counters[threadIdx.x] = 0;
+    if (threadIdx.x == 0) counters[kCounters + NBSP_BH_END] = 0;
     if (threadIdx.x < 2) t.leaves[threadIdx.x] = 0;
   }
 }
@@ -386,9 +403,9 @@ __global__ void __launch_bounds__(256) keys_kernel(
     uint64_t* __restrict__ keys, uint32_t* __restrict__ index, float4* __restrict__ unsorted,
     uint32_t* __restrict__ hist, const double* __restrict__ ax, const double* __restrict__ ay,
     const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol, Tree tree,
-    unsigned long long* counters) {
+    unsigned long long* counters, unsigned long long* stamp) {
   __shared__ uint32_t h[kSortPasses][kRadix];
-  start_tree(tree, counters);
+  start_tree(tree, counters, stamp);
   for (int k = threadIdx.x; k < kSortPasses * kRadix; k += blockDim.x) (&h[0][0])[k] = 0;
   __syncthreads();
   double geo[8];
@@ -440,7 +457,9 @@ template <class S>
 __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n, int shift,
-    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* status, int* err) {
+    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* status, int* err,
+    unsigned long long* stamp) {
+  stamp_start(stamp);
   constexpr int kSortThreads = S::kThreads, kSortItems = S::kItems;
   constexpr int kSortWarps = kSortThreads / 32, kSortTile = sort_tile<S>();
   extern __shared__ __align__(16) unsigned char smem[];
@@ -613,13 +632,13 @@ __global__ void __launch_bounds__(kSmallTile) small_keys_kernel(
     double* __restrict__ geometry, uint64_t* __restrict__ keys, uint32_t* __restrict__ index,
     float4* __restrict__ unsorted, const double* __restrict__ ax, const double* __restrict__ ay,
     const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol, Tree tree,
-    unsigned long long* counters) {
+    unsigned long long* counters, unsigned long long* stamp) {
   __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
   __shared__ double s_geo[8];
   __shared__ uint64_t sk[kSmallTile];
   __shared__ uint32_t sv[kSmallTile];
   const int t = threadIdx.x;
-  start_tree(tree, counters);
+  start_tree(tree, counters, stamp);
   root_geometry(partial, blocks, n, sh, s_geo);
   __syncthreads();
   double geo[8];
@@ -670,7 +689,9 @@ __global__ void __launch_bounds__(32 * kMergeWarps) small_merge_kernel(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, int n,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
     const float4* __restrict__ unsorted, float4* __restrict__ pos,
-    const float* __restrict__ unsorted_tol, float* __restrict__ tol, int* err) {
+    const float* __restrict__ unsorted_tol, float* __restrict__ tol, int* err,
+    unsigned long long* stamp) {
+  stamp_start(stamp);
   __shared__ int s_rank[kMergeWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int s = blockIdx.x * 32 + lane;
@@ -754,7 +775,8 @@ __device__ __forceinline__ void flag_duplicates(size_t s, const uint64_t* __rest
 __global__ void gather_kernel(const float4* __restrict__ unsorted,
                               const uint32_t* __restrict__ perm, size_t n,
                               float4* __restrict__ pos, const float* __restrict__ unsorted_tol,
-                              float* __restrict__ tol, int* status) {
+                              float* __restrict__ tol, int* status, unsigned long long* stamp) {
+  stamp_start(stamp);
   for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < n;
        s += (size_t)gridDim.x * blockDim.x) {
     const uint32_t i = perm[s];
@@ -779,7 +801,8 @@ __global__ void unsort_kernel(const double4* __restrict__ acc, size_t n, double 
                               double* __restrict__ ax, double* __restrict__ ay,
                               double* __restrict__ az, double* __restrict__ vx,
                               double* __restrict__ vy, double* __restrict__ vz, double h, Tree t,
-                              unsigned long long* counters) {
+                              unsigned long long* counters, unsigned long long* stamp) {
+  stamp_start(stamp);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     counters[2] = t.offset[t.n];
     counters[3] = t.leaves[0];
@@ -798,6 +821,8 @@ __global__ void unsort_kernel(const double4* __restrict__ acc, size_t n, double 
       vz[i] = __dadd_rn(vz[i], __dmul_rn(gz, h));
     }
   }
+  if (stamp != nullptr && threadIdx.x == 0)  // the last block's end is the evaluation's
+    atomicMax(stamp + (NBSP_BH_END - NBSP_BH_INTEGRATE), gpu_clock());
 }
 
 // ---------------------------------------------------------------------------
@@ -831,7 +856,8 @@ __device__ __forceinline__ int level_of_delta(int delta) { return min(delta / 3,
 __global__ void radix_tree_kernel(const uint64_t* __restrict__ keys,
                                   const uint32_t* __restrict__ perm, const double* __restrict__ x,
                                   const double* __restrict__ y, const double* __restrict__ z,
-                                  Tree t, int* status) {
+                                  Tree t, int* status, unsigned long long* stamp) {
+  stamp_start(stamp);
   const int n = t.n;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
@@ -1374,7 +1400,9 @@ __device__ __forceinline__ int arrive_acq_rel(int* p) {
 // the quadrupole pass would spill hundreds of bytes per thread at 40 or 64.
 template <bool QUAD, int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS) moments_kernel(const float4* __restrict__ pos, Tree t,
-                                                              Opening open, int* status) {
+                                                              Opening open, int* status,
+                                                              unsigned long long* stamp) {
+  stamp_start(stamp);
   const int total = (int)t.offset[t.n];
   const OpeningTerms terms = opening_terms(open);
   for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < total;
@@ -1665,7 +1693,8 @@ template <int ORDER, bool REL>
 __global__ void __launch_bounds__(kWalkThreads) walk_kernel(
     const float4* __restrict__ pos, const float* __restrict__ tol, int n, Tree t, float eps2,
     const uint32_t* __restrict__ perm, double4* __restrict__ acc,
-    unsigned long long* __restrict__ counters, int* status) {
+    unsigned long long* __restrict__ counters, int* status, unsigned long long* stamp) {
+  stamp_start(stamp);
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kWalkThreads + threadIdx.x) >> 5;
   if (warp * 32 >= n) return;
@@ -2205,7 +2234,9 @@ __global__ void __launch_bounds__(kListThreads, (list_walk_blocks<ORDER, STACK, 
     const float4* __restrict__ pos, const float* __restrict__ tol, int n, Tree t, float eps2,
     const uint32_t* __restrict__ perm, double4* __restrict__ acc,
     unsigned long long* __restrict__ counters, int* status,
-    const nbsp_mlp::Net* __restrict__ net, NbspCorrectionLists lists) {
+    const nbsp_mlp::Net* __restrict__ net, NbspCorrectionLists lists,
+    unsigned long long* stamp) {
+  stamp_start(stamp);
   static_assert(!SHARED || (ORDER == 1 && !CORR && STACK == kListStack), "shared top: monopole walk");
   __shared__ int s_stack[kListThreads / 32][STACK];
   __shared__ float s_probe_k[kListThreads / 32][REL ? 32 : 1];  // their M side^2
@@ -2917,38 +2948,38 @@ template <bool REL>
 void launch_walk(const float4* p, const float* tol, size_t n, Tree t, int order, int mode,
                  const nbsp_mlp::Net* net, const NbspCorrectionLists* lists, float eps2,
                  const uint32_t* perm, double4* out, unsigned long long* counters, int* status,
-                 cudaStream_t stream) {
+                 unsigned long long* stamp, cudaStream_t stream) {
   if (mode == NBSP_BH_WALK_LISTS || mode == NBSP_BH_WALK_SHARED || net != nullptr) {
     const unsigned blocks = (unsigned)((n + kListThreads - 1) / kListThreads);
     NbspCorrectionLists none{};
     if (net != nullptr && lists != nullptr) {  // the network corrects the monopole term
       NBSP_COUNT_LAUNCH(1), walk_lists_kernel<1, kListStack, true, REL><<<blocks, kListThreads, 0, stream>>>(
-          p, tol, (int)n, t, eps2, perm, out, counters, status, net, *lists);
+          p, tol, (int)n, t, eps2, perm, out, counters, status, net, *lists, stamp);
     } else if (order == 1 && mode == NBSP_BH_WALK_SHARED) {
       NBSP_COUNT_LAUNCH(1), walk_lists_kernel<1, kListStack, false, REL, true><<<blocks, kListThreads, 0, stream>>>(
-          p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none);
+          p, tol, (int)n, t, eps2, perm, out, counters, status, nullptr, none, stamp);
     } else if (order == 2) {
       NBSP_COUNT_LAUNCH(1), (blocks <= kLatencyBlocks ? walk_lists_kernel<2, kListStack, false, REL, false, 4>
                                                : walk_lists_kernel<2, kListStack, false, REL>)
           <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
-                                                status, nullptr, none);
+                                                status, nullptr, none, stamp);
     } else {
       constexpr int kStack = REL ? kListStackRel : kListStack;
       NBSP_COUNT_LAUNCH(1), (blocks <= 148 * 4   ? walk_lists_kernel<1, kStack, false, REL, false, 4>
                              : blocks <= kLatencyBlocks ? walk_lists_kernel<1, kStack, false, REL, false, 6>
                                                  : walk_lists_kernel<1, kStack, false, REL>)
           <<<blocks, kListThreads, 0, stream>>>(p, tol, (int)n, t, eps2, perm, out, counters,
-                                                status, nullptr, none);
+                                                status, nullptr, none, stamp);
     }
     return;
   }
   const unsigned blocks = (unsigned)((n + kWalkThreads - 1) / kWalkThreads);
   if (order == 2) {
     NBSP_COUNT_LAUNCH(1), walk_kernel<2, REL><<<blocks, kWalkThreads, 0, stream>>>(
-        p, tol, (int)n, t, eps2, perm, out, counters, status);
+        p, tol, (int)n, t, eps2, perm, out, counters, status, stamp);
   } else {
     NBSP_COUNT_LAUNCH(1), walk_kernel<1, REL><<<blocks, kWalkThreads, 0, stream>>>(
-        p, tol, (int)n, t, eps2, perm, out, counters, status);
+        p, tol, (int)n, t, eps2, perm, out, counters, status, stamp);
   }
 }
 
@@ -2959,16 +2990,16 @@ extern "C" {
 void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n, double* partial,
                     double* geometry, int* status, const double* ax, const double* ay,
                     const double* az, int rms_of_a, const NbspLeapfrogFusion* leapfrog,
-                    cudaStream_t stream) {
+                    unsigned long long* stamp, cudaStream_t stream) {
   const int blocks = bounds_blocks(n);
   if (leapfrog != nullptr && leapfrog->vx != nullptr) {
     NBSP_COUNT_LAUNCH(1), bounds_kernel<true><<<blocks, kBoundsThreads, 0, stream>>>(
         x, y, z, m, n, partial, status, ax, ay, az, rms_of_a != 0, leapfrog->vx, leapfrog->vy,
-        leapfrog->vz, leapfrog->half_dt, leapfrog->dt);
+        leapfrog->vz, leapfrog->half_dt, leapfrog->dt, stamp);
   } else {
     NBSP_COUNT_LAUNCH(1), bounds_kernel<false><<<blocks, kBoundsThreads, 0, stream>>>(
         x, y, z, m, n, partial, status, ax, ay, az, rms_of_a != 0, nullptr, nullptr, nullptr,
-        0.0, 0.0);
+        0.0, 0.0, stamp);
   }
   if (geometry != nullptr)
     NBSP_COUNT_LAUNCH(1), bounds_final_kernel<<<1, kBoundsThreads, 0, stream>>>(partial, blocks, n,
@@ -2979,20 +3010,21 @@ void nbsp_bh_small_keys(const double* x, const double* y, const double* z, const
                         size_t n, const double* partial, double* geometry, uint64_t* keys,
                         uint32_t* index, void* unsorted, const double* ax, const double* ay,
                         const double* az, double tol_scale, float* unsorted_tol, void* tree,
-                        unsigned long long* counters, cudaStream_t stream) {
+                        unsigned long long* counters, unsigned long long* stamp,
+                        cudaStream_t stream) {
   const unsigned tiles = (unsigned)((n + kSmallTile - 1) / kSmallTile);
   NBSP_COUNT_LAUNCH(1), small_keys_kernel<<<tiles, kSmallTile, 0, stream>>>(
       x, y, z, m, n, partial, bounds_blocks(n), geometry, keys, index, (float4*)unsorted, ax, ay,
-      az, tol_scale, unsorted_tol, tree_view(tree, n), counters);
+      az, tol_scale, unsorted_tol, tree_view(tree, n), counters, stamp);
 }
 
 void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
                          uint64_t* keys, uint32_t* index, const void* unsorted, void* pos4,
                          const float* unsorted_tol, float* tol, int* status,
-                         cudaStream_t stream) {
+                         unsigned long long* stamp, cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), small_merge_kernel<<<(unsigned)((n + 31) / 32), 32 * kMergeWarps, 0, stream>>>(
       keys_in, index_in, (int)n, keys, index, (const float4*)unsorted, (float4*)pos4,
-      unsorted_tol, tol, status);
+      unsorted_tol, tol, status, stamp);
 }
 
 // (buffers for n hold every smaller system too, whose narrow tiles may be more)
@@ -3006,7 +3038,7 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
                   const double* geometry, uint64_t* keys, uint32_t* index, void* unsorted,
                   uint32_t* scratch, const double* ax, const double* ay, const double* az,
                   double tol_scale, float* unsorted_tol, void* tree,
-                  unsigned long long* counters, cudaStream_t stream) {
+                  unsigned long long* counters, unsigned long long* stamp, cudaStream_t stream) {
   cudaMemsetAsync(scratch, 0, sort_scratch_words(n) * sizeof(uint32_t), stream);
   const SortScratch sc = sort_scratch(scratch);
   size_t blocks = (n + 255) / 256;
@@ -3014,11 +3046,12 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
   if (blocks > (size_t)kKeysBlocks) blocks = kKeysBlocks;
   NBSP_COUNT_LAUNCH(1), keys_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
       x, y, z, m, n, geometry, keys, index, (float4*)unsorted, sc.hist, ax, ay, az, tol_scale,
-      unsorted_tol, tree_view(tree, n), counters);
+      unsorted_tol, tree_view(tree, n), counters, stamp);
 }
 
 void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t* index_alt,
-                  size_t n, uint32_t* scratch, int* status, cudaStream_t stream) {
+                  size_t n, uint32_t* scratch, int* status, unsigned long long* stamp,
+                  cudaStream_t stream) {
   const bool narrow = n < kSortWide;
   const auto pass_kernel = narrow ? sort_pass_kernel<SortNarrow> : sort_pass_kernel<SortWide>;
   const int threads = narrow ? SortNarrow::kThreads : SortWide::kThreads;
@@ -3033,7 +3066,7 @@ void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t*
   for (int pass = 0; pass < kSortPasses; ++pass) {
     NBSP_COUNT_LAUNCH(1), pass_kernel<<<(unsigned)tiles, threads, smem, stream>>>(
         kin, vin, kout, vout, n, 8 * pass, sc.hist + pass * kRadix, sc.ticket + pass,
-        sc.status + (size_t)pass * tiles * kRadix, status);
+        sc.status + (size_t)pass * tiles * kRadix, status, pass == 0 ? stamp : nullptr);
     uint64_t* tk = kin;
     kin = kout;
     kout = tk;
@@ -3045,20 +3078,21 @@ void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t*
 }
 
 void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* pos4,
-                    const float* unsorted_tol, float* tol, int* status, cudaStream_t stream) {
+                    const float* unsorted_tol, float* tol, int* status, unsigned long long* stamp,
+                    cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), gather_kernel<<<grid_for(n, 256), 256, 0, stream>>>(
-      (const float4*)unsorted, perm, n, (float4*)pos4, unsorted_tol, tol, status);
+      (const float4*)unsorted, perm, n, (float4*)pos4, unsorted_tol, tol, status, stamp);
 }
 
 size_t nbsp_bh_tree_bytes(size_t n) { return tree_bytes(n); }
 
 void nbsp_bh_build(const uint64_t* keys, const uint32_t* perm, const double* x, const double* y,
                    const double* z, size_t n, int leaf_capacity, void* tree, int* status,
-                   cudaStream_t stream) {
+                   unsigned long long* stamp, cudaStream_t stream) {
   Tree t = tree_view(tree, n);
   if (n >= 2)
     NBSP_COUNT_LAUNCH(1), radix_tree_kernel<<<(unsigned)((n - 1 + 255) / 256), 256, 0, stream>>>(
-        keys, perm, x, y, z, t, status);
+        keys, perm, x, y, z, t, status, stamp);
   // (n >= 2: the caller handles a lone particle without a tree)
   const unsigned keep_blocks = (unsigned)((n - 1 + kKeepNodes - 1) / kKeepNodes);
   if (keep_blocks > 0)
@@ -3083,7 +3117,7 @@ void nbsp_bh_build(const uint64_t* keys, const uint32_t* perm, const double* x, 
 
 void nbsp_bh_moments(const void* pos4, const uint64_t* keys, size_t n, const double* geometry,
                      double theta, double start_theta, int opening, int quadrupoles, void* tree,
-                     int* status, cudaStream_t stream) {
+                     int* status, unsigned long long* stamp, cudaStream_t stream) {
   Tree t = tree_view(tree, n);
   const size_t nb = 2 * n - 1;
   Opening o;
@@ -3099,26 +3133,26 @@ void nbsp_bh_moments(const void* pos4, const uint64_t* keys, size_t n, const dou
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (quadrupoles)
     NBSP_COUNT_LAUNCH(1), moments_kernel<true, 1><<<(unsigned)blocks, 256, 0, stream>>>(
-                              (const float4*)pos4, t, o, status);
+                              (const float4*)pos4, t, o, status, stamp);
   else
     NBSP_COUNT_LAUNCH(1), (n < kMomentsWide ? moments_kernel<false, 1> : moments_kernel<false, 6>)
-        <<<(unsigned)blocks, 256, 0, stream>>>((const float4*)pos4, t, o, status);
+        <<<(unsigned)blocks, 256, 0, stream>>>((const float4*)pos4, t, o, status, stamp);
 }
 
 void nbsp_bh_walk(const void* pos4, const float* tol, size_t n, const void* tree, int order,
                   int mode, const void* correction, const NbspCorrectionLists* lists, float eps2,
                   const uint32_t* perm, void* acc, unsigned long long* counters, int* status,
-                  cudaStream_t stream) {
+                  unsigned long long* stamp, cudaStream_t stream) {
   Tree t = tree_view(const_cast<void*>(tree), n);
   const nbsp_mlp::Net* net = (const nbsp_mlp::Net*)correction;
   const float4* p = (const float4*)pos4;
   double4* out = (double4*)acc;
   if (tol != nullptr)
     launch_walk<true>(p, tol, n, t, order, mode, net, lists, eps2, perm, out, counters, status,
-                      stream);
+                      stamp, stream);
   else
     launch_walk<false>(p, nullptr, n, t, order, mode, net, lists, eps2, perm, out, counters,
-                       status, stream);
+                       status, stamp, stream);
 }
 
 void nbsp_bh_correct(const void* pos4, size_t n, const void* tree, const void* correction,
@@ -3141,15 +3175,16 @@ void nbsp_bh_correct(const void* pos4, size_t n, const void* tree, const void* c
 
 void nbsp_bh_unsort(const void* acc, size_t n, double g, double* ax, double* ay, double* az,
                     const NbspLeapfrogFusion* leapfrog, const void* tree,
-                    unsigned long long* counters, cudaStream_t stream) {
+                    unsigned long long* counters, unsigned long long* stamp,
+                    cudaStream_t stream) {
   const Tree t = tree_view(const_cast<void*>(tree), n);
   if (leapfrog != nullptr && leapfrog->vx != nullptr) {
     NBSP_COUNT_LAUNCH(1), unsort_kernel<true><<<grid_for(n, 256), 256, 0, stream>>>(
         (const double4*)acc, n, g, ax, ay, az, leapfrog->vx, leapfrog->vy, leapfrog->vz,
-        leapfrog->half_dt, t, counters);
+        leapfrog->half_dt, t, counters, stamp);
   } else {
     NBSP_COUNT_LAUNCH(1), unsort_kernel<false><<<grid_for(n, 256), 256, 0, stream>>>(
-        (const double4*)acc, n, g, ax, ay, az, nullptr, nullptr, nullptr, 0.0, t, counters);
+        (const double4*)acc, n, g, ax, ay, az, nullptr, nullptr, nullptr, 0.0, t, counters, stamp);
   }
 }
 

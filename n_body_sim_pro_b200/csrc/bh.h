@@ -91,6 +91,22 @@ NBSP_HIDDEN void nbsp_bh_destroy(NbspBarnesHut* bh);
 
 /* ---- kernel launchers (bh.cu) -------------------------------------------- */
 
+/* The device counters of an evaluation are followed by the GPU clock (ns) at the
+ * start of its phases; a launcher's `stamp` is the place of its phase (NULL: not
+ * timed). */
+enum { NBSP_BH_COUNTERS = 8 };
+enum {
+    NBSP_BH_BOUNDS,
+    NBSP_BH_KEYS,
+    NBSP_BH_SORT,
+    NBSP_BH_BUILD,
+    NBSP_BH_MOMENTS,
+    NBSP_BH_WALK,
+    NBSP_BH_INTEGRATE,
+    NBSP_BH_END,
+    NBSP_BH_STAMPS
+};
+
 /* Systems of up to this many particles are sorted by nbsp_bh_small_keys and
  * nbsp_bh_small_merge (bh.cu says why). */
 #define NBSP_BH_SMALL_SORT ((size_t)98304)
@@ -101,7 +117,7 @@ NBSP_HIDDEN void nbsp_bh_destroy(NbspBarnesHut* bh);
 NBSP_HIDDEN void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n,
                                 double* partial, double* geometry, int* status, const double* ax,
                                 const double* ay, const double* az, int rms_of_a,
-                                const NbspLeapfrogFusion* leapfrog, cudaStream_t stream);
+                                const NbspLeapfrogFusion* leapfrog, unsigned long long* stamp, cudaStream_t stream);
 /* geometry: root centre [0..2], half side [3], centre of mass [4..6], and with
  * rms_of_a the rms |a| [7] of (ax, ay, az) (the relative test's floor); with a
  * leapfrog fusion (NULL: none) the kick and drift come first and the rest is of
@@ -115,7 +131,7 @@ NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z,
                               void* unsorted, uint32_t* sort_scratch, const double* ax,
                               const double* ay, const double* az, double tol_scale,
                               float* unsorted_tol, void* tree, unsigned long long* counters,
-                              cudaStream_t stream);
+                              unsigned long long* stamp, cudaStream_t stream);
 /* (with unsorted_tol != NULL also the relative opening test's tolerance of each
  * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0;
  * the tree's masks and leaf counts and the 8 counters are set to zero) */
@@ -130,11 +146,11 @@ NBSP_HIDDEN void nbsp_bh_small_keys(const double* x, const double* y, const doub
                                     void* unsorted, const double* ax, const double* ay,
                                     const double* az, double tol_scale, float* unsorted_tol,
                                     void* tree, unsigned long long* counters,
-                                    cudaStream_t stream);
+                                    unsigned long long* stamp, cudaStream_t stream);
 NBSP_HIDDEN void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* index_in, size_t n,
                                      uint64_t* keys, uint32_t* index, const void* unsorted,
                                      void* pos4, const float* unsorted_tol, float* tol,
-                                     int* status, cudaStream_t stream);
+                                     int* status, unsigned long long* stamp, cudaStream_t stream);
 
 /* 32-bit words of sort scratch for n keys (digit histograms, tile
  * tickets and look-back status words), enough for every smaller n too. */
@@ -146,12 +162,12 @@ NBSP_HIDDEN size_t nbsp_bh_sort_scratch_words(size_t n);
  * ends in the first pair. */
 NBSP_HIDDEN void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt,
                               uint32_t* index_alt, size_t n, uint32_t* sort_scratch, int* status,
-                              cudaStream_t stream);
+                              unsigned long long* stamp, cudaStream_t stream);
 
 /* pos4[s] = unsorted[perm[s]] (Morton order), tol[s] = unsorted_tol[perm[s]]. */
 NBSP_HIDDEN void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* pos4,
                                 const float* unsorted_tol, float* tol, int* status,
-                                cudaStream_t stream);
+                                unsigned long long* stamp, cudaStream_t stream);
 
 /* Device-side layout of the tree build scratch; sized by nbsp_bh_tree_bytes. */
 NBSP_HIDDEN size_t nbsp_bh_tree_bytes(size_t n);
@@ -161,7 +177,7 @@ NBSP_HIDDEN size_t nbsp_bh_tree_bytes(size_t n);
  * started by nbsp_bh_keys or nbsp_bh_small_keys. */
 NBSP_HIDDEN void nbsp_bh_build(const uint64_t* keys, const uint32_t* perm, const double* x,
                                const double* y, const double* z, size_t n, int leaf_capacity,
-                               void* tree, int* status, cudaStream_t stream);
+                               void* tree, int* status, unsigned long long* stamp, cudaStream_t stream);
 
 /* Moments + walk-format node records.  order 1 or 2. */
 /* Opening tests: the reference's (2h)^2 < theta^2 d^2 (barnes_hut.c:596-599), or
@@ -179,7 +195,7 @@ enum { NBSP_BH_OPENING_REFERENCE = 0, NBSP_BH_OPENING_OFFSET = 1 };
 NBSP_HIDDEN void nbsp_bh_moments(const void* pos4, const uint64_t* keys, size_t n,
                                  const double* geometry, double theta, double start_theta,
                                  int opening, int quadrupoles, void* tree, int* status,
-                                 cudaStream_t stream);
+                                 unsigned long long* stamp, cudaStream_t stream);
 
 enum { NBSP_BH_WALK_STACKLESS = 0, NBSP_BH_WALK_LISTS = 1, NBSP_BH_WALK_SHARED = 2 };
 
@@ -204,7 +220,7 @@ NBSP_HIDDEN void nbsp_bh_walk(const void* pos4, const float* tol, size_t n, cons
                               int order, int mode, const void* correction,
                               const NbspCorrectionLists* lists, float softening_squared,
                               const uint32_t* perm, void* acc, unsigned long long* counters,
-                              int* status, cudaStream_t stream);
+                              int* status, unsigned long long* stamp, cudaStream_t stream);
 /* (acc: one double4 per particle, stored at the target's input index perm[s];
  * tol != NULL: every opening test also takes the relative test with the
  * per-target tolerances tol, Morton order; correction != NULL: the monopole
@@ -258,7 +274,7 @@ NBSP_HIDDEN const void* nbsp_bh_tree(const NbspBarnesHut* bh);
 NBSP_HIDDEN void nbsp_bh_unsort(const void* acc, size_t n, double gravitational_constant,
                                 double* ax, double* ay, double* az,
                                 const NbspLeapfrogFusion* leapfrog, const void* tree,
-                                unsigned long long* counters, cudaStream_t stream);
+                                unsigned long long* counters, unsigned long long* stamp, cudaStream_t stream);
 /* (with a leapfrog fusion, NULL: none, v is then kicked by half_dt * a; the
  * tree's node_count, leaf_count and depth go to counters[2..4]) */
 

@@ -12,7 +12,8 @@
 #include <stdlib.h>
 #include <string.h>
 
-enum { BH_EVENTS = 8, BH_COUNTERS = 8 };
+/* device words copied after an evaluation: its counters, then its clock stamps */
+enum { BH_WORDS = NBSP_BH_COUNTERS + NBSP_BH_STAMPS };
 /* cells a corrected walk lists per 32-target group for the network; further
  * ones keep the plain monopole (counted in counters[7]) */
 enum { BH_CORRECTION_CAPACITY = 512 };
@@ -36,9 +37,7 @@ struct NbspBarnesHut {
     size_t lists_groups;
     unsigned long long* counters;       /* device */
     unsigned long long* host_counters;  /* pinned */
-    cudaEvent_t events[BH_EVENTS];
-    int timed;                          /* events hold a full evaluation */
-    int unread;                         /* NbspBarnesHutParams.unread of this evaluation */
+    int timed;                          /* host_counters hold a full evaluation */
 };
 
 static NBodySimProStatus bh_fail(NBodySimProError* error, NBodySimProStatus status,
@@ -116,8 +115,6 @@ void nbsp_bh_destroy(NbspBarnesHut* b) {
     release_lists(b);
     cudaFree(b->counters);
     cudaFreeHost(b->host_counters);
-    for (int k = 0; k < BH_EVENTS; ++k)
-        if (b->events[k] != NULL) cudaEventDestroy(b->events[k]);
     free(b);
 }
 
@@ -129,10 +126,9 @@ static NBodySimProStatus ensure(NbspBarnesHut** handle, size_t n, NBodySimProErr
             return bh_fail(error, N_BODY_SIM_PRO_STATUS_OUT_OF_MEMORY, __FILE__, __LINE__,
                            "failed to allocate Barnes-Hut context");
         *handle = b;
-        for (int k = 0; k < BH_EVENTS; ++k) BH_TRY(cudaEventCreate(&b->events[k]));
-        BH_TRY(cudaMalloc((void**)&b->counters, BH_COUNTERS * sizeof(unsigned long long)));
-        BH_TRY(cudaMallocHost((void**)&b->host_counters, BH_COUNTERS * sizeof(unsigned long long)));
-        memset(b->host_counters, 0, BH_COUNTERS * sizeof(unsigned long long));
+        BH_TRY(cudaMalloc((void**)&b->counters, BH_WORDS * sizeof(unsigned long long)));
+        BH_TRY(cudaMallocHost((void**)&b->host_counters, BH_WORDS * sizeof(unsigned long long)));
+        memset(b->host_counters, 0, BH_WORDS * sizeof(unsigned long long));
     }
     if (n <= b->capacity) return N_BODY_SIM_PRO_STATUS_OK;
     release_buffers(b);
@@ -154,44 +150,39 @@ static NBodySimProStatus ensure(NbspBarnesHut** handle, size_t n, NBodySimProErr
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
-/* A phase boundary of an evaluation whose timings are read.  (An event between
- * two kernels holds the second one back; eight of them were a tenth of a step at
- * 10k particles.) */
-static void mark(NbspBarnesHut* b, int event, cudaStream_t stream) {
-    if (!b->unread) cudaEventRecord(b->events[event], stream);
+/* Where a phase of an evaluation leaves its start (NULL: nobody will read it). */
+static unsigned long long* stamp_of(NbspBarnesHut* b, int unread, int phase) {
+    return unread ? NULL : b->counters + NBSP_BH_COUNTERS + phase;
 }
 
 /* The bounds, the sorted keys and permutation, and the walk's records in that
  * order.  tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
 static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, double tol_scale,
-                                int* status, cudaStream_t stream) {
+                                int unread, int* status, cudaStream_t stream) {
     const int rel = tol_scale > 0.0;
     const NbspLeapfrogFusion* lf = s->leapfrog.vx != NULL ? &s->leapfrog : NULL;
     const int with_a = rel || lf != NULL;
     const int small = s->n <= NBSP_BH_SMALL_SORT;
     nbsp_bh_bounds(s->x, s->y, s->z, s->m, s->n, b->partial, small ? NULL : b->geometry, status,
                    with_a ? s->ax : NULL, with_a ? s->ay : NULL, with_a ? s->az : NULL, rel, lf,
-                   stream);
-    mark(b, 1, stream);
+                   stamp_of(b, unread, NBSP_BH_BOUNDS), stream);
     if (small) {
         nbsp_bh_small_keys(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, b->keys_alt,
                            b->index_alt, b->unsorted, s->ax, s->ay, s->az, tol_scale,
-                           rel ? b->tol_unsorted : NULL, b->tree, b->counters, stream);
-        mark(b, 2, stream);
+                           rel ? b->tol_unsorted : NULL, b->tree, b->counters,
+                           stamp_of(b, unread, NBSP_BH_KEYS), stream);
         nbsp_bh_small_merge(b->keys_alt, b->index_alt, s->n, b->keys, b->index, b->unsorted,
                             b->pos4, rel ? b->tol_unsorted : NULL, rel ? b->tol : NULL, status,
-                            stream);
-        mark(b, 3, stream);
+                            stamp_of(b, unread, NBSP_BH_SORT), stream);
         return N_BODY_SIM_PRO_STATUS_OK;
     }
     nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys, b->index, b->unsorted,
                  b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, b->tree,
-                 b->counters, stream);
-    mark(b, 2, stream);
-    nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status, stream);
-    mark(b, 3, stream);
+                 b->counters, stamp_of(b, unread, NBSP_BH_KEYS), stream);
+    nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status,
+                 stamp_of(b, unread, NBSP_BH_SORT), stream);
     nbsp_bh_gather(b->unsorted, b->index, s->n, b->pos4, rel ? b->tol_unsorted : NULL,
-                   rel ? b->tol : NULL, status, stream);
+                   rel ? b->tol : NULL, status, stamp_of(b, unread, NBSP_BH_BUILD), stream);
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
@@ -204,7 +195,7 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     NbspBarnesHut* b = *handle;
     const size_t n = s->n;
-    b->unread = p->unread;
+    const int unread = p->unread;
     if (n == 1) { /* a lone particle feels nothing; no tree to walk */
         BH_TRY(cudaMemsetAsync(s->ax, 0, sizeof(double), stream));
         BH_TRY(cudaMemsetAsync(s->ay, 0, sizeof(double), stream));
@@ -214,35 +205,32 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
         b->timed = 0;
         return N_BODY_SIM_PRO_STATUS_OK;
     }
-    mark(b, 0, stream);
     /* relative opening test: tolerance alpha |a_old| / G */
     const double g = fabs(p->gravitational_constant);
     const double tol_scale = p->tolerance > 0.0 ? (g > 0.0 ? p->tolerance / g : INFINITY) : 0.0;
     if (p->correction != NULL && (st = ensure_lists(b, n, error)) != N_BODY_SIM_PRO_STATUS_OK)
         return st;
     const int rel = tol_scale > 0.0;
-    morton(b, s, tol_scale, status, stream);
+    morton(b, s, tol_scale, unread, status, stream);
     nbsp_bh_build(b->keys, b->index, s->x, s->y, s->z, n, p->leaf_capacity, b->tree, status,
-                  stream);
-    mark(b, 4, stream);
+                  n <= NBSP_BH_SMALL_SORT ? stamp_of(b, unread, NBSP_BH_BUILD) : NULL, stream);
     nbsp_bh_moments(b->pos4, b->keys, n, b->geometry, p->theta,
                     rel ? fmin(p->theta, NBSP_BH_START_THETA) : 0.0, p->opening,
                     p->multipole_order == 2 || p->correction != NULL || p->quadrupoles, b->tree,
-                    status, stream);
-    mark(b, 5, stream);
+                    status, stamp_of(b, unread, NBSP_BH_MOMENTS), stream);
     nbsp_bh_walk(b->pos4, rel ? b->tol : NULL, n, b->tree, p->multipole_order, p->walk_mode,
                  p->correction, p->correction != NULL ? &b->lists : NULL,
-                 (float)p->softening_squared, b->index, b->acc, b->counters, status, stream);
+                 (float)p->softening_squared, b->index, b->acc, b->counters, status,
+                 stamp_of(b, unread, NBSP_BH_WALK), stream);
     if (p->correction != NULL)
         nbsp_bh_correct(b->pos4, n, b->tree, p->correction, &b->lists, b->index, b->acc,
                         b->counters, status, stream);
-    mark(b, 6, stream);
     nbsp_bh_unsort(b->acc, n, p->gravitational_constant, s->ax, s->ay, s->az,
-                   s->leapfrog.vx != NULL ? &s->leapfrog : NULL, b->tree, b->counters, stream);
-    mark(b, 7, stream);
+                   s->leapfrog.vx != NULL ? &s->leapfrog : NULL, b->tree, b->counters,
+                   stamp_of(b, unread, NBSP_BH_INTEGRATE), stream);
     BH_TRY(cudaGetLastError());
-    if (p->unread) return N_BODY_SIM_PRO_STATUS_OK;
-    BH_TRY(cudaMemcpyAsync(b->host_counters, b->counters, BH_COUNTERS * sizeof(unsigned long long),
+    if (unread) return N_BODY_SIM_PRO_STATUS_OK;
+    BH_TRY(cudaMemcpyAsync(b->host_counters, b->counters, BH_WORDS * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, stream));
     b->timed = 1;
     /* stats/timings are read after the caller synchronises */
@@ -255,9 +243,8 @@ const void* nbsp_bh_positions(const NbspBarnesHut* b) { return b != NULL ? b->po
 const void* nbsp_bh_tree(const NbspBarnesHut* b) { return b != NULL ? b->tree : NULL; }
 
 static double elapsed(const NbspBarnesHut* b, int from, int to) {
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, b->events[from], b->events[to]) != cudaSuccess) return 0.0;
-    return (double)ms;
+    const unsigned long long* t = b->host_counters + NBSP_BH_COUNTERS;
+    return t[to] > t[from] ? (double)(t[to] - t[from]) * 1e-6 : 0.0;
 }
 
 void nbsp_bh_collect(NbspBarnesHut* b, NBodySimProBarnesHutStats* stats,
@@ -273,14 +260,14 @@ void nbsp_bh_collect(NbspBarnesHut* b, NBodySimProBarnesHutStats* stats,
     stats->maximum_depth = (size_t)c[4];
     *walk_restarts = (size_t)c[5];
     *corrected_cells = (size_t)c[6];
-    timings->bounds_ms = elapsed(b, 0, 1);
-    timings->keys_ms = elapsed(b, 1, 2);
-    timings->sort_ms = elapsed(b, 2, 3);
-    timings->build_ms = elapsed(b, 3, 4);
-    timings->moments_ms = elapsed(b, 4, 5);
-    timings->walk_ms = elapsed(b, 5, 6);
-    timings->integrate_ms = elapsed(b, 6, 7);
-    timings->total_ms = elapsed(b, 0, 7);
+    timings->bounds_ms = elapsed(b, NBSP_BH_BOUNDS, NBSP_BH_KEYS);
+    timings->keys_ms = elapsed(b, NBSP_BH_KEYS, NBSP_BH_SORT);
+    timings->sort_ms = elapsed(b, NBSP_BH_SORT, NBSP_BH_BUILD);
+    timings->build_ms = elapsed(b, NBSP_BH_BUILD, NBSP_BH_MOMENTS);
+    timings->moments_ms = elapsed(b, NBSP_BH_MOMENTS, NBSP_BH_WALK);
+    timings->walk_ms = elapsed(b, NBSP_BH_WALK, NBSP_BH_INTEGRATE);
+    timings->integrate_ms = elapsed(b, NBSP_BH_INTEGRATE, NBSP_BH_END);
+    timings->total_ms = elapsed(b, NBSP_BH_BOUNDS, NBSP_BH_END);
     stats->build_time_seconds = (timings->total_ms - timings->walk_ms - timings->integrate_ms) * 1e-3;
     stats->evaluation_time_seconds = timings->walk_ms * 1e-3;
 }
@@ -292,9 +279,7 @@ NBodySimProStatus nbsp_bh_morton(NbspBarnesHut** handle, const NbspBarnesHutStat
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     NbspBarnesHut* b = *handle;
     const size_t n = s->n;
-    b->unread = 0;
-    mark(b, 0, stream);
-    morton(b, s, 0.0, status, stream);
+    morton(b, s, 0.0, 1, status, stream);
     BH_TRY(cudaGetLastError());
     uint32_t* perm32 = NULL;
     if (permutation != NULL) {
