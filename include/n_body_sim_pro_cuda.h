@@ -195,7 +195,9 @@ typedef enum NBodySimProCudaAlgorithm {
 } NBodySimProCudaAlgorithm;
 
 /* Per-phase device time of the most recent evaluation, milliseconds: Barnes-Hut
- * phases from the GPU's clock at each phase's start, the rest from CUDA events. */
+ * phases from the GPU's clock at each phase's start (it ticks every 1 to 2 us), the
+ * rest from CUDA events.  A plugin call's wait for its accelerations, which come in
+ * while the tree is built, counts with build_ms. */
 typedef struct NBodySimProCudaTimings {
     double bounds_ms;      /* bbox + centre-of-mass reduction */
     double keys_ms;        /* Morton keys */

@@ -40,34 +40,35 @@ constexpr int kBoundsThreads = 256;
 constexpr int kBoundsBlocks = 4 * 148;  // one wave at 4 blocks of 256 per SM (58 registers)
 constexpr int kBoundsVals = 11;  // min xyz, max xyz, m, mx, my, mz, |a|^2
 
-// The combined values of the block's first kBoundsThreads threads in thread 0:
-// each warp by shuffles, then the warps' results by the first warp.
+// The combined values (from FIRST on) of the block's first kBoundsThreads threads
+// in thread 0: each warp by shuffles, then the warps' results by the first warp.
+template <int FIRST = 0>
 __device__ __forceinline__ void bounds_block_reduce(double (&v)[kBoundsVals],
                                                     double (*sh)[kBoundsThreads / 32]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (w < kBoundsThreads / 32) {
     for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
-      for (int q = 0; q < kBoundsVals; ++q) {
+      for (int q = FIRST; q < kBoundsVals; ++q) {
         const double o = __shfl_xor_sync(0xffffffffu, v[q], off);
         v[q] = q < 3 ? fmin(v[q], o) : q < 6 ? fmax(v[q], o) : v[q] + o;
       }
     }
     if (lane == 0)
 #pragma unroll
-      for (int q = 0; q < kBoundsVals; ++q) sh[q][w] = v[q];
+      for (int q = FIRST; q < kBoundsVals; ++q) sh[q][w] = v[q];
   }
   __syncthreads();
   if (w != 0) return;
 #pragma unroll
-  for (int q = 0; q < kBoundsVals; ++q)
+  for (int q = FIRST; q < kBoundsVals; ++q)
     v[q] = lane < kBoundsThreads / 32 ? sh[q][lane]
            : q < 3                    ? INFINITY
            : q < 6                    ? -INFINITY
                                       : 0.0;
   for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
-    for (int q = 0; q < kBoundsVals; ++q) {
+    for (int q = FIRST; q < kBoundsVals; ++q) {
       const double o = __shfl_xor_sync(0xffffffffu, v[q], off);
       v[q] = q < 3 ? fmin(v[q], o) : q < 6 ? fmax(v[q], o) : v[q] + o;
     }
@@ -84,6 +85,11 @@ __device__ __forceinline__ unsigned long long gpu_clock() {
 }
 __device__ __forceinline__ void stamp_start(unsigned long long* stamp) {
   if (stamp != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *stamp = gpu_clock();
+}
+
+// |a|^2, contracted the same way wherever it is summed.
+__device__ __forceinline__ double square_sum(double x, double y, double z) {
+  return fma(z, z, fma(y, y, x * x));
 }
 
 // KICK: the opening kick and drift of a device-resident leapfrog step first
@@ -131,7 +137,7 @@ __global__ void __launch_bounds__(kBoundsThreads) bounds_kernel(
     v[7] += pm * px;
     v[8] += pm * py;
     v[9] += pm * pz;
-    if (rms_of_a) v[10] += ax[i] * ax[i] + ay[i] * ay[i] + az[i] * az[i];
+    if (rms_of_a) v[10] += square_sum(ax[i], ay[i], az[i]);
   }
   if (bad) atomicOr(status, NBSP_DEVICE_ERROR_NONFINITE_POSITION);
   bounds_block_reduce(v, sh);
@@ -377,9 +383,18 @@ __device__ __forceinline__ void start_tree(const Tree& t, unsigned long long* co
   }
 }
 
+// The relative opening test's alpha max(|a_old|, rms) / G of particle i.
+__device__ __forceinline__ float opening_tolerance(size_t i, const double* __restrict__ ax,
+                                                   const double* __restrict__ ay,
+                                                   const double* __restrict__ az, double rms,
+                                                   double tol_scale) {
+  const double a = fmax(sqrt(square_sum(ax[i], ay[i], az[i])), rms);
+  return a > 0.0 && isfinite(a) ? (float)(tol_scale * a) : INFINITY;
+}
+
 // Particle i's Morton key under root cube `geometry`, and its record for the
 // walk, still in input order: the float4 (relative to the centre of mass) and
-// with `unsorted_tol` the relative opening test's alpha max(|a_old|, rms) / G.
+// with `unsorted_tol` the relative opening test's tolerance.
 __device__ __forceinline__ uint64_t particle_key(
     size_t i, const double* __restrict__ x, const double* __restrict__ y,
     const double* __restrict__ z, const double* __restrict__ m, const double (&geometry)[8],
@@ -388,10 +403,8 @@ __device__ __forceinline__ uint64_t particle_key(
   const double xi = x[i], yi = y[i], zi = z[i];
   unsorted[i] = make_float4((float)__dsub_rn(xi, geometry[4]), (float)__dsub_rn(yi, geometry[5]),
                             (float)__dsub_rn(zi, geometry[6]), (float)m[i]);
-  if (unsorted_tol != nullptr) {
-    const double a = fmax(sqrt(ax[i] * ax[i] + ay[i] * ay[i] + az[i] * az[i]), geometry[7]);
-    unsorted_tol[i] = a > 0.0 && isfinite(a) ? (float)(tol_scale * a) : INFINITY;
-  }
+  if (unsorted_tol != nullptr)
+    unsorted_tol[i] = opening_tolerance(i, ax, ay, az, geometry[7], tol_scale);
   return spread3(axis_code(xi, geometry[0], geometry[3])) |
          (spread3(axis_code(yi, geometry[1], geometry[3])) << 1) |
          (spread3(axis_code(zi, geometry[2], geometry[3])) << 2);
@@ -787,6 +800,48 @@ __global__ void gather_kernel(const float4* __restrict__ unsorted,
     }
     pos[s] = unsorted[i];
     if (tol != nullptr) tol[s] = unsorted_tol[i];
+  }
+}
+
+// The relative test's tolerances of accelerations that were still on their way
+// while the tree was built (pinned upload at 1M particles: 24 MB, 0.44 ms, beside
+// 0.3 ms of bounds, sort and build).  First the blocks' sums of |a|^2 in
+// bounds_kernel's places and order, then, in every block again, their total as
+// root_geometry forms it, and each sorted particle's tolerance.
+__global__ void __launch_bounds__(kBoundsThreads) late_squares_kernel(
+    const double* __restrict__ ax, const double* __restrict__ ay, const double* __restrict__ az,
+    size_t n, double* __restrict__ partial) {
+  __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
+  double v[kBoundsVals];
+  v[10] = 0.0;
+#pragma unroll 4
+  for (size_t i = blockIdx.x * (size_t)kBoundsThreads + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * kBoundsThreads)
+    v[10] += square_sum(ax[i], ay[i], az[i]);
+  bounds_block_reduce<10>(v, sh);
+  if (threadIdx.x == 0) partial[blockIdx.x * kBoundsVals + 10] = v[10];
+}
+
+__global__ void __launch_bounds__(kBoundsThreads) late_tolerances_kernel(
+    const double* __restrict__ ax, const double* __restrict__ ay, const double* __restrict__ az,
+    const double* __restrict__ partial, int blocks, size_t n, double tol_scale,
+    const uint32_t* __restrict__ perm, float* __restrict__ tol, double* __restrict__ geometry) {
+  __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
+  __shared__ double s_rms;
+  double v[kBoundsVals];
+  v[10] = 0.0;
+  for (int b = threadIdx.x; b < blocks; b += kBoundsThreads) v[10] += partial[b * kBoundsVals + 10];
+  bounds_block_reduce<10>(v, sh);
+  if (threadIdx.x == 0) {
+    s_rms = sqrt(v[10] / (double)n);
+    if (blockIdx.x == 0) geometry[7] = s_rms;
+  }
+  __syncthreads();
+  const double rms = s_rms;
+  for (size_t s = blockIdx.x * (size_t)kBoundsThreads + threadIdx.x; s < n;
+       s += (size_t)gridDim.x * kBoundsThreads) {
+    const uint32_t i = perm[s];  // (a bad one is the gather's to report)
+    tol[s] = i < n ? opening_tolerance(i, ax, ay, az, rms, tol_scale) : INFINITY;
   }
 }
 
@@ -3082,6 +3137,16 @@ void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* 
                     cudaStream_t stream) {
   NBSP_COUNT_LAUNCH(1), gather_kernel<<<grid_for(n, 256), 256, 0, stream>>>(
       (const float4*)unsorted, perm, n, (float4*)pos4, unsorted_tol, tol, status, stamp);
+}
+
+void nbsp_bh_late_tolerances(const double* ax, const double* ay, const double* az, size_t n,
+                             double tol_scale, const uint32_t* perm, double* partial, float* tol,
+                             double* geometry, cudaStream_t stream) {
+  const int blocks = bounds_blocks(n);
+  NBSP_COUNT_LAUNCH(1), late_squares_kernel<<<blocks, kBoundsThreads, 0, stream>>>(ax, ay, az, n,
+                                                                                 partial);
+  NBSP_COUNT_LAUNCH(1), late_tolerances_kernel<<<blocks, kBoundsThreads, 0, stream>>>(
+      ax, ay, az, partial, blocks, n, tol_scale, perm, tol, geometry);
 }
 
 size_t nbsp_bh_tree_bytes(size_t n) { return tree_bytes(n); }

@@ -56,12 +56,22 @@ typedef struct NbspLeapfrogFusion {
     double half_dt, dt;
 } NbspLeapfrogFusion;
 
+/* The accelerations the relative test reads, still in the caller's arrays when an
+ * evaluation is enqueued: they come in on a stream of their own, behind what the
+ * evaluation's stream holds at that time, while the tree is built. */
+typedef struct NbspLateAccelerations {
+    const double* source[3];
+    cudaStream_t stream;
+    cudaEvent_t before, after;
+} NbspLateAccelerations;
+
 typedef struct NbspBarnesHutState {
     double *x, *y, *z;  /* written only by a fused drift */
     const double* m;
     double *ax, *ay, *az;
     size_t n;
     NbspLeapfrogFusion leapfrog;
+    const NbspLateAccelerations* late; /* NULL: ax, ay, az are there already */
 } NbspBarnesHutState;
 
 /* Enqueue one full Barnes-Hut force evaluation; accelerations into s->ax/ay/az.
@@ -135,6 +145,13 @@ NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z,
 /* (with unsorted_tol != NULL also the relative opening test's tolerance of each
  * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0;
  * the tree's masks and leaf counts and the 8 counters are set to zero) */
+
+/* geometry[7] and the sorted tolerances of accelerations that came in after the
+ * sort (`partial` is nbsp_bh_bounds's). */
+NBSP_HIDDEN void nbsp_bh_late_tolerances(const double* ax, const double* ay, const double* az,
+                                         size_t n, double tol_scale, const uint32_t* perm,
+                                         double* partial, float* tol, double* geometry,
+                                         cudaStream_t stream);
 
 /* For n <= NBSP_BH_SMALL_SORT, after nbsp_bh_bounds without geometry: geometry,
  * `unsorted` and `unsorted_tol` as nbsp_bh_bounds and nbsp_bh_keys write them,

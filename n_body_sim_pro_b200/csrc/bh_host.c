@@ -150,6 +150,20 @@ static NBodySimProStatus ensure(NbspBarnesHut** handle, size_t n, NBodySimProErr
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
+/* The late accelerations into (ax, ay, az), and `stream` made to wait for them. */
+static cudaError_t fetch_late(const NbspBarnesHutState* s, cudaStream_t stream) {
+    const NbspLateAccelerations* late = s->late;
+    double* const to[3] = {s->ax, s->ay, s->az};
+    cudaError_t code = cudaStreamWaitEvent(late->stream, late->before, 0);
+    for (int k = 0; k < 3 && code == cudaSuccess; ++k)
+        code = cudaMemcpyAsync(to[k], late->source[k], s->n * sizeof(double),
+                               cudaMemcpyHostToDevice, late->stream);
+    if (code == cudaSuccess) code = cudaEventRecord(late->after, late->stream);
+    if (code == cudaSuccess) code = cudaStreamWaitEvent(stream, late->after, 0);
+    if (code != cudaSuccess) cudaStreamSynchronize(late->stream); /* the arrays are the caller's */
+    return code;
+}
+
 /* Where a phase of an evaluation leaves its start (NULL: nobody will read it). */
 static unsigned long long* stamp_of(NbspBarnesHut* b, int unread, int phase) {
     return unread ? NULL : b->counters + NBSP_BH_COUNTERS + phase;
@@ -211,9 +225,16 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     if (p->correction != NULL && (st = ensure_lists(b, n, error)) != N_BODY_SIM_PRO_STATUS_OK)
         return st;
     const int rel = tol_scale > 0.0;
-    morton(b, s, tol_scale, unread, status, stream);
+    const int late = rel && s->late != NULL;
+    if (late) BH_TRY(cudaEventRecord(s->late->before, stream));
+    morton(b, s, late ? 0.0 : tol_scale, unread, status, stream);
     nbsp_bh_build(b->keys, b->index, s->x, s->y, s->z, n, p->leaf_capacity, b->tree, status,
                   n <= NBSP_BH_SMALL_SORT ? stamp_of(b, unread, NBSP_BH_BUILD) : NULL, stream);
+    if (late) {
+        BH_TRY(fetch_late(s, stream));
+        nbsp_bh_late_tolerances(s->ax, s->ay, s->az, n, tol_scale, b->index, b->partial, b->tol,
+                                b->geometry, stream);
+    }
     nbsp_bh_moments(b->pos4, b->keys, n, b->geometry, p->theta,
                     rel ? fmin(p->theta, NBSP_BH_START_THETA) : 0.0, p->opening,
                     p->multipole_order == 2 || p->correction != NULL || p->quadrupoles, b->tree,
