@@ -12,7 +12,8 @@
 // A step of a small minibatch is bound by latency (1024 rows: 8 CTAs, 3e7 flop),
 // so an epoch is one cooperative launch instead of three a step: with it, the
 // ldmatrix fragments and the forward-only losses an epoch of 245,760 rows in
-// steps of 1024, its shuffle and losses included, takes 4.9 ms instead of 8.7.
+// steps of 1024, its shuffle and losses included, takes 3.5 ms instead of 8.7
+// (1.25 of them the shuffle, on the host).
 //
 // Loss: mean squared error over the 3 outputs of the standardised labels,
 // L = 1 / (3 B) sum_r sum_c (y_rc - t_rc)^2.
@@ -74,6 +75,15 @@ __device__ __forceinline__ uint2 load_b(const unsigned short* m, int stride, int
                : "r"(smem_address(m + (row0 + (lane & 15)) * stride + col0))
                : "memory");
   return b;
+}
+
+// Two of them, for columns col0.. and col0 + 8..
+__device__ __forceinline__ void load_b2(const unsigned short* m, int stride, int row0, int col0,
+                                        int lane, uint2* b) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(b[0].x), "=r"(b[0].y), "=r"(b[1].x), "=r"(b[1].y)
+               : "r"(smem_address(m + (row0 + (lane & 15)) * stride + col0 + ((lane >> 4) << 3)))
+               : "memory");
 }
 
 // Store a 16 x 8 C fragment (rows row0.., cols col0..) as BF16.
@@ -149,19 +159,17 @@ __device__ __forceinline__ void rows_pass(Stage& st, const RowInputs& in, int wa
     xs[(lr + g) * (kStrideX / 2) + t + 4] = in.x[2];
     xs[(lr + g + 8) * (kStrideX / 2) + t + 4] = in.x[3];
   }
-  // forward, keeping pre-activations
-  float z1[8][4], z2[8][4];
+  // forward, keeping the activations' derivatives
+  float g1[8][4], g2[8][4];
   uint32_t h1[16], h2[16];
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) {
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     mma_bf16(c, in.x, f.w1[nt * 32 + lane]);
     const float bb0 = f.b1[8 * nt + 2 * t], bb1 = f.b1[8 * nt + 2 * t + 1];
-    z1[nt][0] = c[0] + bb0;
-    z1[nt][1] = c[1] + bb1;
-    z1[nt][2] = c[2] + bb0;
-    z1[nt][3] = c[3] + bb1;
-    float a[4] = {gelu(z1[nt][0]), gelu(z1[nt][1]), gelu(z1[nt][2]), gelu(z1[nt][3])};
+    float a[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] = gelu_with_grad(c[q] + (q & 1 ? bb1 : bb0), g1[nt][q]);
     if (!LOSS_ONLY) store_c(st.h1, kStrideH, lr, 8 * nt, lane, a);
     const int ks = nt >> 1, hi = (nt & 1) * 2;
     h1[4 * ks + hi] = pack_bf16(a[0], a[1]);
@@ -173,11 +181,9 @@ __device__ __forceinline__ void rows_pass(Stage& st, const RowInputs& in, int wa
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &h1[4 * ks], f.w2[(ks * 8 + nt) * 32 + lane]);
     const float bb0 = f.b2[8 * nt + 2 * t], bb1 = f.b2[8 * nt + 2 * t + 1];
-    z2[nt][0] = c[0] + bb0;
-    z2[nt][1] = c[1] + bb1;
-    z2[nt][2] = c[2] + bb0;
-    z2[nt][3] = c[3] + bb1;
-    float a[4] = {gelu(z2[nt][0]), gelu(z2[nt][1]), gelu(z2[nt][2]), gelu(z2[nt][3])};
+    float a[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] = gelu_with_grad(c[q] + (q & 1 ? bb1 : bb0), g2[nt][q]);
     if (!LOSS_ONLY) store_c(st.h2, kStrideH, lr, 8 * nt, lane, a);
     const int ks = nt >> 1, hi = (nt & 1) * 2;
     h2[4 * ks + hi] = pack_bf16(a[0], a[1]);
@@ -214,7 +220,7 @@ __device__ __forceinline__ void rows_pass(Stage& st, const RowInputs& in, int wa
     mma_bf16(c, dya, f.w3t[nt * 32 + lane]);
     float d[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z2[nt][q]);
+    for (int q = 0; q < 4; ++q) d[q] = c[q] * g2[nt][q];
     store_c(st.dz2, kStrideH, lr, 8 * nt, lane, d);
     const int ks = nt >> 1, hi = (nt & 1) * 2;
     dz2a[4 * ks + hi] = pack_bf16(d[0], d[1]);
@@ -228,7 +234,7 @@ __device__ __forceinline__ void rows_pass(Stage& st, const RowInputs& in, int wa
     for (int ks = 0; ks < 4; ++ks) mma_bf16(c, &dz2a[4 * ks], f.w2t[(ks * 8 + nt) * 32 + lane]);
     float d[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) d[q] = c[q] * gelu_grad(z1[nt][q]);
+    for (int q = 0; q < 4; ++q) d[q] = c[q] * g1[nt][q];
     store_c(st.dz1, kStrideH, lr, 8 * nt, lane, d);
   }
 }
@@ -239,8 +245,11 @@ __device__ __forceinline__ float bf16_value(unsigned short b) {
 
 // After rows_pass of all 128 rows and a barrier: the CTA's gradient into its slot
 // `grad`.  Weight gradients on tensor cores, dW = dZ^T H over the 128 rows (8
-// k-steps): output tiles dW2 4 x 8 (32), dW1 4 x 2 (8), dW3 1 x 8 (8), six for
-// each of the first eight warps; the last four sum the bias columns meanwhile.
+// k-steps), by the first eight warps: four of dW2's 4 x 8 output tiles (one row of
+// them, so that they share dZ2's fragment), one of dW1's 4 x 2 and one of dW3's
+// 1 x 8 each, all six sums side by side (one tile after the other the products
+// waited for their own sums: 2.0 us of a step instead of 1.4).  The last four
+// warps sum the bias columns meanwhile.
 __device__ __forceinline__ void weight_gradients(const Stage& st, int warp, int lane, int tid,
                                                  float* __restrict__ grad) {
   const int g = lane >> 2, t = lane & 3;
@@ -259,49 +268,43 @@ __device__ __forceinline__ void weight_gradients(const Stage& st, int warp, int 
     }
     return;
   }
-#pragma unroll 1
-  for (int q = 0; q < 6; ++q) {
-    const int tile = warp + kWarps * q;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    if (tile < 32) {  // dW2[out][in] = sum_r dZ2[r][out] H1[r][in]
-      const int mi = tile >> 3, nj = tile & 7;
+  const int m2 = warp & 3, n2 = (warp >> 2) * 4;  // dW2[out][in] = sum_r dZ2[r][out] H1[r][in]
+  const int m1 = warp >> 1, n1 = warp & 1;        // dW1[out][in] = sum_r dZ1[r][out] X[r][in], in < 10
+  const int n3 = warp;                            // dW3[out][in] = sum_r dY[r][out] H2[r][in], out < 3
+  float c2[4][4] = {}, c1[4] = {}, c3[4] = {};
+#pragma unroll 2
+  for (int r = 0; r < kRows; r += 16) {
+    uint32_t a2[4], a1[4];
+    uint2 b2[4];
+    load_at(st.dz2, kStrideH, r, m2 * 16, lane, a2);
+    load_b2(st.h1, kStrideH, r, n2 * 8, lane, b2);
+    load_b2(st.h1, kStrideH, r, n2 * 8 + 16, lane, b2 + 2);
+    load_at(st.dz1, kStrideH, r, m1 * 16, lane, a1);
+    const uint2 b1 = load_b(st.x, kStrideX, r, n1 * 8, lane);
+    const uint2 y = load_b(st.dy, kStrideY, r, 0, lane);
+    const uint2 b3 = load_b(st.h2, kStrideH, r, n3 * 8, lane);
+    const uint32_t a3[4] = {y.x, 0u, y.y, 0u};  // A[i][k] = dY[k][i], zero for i >= 8
 #pragma unroll
-      for (int ks = 0; ks < kRows / 16; ++ks) {
-        uint32_t a[4];
-        load_at(st.dz2, kStrideH, ks * 16, mi * 16, lane, a);
-        mma_bf16(c, a, load_b(st.h1, kStrideH, ks * 16, nj * 8, lane));
-      }
-      const int o0 = mi * 16 + g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + kOffW2;
-      *reinterpret_cast<float2*>(&gw[o0 * kHidden + i0]) = make_float2(c[0], c[1]);
-      *reinterpret_cast<float2*>(&gw[(o0 + 8) * kHidden + i0]) = make_float2(c[2], c[3]);
-    } else if (tile < 40) {  // dW1[out][in] = sum_r dZ1[r][out] X[r][in], in < 10
-      const int mi = (tile - 32) >> 1, nj = (tile - 32) & 1;
+    for (int j = 0; j < 4; ++j) mma_bf16(c2[j], a2, b2[j]);
+    mma_bf16(c1, a1, b1);
+    mma_bf16(c3, a3, b3);
+  }
 #pragma unroll
-      for (int ks = 0; ks < kRows / 16; ++ks) {
-        uint32_t a[4];
-        load_at(st.dz1, kStrideH, ks * 16, mi * 16, lane, a);
-        mma_bf16(c, a, load_b(st.x, kStrideX, ks * 16, nj * 8, lane));
-      }
-      const int o0 = mi * 16 + g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + kOffW1;
-      if (i0 < kIn) gw[o0 * kIn + i0] = c[0], gw[(o0 + 8) * kIn + i0] = c[2];
-      if (i0 + 1 < kIn) gw[o0 * kIn + i0 + 1] = c[1], gw[(o0 + 8) * kIn + i0 + 1] = c[3];
-    } else {  // dW3[out][in] = sum_r dY[r][out] H2[r][in], out < 3 (M 16 from 8 padded)
-      const int nj = tile - 40;
-#pragma unroll
-      for (int ks = 0; ks < kRows / 16; ++ks) {
-        const uint2 y = load_b(st.dy, kStrideY, ks * 16, 0, lane);
-        const uint32_t a[4] = {y.x, 0u, y.y, 0u};  // A[i][k] = dY[k][i], zero for i >= 8
-        mma_bf16(c, a, load_b(st.h2, kStrideH, ks * 16, nj * 8, lane));
-      }
-      const int o0 = g, i0 = nj * 8 + 2 * t;
-      float* gw = grad + kOffW3;
-      if (o0 < kOut) {
-        gw[o0 * kHidden + i0] = c[0];
-        gw[o0 * kHidden + i0 + 1] = c[1];
-      }
-    }
+  for (int j = 0; j < 4; ++j) {
+    float* gw = grad + kOffW2 + (m2 * 16 + g) * kHidden + (n2 + j) * 8 + 2 * t;
+    *reinterpret_cast<float2*>(gw) = make_float2(c2[j][0], c2[j][1]);
+    *reinterpret_cast<float2*>(gw + 8 * kHidden) = make_float2(c2[j][2], c2[j][3]);
+  }
+  {
+    float* gw = grad + kOffW1;
+    const int o0 = m1 * 16 + g, i0 = n1 * 8 + 2 * t;
+    if (i0 < kIn) gw[o0 * kIn + i0] = c1[0], gw[(o0 + 8) * kIn + i0] = c1[2];
+    if (i0 + 1 < kIn) gw[o0 * kIn + i0 + 1] = c1[1], gw[(o0 + 8) * kIn + i0 + 1] = c1[3];
+  }
+  if (g < kOut) {
+    float* gw = grad + kOffW3 + g * kHidden + n3 * 8 + 2 * t;
+    gw[0] = c3[0];
+    gw[1] = c3[1];
   }
 }
 
@@ -309,7 +312,8 @@ __device__ __forceinline__ void copy_frags(Stage& st, const TrainFrags* f) {
   static_assert(sizeof(TrainFrags) % 16 == 0, "copied as uint4");
   const uint4* src = reinterpret_cast<const uint4*>(f);
   uint4* dst = reinterpret_cast<uint4*>(&st.f);
-  for (int k = threadIdx.x; k < (int)(sizeof(TrainFrags) / 16); k += blockDim.x) dst[k] = src[k];
+  for (int k = threadIdx.x; k < (int)(sizeof(TrainFrags) / 16); k += blockDim.x)
+    dst[k] = __ldcg(src + k);  // (another CTA may have written them in this launch)
 }
 
 // One forward/backward: CTA c's rows first_row + 128 c .. of `order` (NULL: rows
@@ -424,72 +428,65 @@ __device__ __forceinline__ bool grid_arrive_wait(int* arrivals, int* failed, int
 }
 
 // All the steps of an epoch in one cooperative launch, a CTA per 128 rows of the
-// minibatch.  A step ends with every CTA summing all slots (two sets of them, by
-// the step's parity, so that one barrier a step is enough) and updating its own
-// copy of the parameters, moments and fragments — the same arithmetic on the same
-// numbers, so the copies stay equal; the first CTA stores them at the end.
+// minibatch.  A step: every CTA's gradient into its slot; then every CTA sums all
+// slots for its share of the parameters, in the slots' order, updates them and
+// their moments (its own, in shared memory until the end) and puts their new
+// BF16 forms into the fragments in global memory; then every CTA takes those.
+// (Each CTA updating all parameters for itself saves the second wait, but the
+// update is division-bound: 6.3 us of a step at 8 CTAs against 4.0, the second wait
+// and the copy included.)
 // bias: the step's 1 - beta^t for both moments.
 constexpr int kEpochCtas = 32;
 __global__ void __launch_bounds__(kTrainThreads, 1) train_epoch_kernel(
     const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
-    int rows_total, int steps, float inv_batch3, const TrainFrags* __restrict__ f,
-    float* __restrict__ slots, float* __restrict__ params, float* __restrict__ m,
-    float* __restrict__ v, float lr, float beta1, float beta2, float eps,
-    const float2* __restrict__ bias, int* arrivals, int* failed) {
+    int rows_total, int steps, float inv_batch3, TrainFrags* f, float* slots,
+    float* __restrict__ params, float* __restrict__ m, float* __restrict__ v, float lr, float beta1,
+    float beta2, float eps, const float2* __restrict__ bias, int* arrivals, int* failed) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Stage& st = *reinterpret_cast<Stage*>(smem_raw);
   __shared__ int s_ok;
-  // this CTA's parameters and moments
+  // this CTA's share of the parameters and moments
   float* own = reinterpret_cast<float*>(smem_raw + sizeof(Stage));
   float *pp = own, *mm = own + kSlot, *vv = own + 2 * kSlot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ctas = gridDim.x, batch = ctas * kRows;
+  const int share = (kParams + ctas - 1) / ctas;
+  const int first = blockIdx.x * share, last = min(first + share, kParams);
   copy_frags(st, f);
-  for (int p = tid; p < kSlot; p += kTrainThreads) {
-    pp[p] = p < kParams ? params[p] : 0.f;
-    mm[p] = p < kParams ? m[p] : 0.f;
-    vv[p] = p < kParams ? v[p] : 0.f;
+  for (int p = first + tid; p < last; p += kTrainThreads) {
+    pp[p] = params[p];
+    mm[p] = m[p];
+    vv[p] = v[p];
   }
   const int row = blockIdx.x * kRows + warp * 16 + (lane >> 2);
   RowInputs in = {};
   if (warp < kWarps) in = load_rows(x_bf16, y, order, row, rows_total, lane);
   __syncthreads();
   for (int step = 0; step < steps; ++step) {
-    float* set = slots + (size_t)(step & 1) * ctas * kSlot;
     if (warp < kWarps) rows_pass<false>(st, in, warp, lane, inv_batch3);
     __syncthreads();
-    weight_gradients(st, warp, lane, tid, set + (size_t)blockIdx.x * kSlot);
+    weight_gradients(st, warp, lane, tid, slots + (size_t)blockIdx.x * kSlot);
     // the next step's rows are on their way while the CTAs wait for each other
     if (warp < kWarps && step + 1 < steps)
       in = load_rows(x_bf16, y, order, (step + 1) * batch + row, rows_total, lane);
     const float2 b = bias[step];
-    if (!grid_arrive_wait(arrivals, failed, step + 1, &s_ok)) return;
-    for (int group = tid; group < kSlot / 4; group += kTrainThreads) {
-      float gsum[4] = {0.f, 0.f, 0.f, 0.f};
+    if (!grid_arrive_wait(arrivals, failed, 2 * step + 1, &s_ok)) return;
+    for (int p = first + tid; p < last; p += kTrainThreads) {
+      float gsum = 0.f;
 #pragma unroll 8
-      for (int s = 0; s < ctas; ++s) {
-        const float4 d = __ldcg(reinterpret_cast<const float4*>(set + (size_t)s * kSlot) + group);
-        gsum[0] += d.x;
-        gsum[1] += d.y;
-        gsum[2] += d.z;
-        gsum[3] += d.w;
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int p = 4 * group + e;
-        if (p >= kParams) continue;
-        float value = pp[p], mp = mm[p], vp = vv[p];
-        adam(gsum[e], value, mp, vp, lr, beta1, beta2, eps, b.x, b.y);
-        pp[p] = value;
-        mm[p] = mp;
-        vv[p] = vp;
-        put_parameter(st.f, p, value);
-      }
+      for (int s = 0; s < ctas; ++s) gsum += __ldcg(slots + (size_t)s * kSlot + p);
+      float value = pp[p], mp = mm[p], vp = vv[p];
+      adam(gsum, value, mp, vp, lr, beta1, beta2, eps, b.x, b.y);
+      pp[p] = value;
+      mm[p] = mp;
+      vv[p] = vp;
+      put_parameter(*f, p, value);
     }
+    if (!grid_arrive_wait(arrivals, failed, 2 * step + 2, &s_ok)) return;
+    copy_frags(st, f);
     __syncthreads();
   }
-  if (blockIdx.x != 0) return;
-  for (int p = tid; p < kParams; p += kTrainThreads) {
+  for (int p = first + tid; p < last; p += kTrainThreads) {
     params[p] = pp[p];
     m[p] = mm[p];
     v[p] = vv[p];
@@ -707,17 +704,17 @@ void nbsp_mlp_adam_bias(int step, float* bias) {
 }
 
 // `steps` minibatches of ctas * 128 rows of `order` from its start, forward,
-// backward and Adam, in one launch (ctas <= nbsp_mlp_epoch_ctas()); slots: two
-// sets of ctas gradient slots; bias: steps pairs of nbsp_mlp_adam_bias on the
-// device; sync: two zeroed ints, the second nonzero when a wait ran out.  The
-// fragments in `frags` and the inference network are not touched.
+// backward and Adam, in one launch (ctas <= nbsp_mlp_epoch_ctas()); slots: ctas
+// gradient slots; bias: steps pairs of nbsp_mlp_adam_bias on the device; sync: two
+// zeroed ints, the second nonzero when a wait ran out.  The fragments in `frags`
+// follow the parameters; the inference network is not touched.
 int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order, int rows_total,
-                         int steps, int ctas, float inv_batch3, const void* frags, float* slots,
+                         int steps, int ctas, float inv_batch3, void* frags, float* slots,
                          float* params, float* m, float* v, float lr, const void* bias, int* sync,
                          cudaStream_t stream) {
   const int smem = (int)(sizeof(Stage) + 3 * kSlot * sizeof(float));
   cudaFuncSetAttribute(train_epoch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  const TrainFrags* f = (const TrainFrags*)frags;
+  TrainFrags* f = (TrainFrags*)frags;
   const float2* b = (const float2*)bias;
   float beta1 = kBeta1, beta2 = kBeta2, eps = kAdamEps;
   int* failed = sync + 1;

@@ -128,12 +128,13 @@ __device__ __forceinline__ uint32_t gelu2_bf16(float z0, float z1, float b0, flo
   return pack_bf16(g0, g1);
 }
 
-// d gelu / dx
-__device__ __forceinline__ float gelu_grad(float x) {
+// gelu(x), with its derivative at x in `grad`: one hyperbolic tangent for both.
+__device__ __forceinline__ float gelu_with_grad(float x, float& grad) {
   const float u = kGeluC * fmaf(kGeluA * x * x, x, x);
   const float th = tanh_hw(u);
   const float du = kGeluC * fmaf(3.f * kGeluA, x * x, 1.f);
-  return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * du;
+  grad = 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * du;
+  return 0.5f * x * (1.f + th);
 }
 
 // Forward pass of one 16-row tile held as an A fragment (x: 16 x 16 BF16,

@@ -39,7 +39,7 @@ NBSP_HIDDEN void nbsp_mlp_loss(const uint32_t* x, const float* y, int first_row,
 NBSP_HIDDEN void nbsp_mlp_adam_bias(int step, float* bias);
 NBSP_HIDDEN int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order,
                                      int rows_total, int steps, int ctas, float inv_batch3,
-                                     const void* frags, float* slots, float* params, float* m,
+                                     void* frags, float* slots, float* params, float* m,
                                      float* v, float lr, const void* bias, int* sync,
                                      cudaStream_t stream);
 NBSP_HIDDEN void nbsp_mlp_reduce_adam(const float* partial, int slots, float* grad_out,
@@ -365,7 +365,7 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
     const int steps = (int)(n / (size_t)batch);
     /* an epoch in one cooperative launch, up to the minibatch its blocks sum */
     const int one_launch = ctas <= nbsp_mlp_epoch_ctas() && steps > 0;
-    NBodySimProStatus st = ensure_slots(c, one_launch ? 2 * ctas : ctas, error);
+    NBodySimProStatus st = ensure_slots(c, ctas, error);
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
     if (one_launch && steps > c->bias_steps) {
         cudaFree(c->bias);
