@@ -12,8 +12,8 @@
 // A step of a small minibatch is bound by latency (1024 rows: 8 CTAs, 3e7 flop),
 // so an epoch is one cooperative launch instead of three a step: with it, the
 // ldmatrix fragments and the forward-only losses an epoch of 245,760 rows in
-// steps of 1024, its shuffle and losses included, takes 3.5 ms instead of 8.7
-// (1.25 of them the shuffle, on the host).
+// steps of 1024, its shuffle and losses included, takes 3.1 ms instead of 8.7
+// (1.2 of them the shuffle, on the host).
 //
 // Loss: mean squared error over the 3 outputs of the standardised labels,
 // L = 1 / (3 B) sum_r sum_c (y_rc - t_rc)^2.
@@ -308,12 +308,25 @@ __device__ __forceinline__ void weight_gradients(const Stage& st, int warp, int 
   }
 }
 
+// (all of a thread's words in flight at once; another CTA may have written them in
+// this launch)
+template <int THREADS>
 __device__ __forceinline__ void copy_frags(Stage& st, const TrainFrags* f) {
   static_assert(sizeof(TrainFrags) % 16 == 0, "copied as uint4");
+  constexpr int kWords = (int)(sizeof(TrainFrags) / 16), kEach = (kWords + THREADS - 1) / THREADS;
   const uint4* src = reinterpret_cast<const uint4*>(f);
   uint4* dst = reinterpret_cast<uint4*>(&st.f);
-  for (int k = threadIdx.x; k < (int)(sizeof(TrainFrags) / 16); k += blockDim.x)
-    dst[k] = __ldcg(src + k);  // (another CTA may have written them in this launch)
+  uint4 v[kEach];
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int k = (int)threadIdx.x + j * THREADS;
+    if (k < kWords) v[j] = __ldcg(src + k);
+  }
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int k = (int)threadIdx.x + j * THREADS;
+    if (k < kWords) dst[k] = v[j];
+  }
 }
 
 // One forward/backward: CTA c's rows first_row + 128 c .. of `order` (NULL: rows
@@ -325,7 +338,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_step_kernel(
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Stage& st = *reinterpret_cast<Stage*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  copy_frags(st, f);
+  copy_frags<kTrainThreads>(st, f);
   RowInputs in = {};
   if (warp < kWarps)
     in = load_rows(x_bf16, y, order, first_row + blockIdx.x * kRows + warp * 16 + (lane >> 2),
@@ -349,7 +362,7 @@ __global__ void __launch_bounds__(kRows * 2) loss_kernel(
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Stage& st = *reinterpret_cast<Stage*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  copy_frags(st, f);
+  copy_frags<kRows * 2>(st, f);
   __syncthreads();
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const RowInputs in =
@@ -427,63 +440,129 @@ __device__ __forceinline__ bool grid_arrive_wait(int* arrivals, int* failed, int
   return *s_ok != 0;
 }
 
-// All the steps of an epoch in one cooperative launch, a CTA per 128 rows of the
-// minibatch.  A step: every CTA's gradient into its slot; then every CTA sums all
+// The same between the CTAs of one cluster by its hardware barrier (which cannot
+// run out): 1.4 us a wait become 0.7 at 8 CTAs.
+__device__ __forceinline__ bool epoch_wait(bool one_cluster, int* arrivals, int* failed, int round,
+                                           int* s_ok) {
+  if (!one_cluster) return grid_arrive_wait(arrivals, failed, round, s_ok);
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  return true;
+}
+
+// A step's rows on their way to the warps that carry them: 8 words of BF16
+// features, 3 labels, 1 if the row exists.  Rows of 12 words: the eight rows of an
+// A fragment's words lie in different banks.  The four warps without rows of their
+// own fetch the next step's during a pass (three dependent loads, 1.2 us where
+// the pass's warps made them).
+constexpr int kRowWords = 12;
+__device__ __forceinline__ void fetch_row(uint32_t* rows, int c, const uint32_t* __restrict__ x_bf16,
+                                          const float* __restrict__ y,
+                                          const int* __restrict__ order, int r, int rows_total) {
+  uint32_t* to = rows + c * kRowWords;
+  uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a, l = a;
+  if (r < rows_total) {
+    const int s = order[r];
+    const uint4* x = reinterpret_cast<const uint4*>(x_bf16 + (size_t)s * 8);
+    a = x[0];
+    b = x[1];
+    l = make_uint4(__float_as_uint(y[s * 3]), __float_as_uint(y[s * 3 + 1]),
+                   __float_as_uint(y[s * 3 + 2]), 1u);
+  }
+  *reinterpret_cast<uint4*>(to) = a;
+  *reinterpret_cast<uint4*>(to + 4) = b;
+  *reinterpret_cast<uint4*>(to + 8) = l;
+}
+__device__ __forceinline__ RowInputs fetched_rows(const uint32_t* rows, int warp, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const uint32_t* r0 = rows + (warp * 16 + g) * kRowWords;
+  const uint32_t* r1 = r0 + 8 * kRowWords;
+  RowInputs in;
+  in.x[0] = r0[t];
+  in.x[1] = r1[t];
+  in.x[2] = r0[t + 4];
+  in.x[3] = r1[t + 4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int col = 2 * t + (q & 1);
+    in.label[q] = col < kOut ? __uint_as_float((q < 2 ? r0 : r1)[8 + col]) : 0.f;
+  }
+  in.v0 = r0[11] != 0u;
+  in.v1 = r1[11] != 0u;
+  return in;
+}
+
+// All the steps of an epoch in one launch (one cluster, or a cooperative launch),
+// a CTA per 128 rows of the minibatch.  A step: every CTA's gradient into its slot; then every CTA sums all
 // slots for its share of the parameters, in the slots' order, updates them and
 // their moments (its own, in shared memory until the end) and puts their new
 // BF16 forms into the fragments in global memory; then every CTA takes those.
 // (Each CTA updating all parameters for itself saves the second wait, but the
-// update is division-bound: 6.3 us of a step at 8 CTAs against 4.0, the second wait
+// update is division-bound: 6.3 us of a step at 8 CTAs against 2.4, the second wait
 // and the copy included.)
 // bias: the step's 1 - beta^t for both moments.
 constexpr int kEpochCtas = 32;
+constexpr int kEpochCluster = 8;  // the largest cluster that every GPU can place
 __global__ void __launch_bounds__(kTrainThreads, 1) train_epoch_kernel(
     const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
     int rows_total, int steps, float inv_batch3, TrainFrags* f, float* slots,
     float* __restrict__ params, float* __restrict__ m, float* __restrict__ v, float lr, float beta1,
-    float beta2, float eps, const float2* __restrict__ bias, int* arrivals, int* failed) {
+    float beta2, float eps, const float2* __restrict__ bias, int* arrivals, int* failed,
+    int one_cluster) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Stage& st = *reinterpret_cast<Stage*>(smem_raw);
   __shared__ int s_ok;
   // this CTA's share of the parameters and moments
   float* own = reinterpret_cast<float*>(smem_raw + sizeof(Stage));
   float *pp = own, *mm = own + kSlot, *vv = own + 2 * kSlot;
+  uint32_t* rows = reinterpret_cast<uint32_t*>(own + 3 * kSlot);  // two steps' by parity
+  constexpr int kStepRows = kRows * kRowWords;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ctas = gridDim.x, batch = ctas * kRows;
   const int share = (kParams + ctas - 1) / ctas;
   const int first = blockIdx.x * share, last = min(first + share, kParams);
-  copy_frags(st, f);
+  copy_frags<kTrainThreads>(st, f);
   for (int p = first + tid; p < last; p += kTrainThreads) {
     pp[p] = params[p];
     mm[p] = m[p];
     vv[p] = v[p];
   }
-  const int row = blockIdx.x * kRows + warp * 16 + (lane >> 2);
-  RowInputs in = {};
-  if (warp < kWarps) in = load_rows(x_bf16, y, order, row, rows_total, lane);
+  const int c = tid - kWarps * 32;  // the fetching threads' row
+  const int row = blockIdx.x * kRows + c;
+  if (c >= 0) fetch_row(rows, c, x_bf16, y, order, row, rows_total);
   __syncthreads();
   for (int step = 0; step < steps; ++step) {
-    if (warp < kWarps) rows_pass<false>(st, in, warp, lane, inv_batch3);
+    if (warp < kWarps)
+      rows_pass<false>(st, fetched_rows(rows + (step & 1) * kStepRows, warp, lane), warp, lane,
+                       inv_batch3);
+    else if (step + 1 < steps)
+      fetch_row(rows + ((step + 1) & 1) * kStepRows, c, x_bf16, y, order, (step + 1) * batch + row,
+                rows_total);
     __syncthreads();
     weight_gradients(st, warp, lane, tid, slots + (size_t)blockIdx.x * kSlot);
-    // the next step's rows are on their way while the CTAs wait for each other
-    if (warp < kWarps && step + 1 < steps)
-      in = load_rows(x_bf16, y, order, (step + 1) * batch + row, rows_total, lane);
     const float2 b = bias[step];
-    if (!grid_arrive_wait(arrivals, failed, 2 * step + 1, &s_ok)) return;
-    for (int p = first + tid; p < last; p += kTrainThreads) {
-      float gsum = 0.f;
+    if (!epoch_wait(one_cluster, arrivals, failed, 2 * step + 1, &s_ok)) return;
+    for (int p0 = first + tid; p0 < last; p0 += 2 * kTrainThreads) {  // two at a time
+      const int p1 = min(p0 + kTrainThreads, last - 1);
+      float gsum[2] = {0.f, 0.f};
 #pragma unroll 8
-      for (int s = 0; s < ctas; ++s) gsum += __ldcg(slots + (size_t)s * kSlot + p);
-      float value = pp[p], mp = mm[p], vp = vv[p];
-      adam(gsum, value, mp, vp, lr, beta1, beta2, eps, b.x, b.y);
-      pp[p] = value;
-      mm[p] = mp;
-      vv[p] = vp;
-      put_parameter(*f, p, value);
+      for (int s = 0; s < ctas; ++s) {
+        gsum[0] += __ldcg(slots + (size_t)s * kSlot + p0);
+        gsum[1] += __ldcg(slots + (size_t)s * kSlot + p1);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int p = p0 + e * kTrainThreads;
+        if (p >= last) break;
+        float value = pp[p], mp = mm[p], vp = vv[p];
+        adam(gsum[e], value, mp, vp, lr, beta1, beta2, eps, b.x, b.y);
+        pp[p] = value;
+        mm[p] = mp;
+        vv[p] = vp;
+        put_parameter(*f, p, value);
+      }
     }
-    if (!grid_arrive_wait(arrivals, failed, 2 * step + 2, &s_ok)) return;
-    copy_frags(st, f);
+    if (!epoch_wait(one_cluster, arrivals, failed, 2 * step + 2, &s_ok)) return;
+    copy_frags<kTrainThreads>(st, f);
     __syncthreads();
   }
   for (int p = first + tid; p < last; p += kTrainThreads) {
@@ -712,17 +791,34 @@ int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order, in
                          int steps, int ctas, float inv_batch3, void* frags, float* slots,
                          float* params, float* m, float* v, float lr, const void* bias, int* sync,
                          cudaStream_t stream) {
-  const int smem = (int)(sizeof(Stage) + 3 * kSlot * sizeof(float));
+  const int smem =
+      (int)(sizeof(Stage) + 3 * kSlot * sizeof(float) + 2 * kRows * kRowWords * sizeof(uint32_t));
   cudaFuncSetAttribute(train_epoch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   TrainFrags* f = (TrainFrags*)frags;
   const float2* b = (const float2*)bias;
   float beta1 = kBeta1, beta2 = kBeta2, eps = kAdamEps;
   int* failed = sync + 1;
+  int one_cluster = ctas <= kEpochCluster;
   void* args[] = {&x, &y, &order, &rows_total, &steps, &inv_batch3, &f, &slots, &params, &m, &v,
-                  &lr, &beta1, &beta2, &eps, &b, &sync, &failed};
+                  &lr, &beta1, &beta2, &eps, &b, &sync, &failed, &one_cluster};
+  cudaLaunchAttribute how;
+  if (one_cluster) {
+    how.id = cudaLaunchAttributeClusterDimension;
+    how.val.clusterDim.x = (unsigned)ctas;
+    how.val.clusterDim.y = how.val.clusterDim.z = 1;
+  } else {
+    how.id = cudaLaunchAttributeCooperative;
+    how.val.cooperative = 1;
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)ctas);
+  config.blockDim = dim3(kTrainThreads);
+  config.dynamicSmemBytes = (size_t)smem;
+  config.stream = stream;
+  config.attrs = &how;
+  config.numAttrs = 1;
   NBSP_COUNT_LAUNCH(1);
-  return (int)cudaLaunchCooperativeKernel((const void*)train_epoch_kernel, dim3((unsigned)ctas),
-                                          dim3(kTrainThreads), args, (size_t)smem, stream);
+  return (int)cudaLaunchKernelExC(&config, (const void*)train_epoch_kernel, args);
 }
 
 void nbsp_mlp_evaluate(const void* net, const float* feat, int rows, float* out, int tcgen05,
