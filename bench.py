@@ -794,8 +794,8 @@ def stage_bandwidth(phases, stats_acc, n, m, peaks, peak_kind):
         # keys: read x, y, z, m; write key 8, index 4, the walk's float4 16
         # (+ read a_old 24, write the relative tolerance 4)
         ("keys", "keys_ms", (32.0 + 28.0 + (28.0 if rel else 0.0)) * n),
-        # 8 LSD passes over (key 8 + index 4), read and written
-        ("sort", "sort_ms", 8 * 24.0 * n),
+        # 7 LSD passes over (key 8 + index 4), read and written
+        ("sort", "sort_ms", 7 * 24.0 * n),
         ("moments", "moments_ms", mom_bytes),
         # unsort + closing kick: read the walk's double4 (32 B, input order) and
         # v 24; write ax/ay/az 24 and v 24
@@ -817,7 +817,7 @@ def stage_bandwidth(phases, stats_acc, n, m, peaks, peak_kind):
                                 "timed_as": "step total minus the Barnes-Hut phases"}
     stages["_note"] = (f"HBM peak {hbm} GB/s ({peak_kind} MEASURED_PEAKS.json); bytes per "
                        "particle: bounds with the opening kick and drift 80 read + 48 written, "
-                       "keys 32 read + 28 written (+28 relative), sort 8 passes x (12 + 12), "
+                       "keys 32 read + 28 written (+28 relative), sort 7 passes x (12 + 12), "
                        "moments " + ("2 x 16 + 328 per node" if quad else "16 + 180 per node")
                        + ", unsort with the closing kick 56 read + 48 written")
     return stages

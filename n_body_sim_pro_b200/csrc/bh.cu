@@ -6,7 +6,7 @@
 //
 // The Morton keys and the sort permutation are bit-exact with the reference:
 // all FP64 arithmetic of the root cube and of morton_axis_code is done with
-// explicitly rounded __d*_rn intrinsics (no contraction), and the 8 x 8-bit
+// explicitly rounded __d*_rn intrinsics (no contraction), and the 7 x 9-bit
 // stable LSD sort yields the same permutation as the reference's stable
 // 3 x 21-bit LSD sort (a stable sort by the full key, ties by original index).
 //
@@ -310,11 +310,10 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v) {
 }
 
 // ---------------------------------------------------------------------------
-// stable LSD radix sort, 8-bit digits, one kernel per pass
+// stable LSD radix sort, 9-bit digits, one kernel per pass
 //
-// The keys kernel also counts the 8 digit histograms (one read of the keys);
-// one block turns them into each pass's digit bases.  Every pass is then a
-// single kernel: tiles take tickets in launch order, rank their keys in shared
+// The keys kernel also counts the 7 digit histograms (one read of the keys), which
+// every tile scans for the digits' bases.  Every pass is a single kernel: tiles take tickets in launch order, rank their keys in shared
 // memory, and find their global offsets with a decoupled look-back over the
 // preceding tiles' published digit counts (flag A: this tile's count, flag P:
 // inclusive prefix).  A tile only waits on tiles with earlier tickets, which
@@ -322,9 +321,10 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v) {
 // runs out.
 // ---------------------------------------------------------------------------
 
-// A tile is THREADS x ITEMS keys.  Large systems: 512 threads of 8 keys (at 10M
-// keys 0.92 ms for the 8 passes against 1.10 with 256 x 16, whose ranking chain
-// per warp is twice as long, and 1.17 with 1024 x 4, one block per SM).  Below
+// A tile is THREADS x ITEMS keys (the figures are of passes by 8-bit digits).
+// Large systems: 512 threads of 8 keys (at 10M keys 0.92 ms for the 8 passes
+// against 1.10 with 256 x 16, whose ranking chain per warp is twice as long, and
+// 1.17 with 1024 x 4, one block per SM).  Below
 // kSortWide keys those tiles leave SMs idle and a pass is one tile's chain of
 // load, rank, look back and scatter: 512 threads of 4 keys take 78 us for the 8
 // passes at 100k-150k and 91 at 262k (wide tiles: 97 and 109; 256 x 4: 79 and
@@ -336,24 +336,30 @@ struct SortNarrow {
   static constexpr int kThreads = 512, kItems = 4, kBlocks = 2;
 };
 constexpr size_t kSortWide = 450000;
-constexpr int kRadix = 256;
+// Digits of nine bits: seven passes over the 63-bit keys, a digit a thread of the
+// tile in its look-back.  Against eight passes of 256 digits: 70 and 76 us at 98k
+// keys, 82 and 92 at 262k, 147 and 152 at 1M, 882 and 934 at 10M.
+constexpr int kRadixBits = 9, kRadix = 1 << kRadixBits;
 constexpr int kLookback = 8;  // predecessors' flags read at once in the look-back
 template <class S>
 constexpr int sort_tile() {
   static_assert(S::kThreads >= kRadix, "one thread per digit");
   return S::kThreads * S::kItems;
 }
-constexpr int kSortPasses = 8;
+constexpr int kSortPasses = 63 / kRadixBits;
 constexpr uint32_t kFlagA = 1u << 30, kFlagP = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr int kLookbackSpins = 1 << 22;  // ~ms per predecessor before the error flag
 constexpr int kKeysBlocks = 5 * 148;  // 40 warps per SM (48 registers): enough loads in flight
 
-// Sort scratch (32-bit words): hist[8][256] | ticket[8] | status[8][tiles][256]
+// Sort scratch (32-bit words): hist[7][512] | ticket[7] | status[7][tiles][512]
 struct SortScratch {
   uint32_t* hist;
   uint32_t* ticket;
   uint32_t* status;
 };
+__device__ __forceinline__ unsigned sort_digit(uint64_t key, int shift) {
+  return (unsigned)(key >> shift) & (unsigned)(kRadix - 1);
+}
 inline size_t sort_tiles(size_t n) {
   const size_t tile = n < kSortWide ? sort_tile<SortNarrow>() : sort_tile<SortWide>();
   return (n + tile - 1) / tile;
@@ -440,14 +446,14 @@ __global__ void __launch_bounds__(256) keys_kernel(
       tree.mask[i] = 0;
     }
 #pragma unroll
-    // digit counts: the low six bytes of the keys of one warp are spread over
-    // many values (plain shared atomics); the top two bytes (the first octree
-    // levels) repeat, so they are aggregated per warp first
+    // digit counts: the low digits of the keys of one warp are spread over many
+    // values (plain shared atomics); the top two (the first six octree levels)
+    // repeat, so they are aggregated per warp first
     for (int p = 0; p < kSortPasses; ++p) {
-      if (p < 6) {
-        if (valid) atomicAdd(&h[p][(unsigned)(key >> (8 * p)) & 0xffu], 1u);
+      if (p < kSortPasses - 2) {
+        if (valid) atomicAdd(&h[p][sort_digit(key, kRadixBits * p)], 1u);
       } else {
-        const unsigned d = valid ? (unsigned)(key >> (8 * p)) & 0xffu : 0x100u;
+        const unsigned d = valid ? sort_digit(key, kRadixBits * p) : kRadix;
         const unsigned peers = __match_any_sync(kFull, d);
         if (valid && lane == (unsigned)(__ffs(peers) - 1)) atomicAdd(&h[p][d], (uint32_t)__popc(peers));
       }
@@ -478,15 +484,15 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t* sk = reinterpret_cast<uint64_t*>(smem);                     // kSortTile
   uint32_t* sv = reinterpret_cast<uint32_t*>(sk + kSortTile);           // kSortTile
-  uint32_t* wc = sv + kSortTile;                                        // kSortWarps * 256
-  uint32_t* start = wc + kSortWarps * kRadix;                           // 256
-  uint32_t* gofs = start + kRadix;                                      // 256
+  uint32_t* wc = sv + kSortTile;                                        // kSortWarps * kRadix
+  uint32_t* start = wc + kSortWarps * kRadix;                           // kRadix
+  uint32_t* gofs = start + kRadix;                                      // kRadix
   __shared__ int s_tile;
   __shared__ uint32_t s_hsum[kRadix / 32];
 
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
   if (t == 0) s_tile = (int)atomicAdd(ticket, 1u);
-  uint32_t digit_base = 0;  // threads t < 256: keys of smaller digits
+  uint32_t digit_base = 0;  // threads t < kRadix: keys of smaller digits
   if (t < kRadix) {
     const uint32_t own = hist[t];
     uint32_t x = own;
@@ -516,7 +522,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
 #pragma unroll
   for (int it = 0; it < kSortItems; ++it) {
     const bool valid = base_i + (size_t)it * 32 + lane < n;
-    const unsigned digit = valid ? ((unsigned)(key[it] >> shift) & 0xffu) : 0x100u;
+    const unsigned digit = valid ? sort_digit(key[it], shift) : kRadix;
     const unsigned peers = __match_any_sync(kFull, digit);
     uint32_t before = 0;
     if (valid) before = wc[w * kRadix + digit];
@@ -526,7 +532,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
     rank[it] = before + __popc(peers & lt);
   }
   __syncthreads();
-  // threads t < 256: digit t — this tile's count, publish, look back, and the
+  // threads t < kRadix: digit t — this tile's count, publish, look back, and the
   // exclusive scan of the tile's digit totals (warp shuffles, then warp sums)
   __shared__ uint32_t s_wsum[kRadix / 32];
   if (t < kRadix) {
@@ -590,7 +596,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
   for (int it = 0; it < kSortItems; ++it) {
     const size_t i = base_i + (size_t)it * 32 + lane;
     if (i < n) {
-      const unsigned digit = (unsigned)(key[it] >> shift) & 0xffu;
+      const unsigned digit = sort_digit(key[it], shift);
       const uint32_t pos = start[digit] + wc[w * kRadix + digit] + rank[it];
       if (pos < (uint32_t)kSortTile) {
         sk[pos] = key[it];
@@ -605,7 +611,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks) sort_pass_kernel(
   const int count_all = (int)(n - tile_base < (size_t)kSortTile ? n - tile_base : (size_t)kSortTile);
   for (int q = t; q < count_all; q += kSortThreads) {
     const uint64_t k = sk[q];
-    const unsigned digit = (unsigned)(k >> shift) & 0xffu;
+    const unsigned digit = sort_digit(k, shift);
     const size_t dst = (size_t)gofs[digit] + (size_t)(q - (int)start[digit]);
     if (dst < n) {
       keys_out[dst] = k;
@@ -625,7 +631,7 @@ constexpr size_t sort_pass_smem() {
 // ---------------------------------------------------------------------------
 // the same sort for up to NBSP_BH_SMALL_SORT keys: two kernels
 //
-// Eight passes of the radix sort are eight chains of load, rank, look back and
+// Seven passes of the radix sort are seven chains of load, rank, look back and
 // scatter on a few tiles, about 10 us each however few keys there are.  Here
 // every CTA computes the keys of one tile of 1024 particles (and first, from the
 // bounds' partial results, the root cube) and sorts them in a bitonic network,
@@ -3114,13 +3120,14 @@ void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t*
   cudaFuncSetAttribute(pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const SortScratch sc = sort_scratch(scratch);
   const size_t tiles = sort_tiles(n);
-  uint64_t* kin = keys;
-  uint32_t* vin = index;
-  uint64_t* kout = keys_alt;
-  uint32_t* vout = index_alt;
+  static_assert(kSortPasses % 2 == 1, "from (keys_alt, index_alt) to (keys, index)");
+  uint64_t* kin = keys_alt;
+  uint32_t* vin = index_alt;
+  uint64_t* kout = keys;
+  uint32_t* vout = index;
   for (int pass = 0; pass < kSortPasses; ++pass) {
     NBSP_COUNT_LAUNCH(1), pass_kernel<<<(unsigned)tiles, threads, smem, stream>>>(
-        kin, vin, kout, vout, n, 8 * pass, sc.hist + pass * kRadix, sc.ticket + pass,
+        kin, vin, kout, vout, n, kRadixBits * pass, sc.hist + pass * kRadix, sc.ticket + pass,
         sc.status + (size_t)pass * tiles * kRadix, status, pass == 0 ? stamp : nullptr);
     uint64_t* tk = kin;
     kin = kout;
@@ -3129,7 +3136,6 @@ void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t*
     vin = vout;
     vout = tv;
   }
-  // kSortPasses = 8 (even): the result is back in (keys, index)
 }
 
 void nbsp_bh_gather(const void* unsorted, const uint32_t* perm, size_t n, void* pos4,

@@ -5,7 +5,7 @@
  * Pipeline per force evaluation (all on one stream, no host synchronisation):
  *   bounds      FP64 bbox -> root cube (barnes_hut.c:453-483) + centre of mass
  *   keys        63-bit Morton keys, bit-exact with barnes_hut.c:286-305
- *   sort        stable LSD radix sort, 8 x 8-bit digits (same permutation as
+ *   sort        stable LSD radix sort, 7 x 9-bit digits (same permutation as
  *               the reference's 3 x 21-bit LSD sort, barnes_hut.c:312-339)
  *   gather      float4 (x - com, m) in Morton order
  *   build       binary radix tree over the sorted keys (one thread per
@@ -133,7 +133,7 @@ NBSP_HIDDEN void nbsp_bh_bounds(double* x, double* y, double* z, const double* m
  * leapfrog fusion (NULL: none) the kick and drift come first and the rest is of
  * the drifted positions */
 
-/* Morton keys, the identity index, the 8 digit histograms (into sort_scratch)
+/* Morton keys, the identity index, the 7 digit histograms (into sort_scratch)
  * and the walk's float4 (x - c, y - c, z - c, m) with c the centre of mass, in
  * input order (`unsorted`, n entries). */
 NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z, const double* m,
@@ -173,10 +173,9 @@ NBSP_HIDDEN void nbsp_bh_small_merge(const uint64_t* keys_in, const uint32_t* in
  * tickets and look-back status words), enough for every smaller n too. */
 NBSP_HIDDEN size_t nbsp_bh_sort_scratch_words(size_t n);
 
-/* Stable LSD radix sort of (keys, index) by all 64 key bits, after nbsp_bh_keys
- * filled `sort_scratch` (nbsp_bh_sort_scratch_words(n) words) on the same stream.
- * `keys`/`index` are ping-ponged with `keys_alt`/`index_alt`; the sorted result
- * ends in the first pair. */
+/* Stable LSD radix sort of (keys_alt, index_alt) by all 63 key bits into (keys,
+ * index), after nbsp_bh_keys filled the first pair and `sort_scratch`
+ * (nbsp_bh_sort_scratch_words(n) words) on the same stream; both pairs are written. */
 NBSP_HIDDEN void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt,
                               uint32_t* index_alt, size_t n, uint32_t* sort_scratch, int* status,
                               unsigned long long* stamp, cudaStream_t stream);

@@ -190,7 +190,7 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
                             stamp_of(b, unread, NBSP_BH_SORT), stream);
         return N_BODY_SIM_PRO_STATUS_OK;
     }
-    nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys, b->index, b->unsorted,
+    nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys_alt, b->index_alt, b->unsorted,
                  b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, b->tree,
                  b->counters, stamp_of(b, unread, NBSP_BH_KEYS), stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status,
