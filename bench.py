@@ -769,25 +769,24 @@ def run_bh(args, wl, world, rank, local, steps, warmup, with_e2e=True):
 
 def stage_bandwidth(phases, stats_acc, n, m, peaks, peak_kind):
     """Achieved HBM bandwidth of the tree-build stages and the integration, from
-    the library's per-phase CUDA events and the algorithmic bytes per particle
+    the library's phase timings and the algorithmic bytes per particle
     (and per node) of each stage."""
     hbm = float(peaks.get("hbm_gbs", 6650.0))
     nodes = float(stats_acc[-1]["node_count"])
     rel = m["relative_alpha"] > 0.0
     quad = m["multipole_order"] == 2 or m["corrected"]
     # moments: the monopole pass reads each particle once (16 B); per node it
-    # writes 100 B (FP64 moments 32, the centre-of-mass float4 16, ropen2, side,
-    # shift and the cell term 16, the walk's 32-byte record, the height 4) and
-    # reads 76 (its record 16, level 4, first key 8; as a child, by its parent:
-    # FP64 moments 32, height 4, child count 4, the arrival counter 4; children
-    # lists 32 per internal node, ~4 per node), plus the 4-byte atomic write of
-    # its arrival: 180 B.  The quadrupole pass reads the particles twice and
-    # adds per node 92 B written (FP64 quadrupole and trace, the walk's
-    # quadrupole, the spread) and 56 read (the children's FP64 quadrupole and trace)
-    mom_bytes = (32.0 * n + 328.0 * nodes) if quad else (16.0 * n + 180.0 * nodes)
+    # writes 100 B (FP64 moments 32, its depth-first record 32, the walk's record
+    # 32, the height 4) and reads 68 (its link 16, level 4, first key 8; as a
+    # child, by its parent: FP64 moments 32, height 4; the arrival counter 4), plus
+    # the 4-byte atomic write of its arrival: 172 B.  The quadrupole pass reads the
+    # particles twice and adds per node 92 B written (FP64 quadrupole and trace,
+    # the walk's quadrupole, the spread) and 56 read (the children's FP64
+    # quadrupole and trace)
+    mom_bytes = (32.0 * n + 320.0 * nodes) if quad else (16.0 * n + 172.0 * nodes)
     # The timed steps are device-resident leapfrog steps: the opening kick and
     # drift run in the bounds pass and the closing kick in the pass that writes
-    # the accelerations (the phase events bracket them)
+    # the accelerations (these phases include them)
     rows = [
         # bounds + kick-drift: read x, y, z, m 32, v 24, a 24; write x, v 48
         ("bounds", "bounds_ms", (32.0 + 24.0 + 24.0 + 48.0) * n),
@@ -808,7 +807,7 @@ def stage_bandwidth(phases, stats_acc, n, m, peaks, peak_kind):
         stages[name] = {"ms": round(ms, 4), "algorithmic_bytes": nbytes,
                         "gbs": round(gbs, 1) if gbs else None,
                         "frac_of_hbm": round(gbs / hbm, 4) if gbs else None}
-    # what the phase events do not cover: the step's total minus the phases
+    # what the phases do not cover: the step's total minus their sum
     # (the memsets and launch gaps between the passes; no kernel of its own)
     gap_ms = float(np.mean([ph["total_ms"] - sum(ph[k] for k in (
         "bounds_ms", "keys_ms", "sort_ms", "build_ms", "moments_ms", "walk_ms", "integrate_ms"))
@@ -818,7 +817,7 @@ def stage_bandwidth(phases, stats_acc, n, m, peaks, peak_kind):
     stages["_note"] = (f"HBM peak {hbm} GB/s ({peak_kind} MEASURED_PEAKS.json); bytes per "
                        "particle: bounds with the opening kick and drift 80 read + 48 written, "
                        "keys 32 read + 28 written (+28 relative), sort 7 passes x (12 + 12), "
-                       "moments " + ("2 x 16 + 328 per node" if quad else "16 + 180 per node")
+                       "moments " + ("2 x 16 + 320 per node" if quad else "16 + 172 per node")
                        + ", unsort with the closing kick 56 read + 48 written")
     return stages
 
