@@ -609,10 +609,11 @@ static NBodySimProCudaContext* context_or_default(void* context, NBodySimProErro
 /* Plugin calls of up to STAGE_MAX particles go through the context's own
  * page-locked rows where the caller's arrays are pageable: a copy from or to
  * pageable memory is staged by the driver one array at a time, each with its own
- * wait.  Barnes-Hut calls with and without: 195 and 208 us at 500 particles, 300
- * and 313 at 8000, 374 and 378 at 20k, 476 and 458 at 33k, where the driver's
- * pipelined staging is faster than a plain memcpy here. */
-enum { STAGE_ROWS = 7, STAGE_MAX = 20480 };
+ * wait.  Barnes-Hut calls with and without: 184 and 199 us at 4000 particles, 208
+ * and 220 at 8000, 231 and 247 at 12000, 276 and 277 at 20k, where page-locking
+ * the rows also costs a context's first call more than everything else in it (2.3
+ * ms against 1.3; 1.0 both ways up to 12000). */
+enum { STAGE_ROWS = 7, STAGE_MAX = 16384 };
 
 static NBodySimProStatus ensure_stage(NBodySimProCudaContext* c, size_t n,
                                       NBodySimProError* error) {

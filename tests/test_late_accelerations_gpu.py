@@ -17,7 +17,7 @@ def page_locked(n):
 
 @pytest.mark.parametrize("kind", ["forces", "zero", "nan"])
 @pytest.mark.parametrize("pinned", [False, True])
-@pytest.mark.parametrize("n", [20480, 20481, 98304, 98305, 300001])
+@pytest.mark.parametrize("n", [16384, 16385, 20480, 20481, 98304, 98305, 300001])
 def test_plugin_call_equals_resident_evaluation(cuda, ctx, n, pinned, kind):
     p = O.preset_parallel("galaxy_collision", n, 13)
     s = cuda.ParticleSystem.zeros(n, page_locked if pinned else None)
