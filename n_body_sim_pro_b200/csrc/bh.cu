@@ -313,12 +313,12 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v) {
 // stable LSD radix sort, 9-bit digits, one kernel per pass
 //
 // The keys kernel also counts the 7 digit histograms (one read of the keys), which
-// every tile scans for the digits' bases.  Every pass is a single kernel: tiles take tickets in launch order, rank their keys in shared
-// memory, and find their global offsets with a decoupled look-back over the
-// preceding tiles' published digit counts (flag A: this tile's count, flag P:
-// inclusive prefix).  A tile only waits on tiles with earlier tickets, which
-// are already resident; every wait is bounded and flags an error when it
-// runs out.
+// every tile scans for the digits' bases.  Every pass is a single kernel: tiles take
+// tickets in launch order, rank their keys in shared memory, and find their global
+// offsets with a decoupled look-back over the preceding tiles' published digit
+// counts (flag A: this tile's count, flag P: inclusive prefix).  A tile only waits
+// on tiles with earlier tickets, which are already resident; every wait is bounded
+// and flags an error when it runs out.
 // ---------------------------------------------------------------------------
 
 // A tile is THREADS x ITEMS keys (the figures are of passes by 8-bit digits).
