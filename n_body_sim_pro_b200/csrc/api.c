@@ -631,19 +631,39 @@ static NBodySimProStatus ensure_stage(NBodySimProCudaContext* c, size_t n,
 }
 
 /* How a plugin call reaches a host array: page-locked (with its device address),
- * pageable, or neither (device or managed memory: the driver's copies decide). */
+ * pageable, or neither (device or managed memory, or page-locked in part: the
+ * driver's copies decide). */
 typedef enum ArrayKind { ARRAY_PAGEABLE, ARRAY_LOCKED, ARRAY_OTHER } ArrayKind;
 
-static ArrayKind array_kind(const double* array, double** device) {
-    struct cudaPointerAttributes at;
+static ArrayKind byte_kind(const char* at, char** device) {
+    struct cudaPointerAttributes a;
     *device = NULL;
-    if (cudaPointerGetAttributes(&at, array) != cudaSuccess) {
+    if (cudaPointerGetAttributes(&a, at) != cudaSuccess) {
         (void)cudaGetLastError(); /* (not an error of this call) */
         return ARRAY_OTHER;
     }
-    if (at.type == cudaMemoryTypeUnregistered) return ARRAY_PAGEABLE;
-    *device = (double*)at.devicePointer;
-    return at.type == cudaMemoryTypeHost && at.devicePointer != NULL ? ARRAY_LOCKED : ARRAY_OTHER;
+    if (a.type == cudaMemoryTypeUnregistered) return ARRAY_PAGEABLE;
+    *device = (char*)a.devicePointer;
+    return a.type == cudaMemoryTypeHost && a.devicePointer != NULL ? ARRAY_LOCKED : ARRAY_OTHER;
+}
+
+/* by_kernel: the array is read or written through *device, so each of its pages has
+ * to be page-locked and at its place there (memory is mapped by pages of 4 KiB or
+ * more); for the copies, which check their range themselves, the two ends tell. */
+static ArrayKind array_kind(const double* array, size_t n, int by_kernel, double** device) {
+    const char* const first = (const char*)array;
+    const char* const last = first + n * sizeof(double) - 1;
+    char *origin, *there;
+    const ArrayKind kind = byte_kind(first, &origin);
+    *device = (double*)origin;
+    for (const char* at = last; at > first;) {
+        if (byte_kind(at, &there) != kind) return ARRAY_OTHER;
+        if (kind != ARRAY_LOCKED) break;
+        if (there - origin != at - first) return ARRAY_OTHER;
+        if (!by_kernel) break;
+        at -= ((uintptr_t)at & 4095) + 1; /* the end of the page before */
+    }
+    return kind;
 }
 
 /* The relative test's accelerations of a plugin call that is not staged come in
@@ -682,7 +702,7 @@ typedef struct StagedView {
 
 static NBodySimProStatus stage_view(NBodySimProCudaContext* c,
                                     const NBodySimProParticleSystemView* v, int with_accelerations,
-                                    StagedView* out, NBodySimProError* error) {
+                                    int by_kernel, StagedView* out, NBodySimProError* error) {
     const size_t n = v->particle_count;
     double* own[STAGE_ROWS] = {v->positions_x, v->positions_y, v->positions_z, v->masses,
                                v->accelerations_x, v->accelerations_y, v->accelerations_z};
@@ -691,7 +711,7 @@ static NBodySimProStatus stage_view(NBodySimProCudaContext* c,
     int staged[STAGE_ROWS];
     for (int k = 0; k < STAGE_ROWS; ++k) {
         if (own[k] == NULL) return N_BODY_SIM_PRO_STATUS_OK; /* reported where it is copied */
-        const ArrayKind kind = array_kind(own[k], &out->device[k]);
+        const ArrayKind kind = array_kind(own[k], n, by_kernel, &out->device[k]);
         if (kind == ARRAY_OTHER) return N_BODY_SIM_PRO_STATUS_OK;
         staged[k] = kind == ARRAY_PAGEABLE;
         out->host[k] = own[k];
@@ -819,12 +839,13 @@ static NBodySimProStatus view_force(const NBodySimProParticleSystemView* view,
     /* the relative opening test reads the view's previous accelerations */
     const int with_accelerations =
         algorithm == N_BODY_SIM_PRO_CUDA_ALGORITHM_BARNES_HUT && c->tolerance > 0.0 && !reuse;
+    const int small =
+        algorithm == N_BODY_SIM_PRO_CUDA_ALGORITHM_ALL_PAIRS && n < NBSP_ALLPAIRS_SMALL;
     StagedView staged;
-    if ((st = stage_view(c, view, with_accelerations, &staged, error)) != N_BODY_SIM_PRO_STATUS_OK)
+    if ((st = stage_view(c, view, with_accelerations, small, &staged, error)) !=
+        N_BODY_SIM_PRO_STATUS_OK)
         return st;
-    if (staged.used && algorithm == N_BODY_SIM_PRO_CUDA_ALGORITHM_ALL_PAIRS &&
-        n < NBSP_ALLPAIRS_SMALL)
-        return small_allpairs_force(c, view, gravity, &staged, error);
+    if (staged.used && small) return small_allpairs_force(c, view, gravity, &staged, error);
     NBodySimProParticleSystemView through = *view; /* the arrays that are copied */
     if (staged.used) {
         through.positions_x = staged.host[0];
