@@ -693,7 +693,8 @@ static NBodySimProStatus late_accelerations(NBodySimProCudaContext* c,
 }
 
 /* The seven arrays of a staged plugin call: where the copies or kernels read and
- * write (the caller's array when page-locked, else a staging row). */
+ * write (the caller's array when page-locked and, for kernels, aligned, else a
+ * staging row). */
 typedef struct StagedView {
     int used; /* 0: the call is not staged */
     double* host[STAGE_ROWS];   /* x, y, z, m, ax, ay, az */
@@ -713,7 +714,9 @@ static NBodySimProStatus stage_view(NBodySimProCudaContext* c,
         if (own[k] == NULL) return N_BODY_SIM_PRO_STATUS_OK; /* reported where it is copied */
         const ArrayKind kind = array_kind(own[k], n, by_kernel, &out->device[k]);
         if (kind == ARRAY_OTHER) return N_BODY_SIM_PRO_STATUS_OK;
-        staged[k] = kind == ARRAY_PAGEABLE;
+        /* (a kernel's loads and stores need the alignment that the copies do not) */
+        staged[k] = kind == ARRAY_PAGEABLE ||
+                    (by_kernel && (uintptr_t)out->device[k] % sizeof(double) != 0);
         out->host[k] = own[k];
     }
     NBodySimProStatus st = ensure_stage(c, n, error);

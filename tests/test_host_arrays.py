@@ -3,7 +3,6 @@ kernels faked on the CPU: a kernel may only be given what it can reach from the
 first element to the last, and every other call takes the copies, whose checks
 decide."""
 import ctypes as C
-import itertools
 
 import numpy as np
 import pytest
@@ -134,3 +133,13 @@ def test_partly_locked_arrays_are_the_copies_to_judge(host, context, n, field):
         status, faults, small = Call(host, n, part, only=[field]).run(context)
         assert (faults, small) == (0, 0)
         assert status == nb.Status.INVALID_STATE
+
+
+@pytest.mark.parametrize("n", [1, 700, 2047])
+@pytest.mark.parametrize("shift", [1, 4, 12])
+def test_unaligned_arrays_go_through_the_rows(host, context, n, shift):
+    """Page-locked or pageable, arrays that are not on 8-byte boundaries are served
+    (the copies never asked for it), but not by a kernel's own loads and stores."""
+    for locked in ([], [(0, 8 * n)]):
+        for only in (None, ["masses"], ["accelerations_y"]):
+            assert Call(host, n, locked, shift, only).run(context) == (nb.Status.OK, 0, 1)
