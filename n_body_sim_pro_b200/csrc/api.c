@@ -615,19 +615,24 @@ static NBodySimProCudaContext* context_or_default(void* context, NBodySimProErro
  * ms against 1.3; 1.0 both ways up to 12000). */
 enum { STAGE_ROWS = 7, STAGE_MAX = 16384 };
 
-static NBodySimProStatus ensure_stage(NBodySimProCudaContext* c, size_t n,
-                                      NBodySimProError* error) {
-    if (n <= c->stage_n) return N_BODY_SIM_PRO_STATUS_OK;
+/* Whether the rows hold n particles; 0 where no page-locked memory can be had. */
+static int ensure_stage(NBodySimProCudaContext* c, size_t n) {
+    if (n <= c->stage_n) return 1;
     size_t rows = 1024;
     while (rows < n) rows *= 2;
+    double *stage = NULL, *device = NULL;
+    if (cudaHostAlloc((void**)&stage, (STAGE_ROWS * rows + 1) * sizeof(double),
+                      cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&device, stage, 0) != cudaSuccess) {
+        (void)cudaGetLastError(); /* (not an error of this call: the copies serve it) */
+        cudaFreeHost(stage);
+        return 0;
+    }
     cudaFreeHost(c->stage);
-    c->stage = NULL;
-    c->stage_n = 0;
-    CUDA_TRY(cudaHostAlloc((void**)&c->stage, (STAGE_ROWS * rows + 1) * sizeof(double),
-                           cudaHostAllocMapped));
-    CUDA_TRY(cudaHostGetDevicePointer((void**)&c->stage_device, c->stage, 0));
+    c->stage = stage;
+    c->stage_device = device;
     c->stage_n = rows;
-    return N_BODY_SIM_PRO_STATUS_OK;
+    return 1;
 }
 
 /* How a plugin call reaches a host array: page-locked (with its device address),
@@ -701,26 +706,24 @@ typedef struct StagedView {
     double* device[STAGE_ROWS]; /* the same as device addresses */
 } StagedView;
 
-static NBodySimProStatus stage_view(NBodySimProCudaContext* c,
-                                    const NBodySimProParticleSystemView* v, int with_accelerations,
-                                    int by_kernel, StagedView* out, NBodySimProError* error) {
+static void stage_view(NBodySimProCudaContext* c, const NBodySimProParticleSystemView* v,
+                       int with_accelerations, int by_kernel, StagedView* out) {
     const size_t n = v->particle_count;
     double* own[STAGE_ROWS] = {v->positions_x, v->positions_y, v->positions_z, v->masses,
                                v->accelerations_x, v->accelerations_y, v->accelerations_z};
     out->used = 0;
-    if (n > STAGE_MAX) return N_BODY_SIM_PRO_STATUS_OK;
+    if (n > STAGE_MAX) return;
     int staged[STAGE_ROWS];
     for (int k = 0; k < STAGE_ROWS; ++k) {
-        if (own[k] == NULL) return N_BODY_SIM_PRO_STATUS_OK; /* reported where it is copied */
+        if (own[k] == NULL) return; /* reported where it is copied */
         const ArrayKind kind = array_kind(own[k], n, by_kernel, &out->device[k]);
-        if (kind == ARRAY_OTHER) return N_BODY_SIM_PRO_STATUS_OK;
+        if (kind == ARRAY_OTHER) return;
         /* (a kernel's loads and stores need the alignment that the copies do not) */
         staged[k] = kind == ARRAY_PAGEABLE ||
                     (by_kernel && (uintptr_t)out->device[k] % sizeof(double) != 0);
         out->host[k] = own[k];
     }
-    NBodySimProStatus st = ensure_stage(c, n, error);
-    if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
+    if (!ensure_stage(c, n)) return;
     for (int k = 0; k < STAGE_ROWS; ++k) {
         if (!staged[k]) continue;
         out->host[k] = c->stage + k * c->stage_n;
@@ -728,7 +731,6 @@ static NBodySimProStatus stage_view(NBodySimProCudaContext* c,
         if (k < 4 || with_accelerations) memcpy(out->host[k], own[k], n * sizeof(double));
     }
     out->used = 1;
-    return N_BODY_SIM_PRO_STATUS_OK;
 }
 
 /* After the call's work has finished: staged results into the caller's arrays. */
@@ -845,9 +847,7 @@ static NBodySimProStatus view_force(const NBodySimProParticleSystemView* view,
     const int small =
         algorithm == N_BODY_SIM_PRO_CUDA_ALGORITHM_ALL_PAIRS && n < NBSP_ALLPAIRS_SMALL;
     StagedView staged;
-    if ((st = stage_view(c, view, with_accelerations, small, &staged, error)) !=
-        N_BODY_SIM_PRO_STATUS_OK)
-        return st;
+    stage_view(c, view, with_accelerations, small, &staged);
     if (staged.used && small) return small_allpairs_force(c, view, gravity, &staged, error);
     NBodySimProParticleSystemView through = *view; /* the arrays that are copied */
     if (staged.used) {

@@ -23,5 +23,5 @@ def build(folder, unit, fakes):
     missing = [s for s in missing if s.startswith(("cuda", "nbsp_", "n_body_"))]
     with open(stubs, "w") as f:
         f.writelines(f"long {s}(void) {{ return 0; }}\n" for s in missing)
-    subprocess.run(cc + ["-shared", "-o", lib, obj, stubs, "-lm"], check=True)
+    subprocess.run(cc + ["-shared", "-Wl,-Bsymbolic", "-o", lib, obj, stubs, "-lm"], check=True)
     return C.CDLL(lib)

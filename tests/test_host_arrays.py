@@ -15,7 +15,7 @@ import n_body_sim_pro_b200 as nb
 FAKES = r"""
 EXPORT int fake_faults, fake_small_calls;
 EXPORT void fake_fail_host_alloc(int on) { fake_host_alloc_fails = on; }
-EXPORT void* fake_stage(NBodySimProCudaContext* c) { return c->stage; }
+EXPORT int fake_error_left(void) { return cudaGetLastError(); }
 int nbsp_allpairs_small(const double* x, const double* y, const double* z, const double* m,
                         size_t n, float eps2, double g, void* packed, double* ax, double* ay,
                         double* az, double* ox, double* oy, double* oz, int* report,
@@ -52,8 +52,7 @@ void nbsp_allpairs_finalize(const void* hi, const void* lo, size_t n, int chunks
 def host(tmp_path_factory):
     lib = host_build.build(str(tmp_path_factory.mktemp("host")), "api.c", FAKES)
     lib.n_body_sim_pro_cuda_context_create.restype = C.c_void_p
-    lib.fake_stage.restype = C.c_void_p
-    for f in ("fake_register", "fake_unregister", "fake_watch", "fake_stage", "n_body_sim_pro_cuda_context_destroy"):
+    for f in ("fake_register", "fake_unregister", "fake_watch", "n_body_sim_pro_cuda_context_destroy"):
         getattr(lib, f).argtypes = [C.c_void_p] + ([C.c_size_t] if f == "fake_register" else [])
     lib.n_body_sim_pro_gravity_compute_acceleration_cuda.argtypes = [C.c_void_p] * 4
     return lib
@@ -65,7 +64,7 @@ FIELDS = ("positions_x", "positions_y", "positions_z", "masses", "accelerations_
 
 class Call:
     """An all-pairs plugin call of n particles whose seven arrays start `shift` bytes
-    behind a page's start; `locked` bytes ranges of each are page-locked."""
+    behind a page's start; `locked` byte ranges of each (or of the fields `only`) are page-locked."""
 
     def __init__(self, host, n, locked=(), shift=0, only=None):
         self.host, self.n = host, n
@@ -143,3 +142,23 @@ def test_unaligned_arrays_go_through_the_rows(host, context, n, shift):
     for locked in ([], [(0, 8 * n)]):
         for only in (None, ["masses"], ["accelerations_y"]):
             assert Call(host, n, locked, shift, only).run(context) == (nb.Status.OK, 0, 1)
+
+
+@pytest.mark.parametrize("n", [5, 1000, 2047])
+def test_calls_survive_a_failing_page_lock(host, context, n):
+    """No page-locked memory for the rows: the copies serve the call, and the rows are
+    there again when it can be had."""
+    assert Call(host, 3).run(context) == (nb.Status.OK, 0, 1)
+    host.fake_fail_host_alloc(1)
+    served = Call(host, n).run(context)
+    assert served == (nb.Status.OK, 0, int(n < 1024))  # (the first call's rows hold 1024)
+    assert host.fake_error_left() == 0
+    assert Call(host, 7).run(context)[0] == nb.Status.OK
+    host.fake_fail_host_alloc(0)
+    assert Call(host, n).run(context) == (nb.Status.OK, 0, 1)
+
+
+def test_first_call_without_rows(host, context):
+    host.fake_fail_host_alloc(1)
+    assert Call(host, 100).run(context) == (nb.Status.OK, 0, 0)
+    assert Call(host, 100, [(0, 800)]).run(context) == (nb.Status.OK, 0, 0)
