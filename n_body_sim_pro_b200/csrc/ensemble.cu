@@ -16,13 +16,15 @@
 // quarters have the same work.  A system of T tiles (64 particles) is T x T
 // tile pairs, 64 targets by 64 sources each; its warps take equal runs of them in
 // target order, so that a tile of targets is shared by two warps at most (no
-// more warps than tiles) and the second one's part is added to the first one's,
-// in FP64, after a barrier.  With whole targets per thread instead (four of
-// them, the system's threads rounded up to warps) a system of 2,100 particles
-// ran on 17 warps, five of them on one quarter of the SM.  Sums wait in shared
-// memory for the update pass, so a lane holds two targets and no spills.
-// Measured on 4096 systems of 32 to 4096 particles (3.4M, 7.1e9 pairs a step),
-// 21 evaluations: 70.4 -> 63.3 ms (2.1e12 -> 2.4e12 pairs / s, 63% of the FP32
+// more warps than tiles).  The second one goes on with the first one's sums, which
+// the first one makes before anything else, so the cut changes no bit and the
+// wait costs nothing (68.4 ms a call either way; adding the parts after a barrier
+// let a system's bits depend on its neighbours).  With whole targets per thread
+// instead (four of them, the system's threads rounded up to warps) a system of
+// 2,100 particles ran on 17 warps, five of them on one quarter of the SM.  Sums
+// wait in shared memory for the update pass, so a lane holds two targets and no
+// spills.  Measured on 4096 systems of 32 to 4096 particles (3.4M, 7.1e9 pairs a
+// step), 21 evaluations: 70.4 -> 63.3 ms (2.1e12 -> 2.4e12 pairs / s, 63% of the FP32
 // peak in 20-flop pairs, of which the 12 instructions per pair allow 83%).  The
 // tile's loop fully unrolled: 16 sources at a time 64.2, 4 at a time 65.9.
 #include "internal.h"
@@ -95,6 +97,42 @@ constexpr float kFarAway = 1e30f;  // padding sources: r^2 overflows to inf, rsq
 constexpr int kCap = 4096;         // particle slots of a CTA (a system's are whole tiles)
 constexpr int kSmemBytes = kCap * (2 * (int)sizeof(float4) + 3 * (int)sizeof(double));
 
+// A target tile whose sources two warps share: the first one leaves its (hi, lo)
+// sums where the tile's FP64 sums will be, the second one folds its sources into
+// them, so that every target has one chain of folds over all tiles in order and
+// its bits do not depend on where the cut lies.
+__device__ __forceinline__ double pack_sum(float hi, float lo) {
+  return __hiloint2double(__float_as_int(hi), __float_as_int(lo));
+}
+__device__ __forceinline__ void unpack_sum(double v, float& hi, float& lo) {
+  hi = __int_as_float(__double2hiint(v));
+  lo = __int_as_float(__double2loint(v));
+}
+__device__ __forceinline__ void sums_begun(unsigned* begun, unsigned turn, int lane) {
+  __syncwarp();  // the warp's sums, then the word
+  if (lane == 0)
+    asm volatile("st.release.cta.shared.u32 [%0], %1;"
+                 :: "r"((unsigned)__cvta_generic_to_shared(begun)), "r"(turn)
+                 : "memory");
+}
+// False when the other warp's word did not come within the polls (it is the first
+// thing that warp does in a step and waits for nothing).
+constexpr int kTurnPolls = 1 << 22;
+__device__ __forceinline__ bool wait_for_sums(const unsigned* begun, unsigned turn, int lane) {
+  bool there = true;
+  if (lane == 0) {
+    unsigned seen = 0;
+    for (int polls = 0; polls < kTurnPolls && seen != turn; ++polls)
+      asm volatile("ld.acquire.cta.shared.u32 %0, [%1];"
+                   : "=r"(seen)
+                   : "r"((unsigned)__cvta_generic_to_shared(begun))
+                   : "memory");
+    there = seen == turn;
+  }
+  __syncwarp();
+  return there;
+}
+
 // GUARD: drop r^2 = 0 terms (eps = 0, or m / eps^3 could overflow); otherwise
 // a target's own entry has d = 0 and adds W * 0 = 0.
 template <int BLOCK, bool GUARD>
@@ -105,7 +143,10 @@ __global__ void __launch_bounds__(BLOCK, 1) ensemble_kernel(EnsembleArgs a) {
   extern __shared__ float4 sp[];
   double* const acc = reinterpret_cast<double*>(sp + 2 * kCap);
   __shared__ int s_item;
+  __shared__ unsigned s_begun[BLOCK / 32];  // the last step whose shared tile a warp has begun
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned turn = 0;  // steps of this CTA, of all its items
+  if (tid < BLOCK / 32) s_begun[tid] = 0;
   for (int guard = 0;; ++guard) {
     if (guard > a.items) {  // each CTA takes each item at most once
       if (tid == 0) atomicOr(a.status, NBSP_DEVICE_ERROR_ENSEMBLE_LIMIT);
@@ -152,23 +193,38 @@ __global__ void __launch_bounds__(BLOCK, 1) ensemble_kernel(EnsembleArgs a) {
     }
     __syncthreads();
     const unsigned long long E2 = pack2(a.eps2, a.eps2);
-    // this warp's run of the system's tile pairs
+    // this warp's run of the system's tile pairs: the sources from tile j0 on of the
+    // first target tile, whole target tiles, the sources before tile j1 of the last
     const int begin = tiles * tiles * lw / warps, end = tiles * tiles * (lw + 1) / warps;
+    const int t0 = tiles > 0 ? begin / tiles : 0, j0 = begin - t0 * tiles;
+    const int t1 = tiles > 0 ? end / tiles : 0, j1 = end - t1 * tiles;
     for (int step = 0; step <= a.steps; ++step) {
-      double part[6];  // of a target tile that another warp began
-      int shared_tile = -1;
-      for (int r = begin; r < end;) {
-        const int target = r / tiles, j0 = r - target * tiles;
-        const int j1 = min(tiles, j0 + (end - r));
+      ++turn;
+      // the last first: the tile that the next warp goes on with is begun at once,
+      // the one that the warp before began comes at the end
+      for (int target = begin == end ? -1 : j1 > 0 ? t1 : t1 - 1; target >= t0; --target) {
+        const bool whole = target < t1;  // to the last source
         const int i0 = target * kTile + lane;
-        const float4 u0 = pos[2 * i0], u1 = pos[2 * i0 + 1];
-        const float4 v0 = pos[2 * (i0 + 32)], v1 = pos[2 * (i0 + 32) + 1];
-        const unsigned long long X = pack2(u0.x, v0.x), Y = pack2(u0.z, v0.z), Z = pack2(u1.x, v1.x);
+        int j = 0;
         float hx[2], hy[2], hz[2], lx[2], ly[2], lz[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;
-        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(pos + 2 * j0 * kTile);
-        for (int j = j0; j < j1; ++j) {
+        if (target == t0 && j0 > 0) {
+          j = j0;
+          if (!wait_for_sums(&s_begun[warp - 1], turn, lane) && lane == 0)
+            atomicOr(a.status, NBSP_DEVICE_ERROR_ENSEMBLE_LIMIT);
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            unpack_sum(sx[i0 + 32 * k], hx[k], lx[k]);
+            unpack_sum(sy[i0 + 32 * k], hy[k], ly[k]);
+            unpack_sum(sz[i0 + 32 * k], hz[k], lz[k]);
+          }
+        }
+        const float4 u0 = pos[2 * i0], u1 = pos[2 * i0 + 1];
+        const float4 v0 = pos[2 * (i0 + 32)], v1 = pos[2 * (i0 + 32) + 1];
+        const unsigned long long X = pack2(u0.x, v0.x), Y = pack2(u0.z, v0.z), Z = pack2(u1.x, v1.x);
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(pos + 2 * j * kTile);
+        for (const int stop = whole ? tiles : j1; j < stop; ++j) {
           unsigned long long AX = 0ull, AY = 0ull, AZ = 0ull;
 #pragma unroll
           for (int k = 0; k < kTile; ++k) {
@@ -200,36 +256,13 @@ __global__ void __launch_bounds__(BLOCK, 1) ensemble_kernel(EnsembleArgs a) {
           fold(hz[0], lz[0], u);
           fold(hz[1], lz[1], v);
         }
-        double sum[6];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          sum[3 * k] = (double)hx[k] + (double)lx[k];
-          sum[3 * k + 1] = (double)hy[k] + (double)ly[k];
-          sum[3 * k + 2] = (double)hz[k] + (double)lz[k];
+          sx[i0 + 32 * k] = whole ? (double)hx[k] + (double)lx[k] : pack_sum(hx[k], lx[k]);
+          sy[i0 + 32 * k] = whole ? (double)hy[k] + (double)ly[k] : pack_sum(hy[k], ly[k]);
+          sz[i0 + 32 * k] = whole ? (double)hz[k] + (double)lz[k] : pack_sum(hz[k], lz[k]);
         }
-        if (j0 == 0) {
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            sx[i0 + 32 * k] = sum[3 * k];
-            sy[i0 + 32 * k] = sum[3 * k + 1];
-            sz[i0 + 32 * k] = sum[3 * k + 2];
-          }
-        } else {
-          shared_tile = target;
-#pragma unroll
-          for (int k = 0; k < 6; ++k) part[k] = sum[k];
-        }
-        r += j1 - j0;
-      }
-      __syncthreads();
-      if (shared_tile >= 0) {
-        const int i0 = shared_tile * kTile + lane;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          sx[i0 + 32 * k] += part[3 * k];
-          sy[i0 + 32 * k] += part[3 * k + 1];
-          sz[i0 + 32 * k] += part[3 * k + 2];
-        }
+        if (!whole) sums_begun(&s_begun[warp], turn, lane);
       }
       __syncthreads();
       for (int i = lw * 32 + lane; i < n; i += warps * 32) {
