@@ -499,15 +499,18 @@ __device__ __forceinline__ RowInputs fetched_rows(const uint32_t* rows, int warp
 // (Each CTA updating all parameters for itself saves the second wait, but the
 // update is division-bound: 6.3 us of a step at 8 CTAs against 2.4, the second wait
 // and the copy included.)
+// The results go to next_params, next_m and next_v, so that an epoch in which a
+// wait ran out leaves what it began with.
 // bias: the step's 1 - beta^t for both moments.
 constexpr int kEpochCtas = 32;
 constexpr int kEpochCluster = 8;  // the largest cluster that every GPU can place
 __global__ void __launch_bounds__(kTrainThreads, 1) train_epoch_kernel(
     const uint32_t* __restrict__ x_bf16, const float* __restrict__ y, const int* __restrict__ order,
     int rows_total, int steps, float inv_batch3, TrainFrags* f, float* slots,
-    float* __restrict__ params, float* __restrict__ m, float* __restrict__ v, float lr, float beta1,
-    float beta2, float eps, const float2* __restrict__ bias, int* arrivals, int* failed,
-    int one_cluster) {
+    const float* __restrict__ params, const float* __restrict__ m, const float* __restrict__ v,
+    float* __restrict__ next_params, float* __restrict__ next_m, float* __restrict__ next_v,
+    float lr, float beta1, float beta2, float eps, const float2* __restrict__ bias, int* arrivals,
+    int* failed, int one_cluster) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Stage& st = *reinterpret_cast<Stage*>(smem_raw);
   __shared__ int s_ok;
@@ -566,9 +569,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_epoch_kernel(
     __syncthreads();
   }
   for (int p = first + tid; p < last; p += kTrainThreads) {
-    params[p] = pp[p];
-    m[p] = mm[p];
-    v[p] = vv[p];
+    next_params[p] = pp[p];
+    next_m[p] = mm[p];
+    next_v[p] = vv[p];
   }
 }
 
@@ -785,11 +788,13 @@ void nbsp_mlp_adam_bias(int step, float* bias) {
 // `steps` minibatches of ctas * 128 rows of `order` from its start, forward,
 // backward and Adam, in one launch (ctas <= nbsp_mlp_epoch_ctas()); slots: ctas
 // gradient slots; bias: steps pairs of nbsp_mlp_adam_bias on the device; sync: two
-// zeroed ints, the second nonzero when a wait ran out.  The fragments in `frags`
-// follow the parameters; the inference network is not touched.
+// zeroed ints, the second nonzero when a wait ran out (next_params, next_m and next_v
+// are then in part).  The fragments in `frags` follow the parameters; the inference
+// network is not touched.
 int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order, int rows_total,
                          int steps, int ctas, float inv_batch3, void* frags, float* slots,
-                         float* params, float* m, float* v, float lr, const void* bias, int* sync,
+                         const float* params, const float* m, const float* v, float* next_params,
+                         float* next_m, float* next_v, float lr, const void* bias, int* sync,
                          cudaStream_t stream) {
   const int smem =
       (int)(sizeof(Stage) + 3 * kSlot * sizeof(float) + 2 * kRows * kRowWords * sizeof(uint32_t));
@@ -800,7 +805,8 @@ int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order, in
   int* failed = sync + 1;
   int one_cluster = ctas <= kEpochCluster;
   void* args[] = {&x, &y, &order, &rows_total, &steps, &inv_batch3, &f, &slots, &params, &m, &v,
-                  &lr, &beta1, &beta2, &eps, &b, &sync, &failed, &one_cluster};
+                  &next_params, &next_m, &next_v, &lr, &beta1, &beta2, &eps, &b, &sync, &failed,
+                  &one_cluster};
   cudaLaunchAttribute how;
   if (one_cluster) {
     how.id = cudaLaunchAttributeClusterDimension;

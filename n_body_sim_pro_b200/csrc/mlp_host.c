@@ -39,9 +39,10 @@ NBSP_HIDDEN void nbsp_mlp_loss(const uint32_t* x, const float* y, int first_row,
 NBSP_HIDDEN void nbsp_mlp_adam_bias(int step, float* bias);
 NBSP_HIDDEN int nbsp_mlp_train_epoch(const uint32_t* x, const float* y, const int* order,
                                      int rows_total, int steps, int ctas, float inv_batch3,
-                                     void* frags, float* slots, float* params, float* m,
-                                     float* v, float lr, const void* bias, int* sync,
-                                     cudaStream_t stream);
+                                     void* frags, float* slots, const float* params,
+                                     const float* m, const float* v, float* next_params,
+                                     float* next_m, float* next_v, float lr, const void* bias,
+                                     int* sync, cudaStream_t stream);
 NBSP_HIDDEN void nbsp_mlp_reduce_adam(const float* partial, int slots, float* grad_out,
                                       float* params, float* m, float* v, float lr, int step,
                                       int apply, cudaStream_t stream);
@@ -56,6 +57,7 @@ struct NBodySimProCudaCorrection {
     int device;
     cudaStream_t stream;
     float *params, *m, *v;  /* device FP32 master weights and Adam moments */
+    float *next_params, *next_m, *next_v; /* an epoch's, until it is known to be whole */
     void* frags;            /* training fragments */
     void* net;              /* inference network (read by the corrected walk) */
     float* partial;         /* per-CTA gradient slots */
@@ -130,8 +132,8 @@ void n_body_sim_pro_cuda_correction_destroy(NBodySimProCudaCorrection* c) {
     cudaSetDevice(c->device);
     if (c->stream != NULL) cudaStreamSynchronize(c->stream);
     free_data(c);
-    void* p[] = {c->params, c->m, c->v, c->frags, c->net, c->partial, c->loss, c->grad,
-                 c->bias, c->sync};
+    void* p[] = {c->params, c->m, c->v, c->next_params, c->next_m, c->next_v, c->frags, c->net,
+                 c->partial, c->loss, c->grad, c->bias, c->sync};
     for (size_t k = 0; k < sizeof(p) / sizeof(p[0]); ++k) cudaFree(p[k]);
     cudaFreeHost(c->host_loss);
     if (c->stream != NULL) cudaStreamDestroy(c->stream);
@@ -196,6 +198,9 @@ NBodySimProCudaCorrection* n_body_sim_pro_cuda_correction_create(uint64_t seed,
     if (code == cudaSuccess) code = cudaMalloc((void**)&c->params, np * sizeof(float));
     if (code == cudaSuccess) code = cudaMalloc((void**)&c->m, np * sizeof(float));
     if (code == cudaSuccess) code = cudaMalloc((void**)&c->v, np * sizeof(float));
+    if (code == cudaSuccess) code = cudaMalloc((void**)&c->next_params, np * sizeof(float));
+    if (code == cudaSuccess) code = cudaMalloc((void**)&c->next_m, np * sizeof(float));
+    if (code == cudaSuccess) code = cudaMalloc((void**)&c->next_v, np * sizeof(float));
     if (code == cudaSuccess) code = cudaMalloc((void**)&c->grad, np * sizeof(float));
     if (code == cudaSuccess) code = cudaMalloc(&c->frags, nbsp_mlp_frags_bytes());
     if (code == cudaSuccess) code = cudaMalloc(&c->net, nbsp_mlp_net_bytes());
@@ -348,6 +353,18 @@ static NBodySimProStatus evaluate(NBodySimProCudaCorrection* c, size_t first, si
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
+/* A whole epoch's weights and moments in place of those it began with. */
+static void take_epoch(NBodySimProCudaCorrection* c, int steps) {
+    float** old[3] = {&c->params, &c->m, &c->v};
+    float** next[3] = {&c->next_params, &c->next_m, &c->next_v};
+    for (int k = 0; k < 3; ++k) {
+        float* p = *old[k];
+        *old[k] = *next[k];
+        *next[k] = p;
+    }
+    c->adam_step += steps;
+}
+
 NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection* c, int epochs,
                                                        int batch, double learning_rate,
                                                        double* train_loss, double* validation_loss,
@@ -403,10 +420,10 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
             if (code == cudaSuccess)
                 code = (cudaError_t)nbsp_mlp_train_epoch(
                     c->x, c->y, c->order, (int)n, steps, ctas, inv_batch3, c->frags, c->partial,
-                    c->params, c->m, c->v, (float)learning_rate, c->bias, c->sync, c->stream);
+                    c->params, c->m, c->v, c->next_params, c->next_m, c->next_v,
+                    (float)learning_rate, c->bias, c->sync, c->stream);
             if (code == cudaSuccess) {
-                c->adam_step += steps;
-                nbsp_mlp_build_frags(c->params, c->frags, c->net, c->stream);
+                nbsp_mlp_build_frags(c->next_params, c->frags, c->net, c->stream);
                 code = cudaGetLastError();
             }
             if (code == cudaSuccess)
@@ -423,8 +440,13 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
             code = cudaGetLastError();
         }
         if (code == cudaSuccess) code = cudaStreamSynchronize(c->stream);
-        if (code == cudaSuccess && one_launch) memcpy(&failed, c->host_loss, sizeof(failed));
-        if (failed) {
+        if (code == cudaSuccess && one_launch) {
+            memcpy(&failed, c->host_loss, sizeof(failed));
+            if (!failed) take_epoch(c, steps);
+        }
+        if (failed) { /* (some blocks wrote their part of it) */
+            nbsp_mlp_build_frags(c->params, c->frags, c->net, c->stream);
+            cudaStreamSynchronize(c->stream);
             free(order);
             free(bias);
             return mfail(error, N_BODY_SIM_PRO_STATUS_INVALID_STATE, __LINE__,
