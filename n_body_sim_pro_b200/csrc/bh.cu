@@ -76,7 +76,8 @@ __device__ __forceinline__ void bounds_block_reduce(double (&v)[kBoundsVals],
 }
 
 // Phase boundaries of an evaluation are read from the GPU's clock by the first
-// thread of each phase's first kernel (stamp NULL: not timed).  A timing event
+// thread of each phase's first kernel, or, where a memset comes before that, at the
+// end of the kernel before (stamp NULL: not timed).  A timing event
 // between two kernels held the second one back by about 3.5 us.
 __device__ __forceinline__ unsigned long long gpu_clock() {
   unsigned long long t;
@@ -180,9 +181,11 @@ __device__ __forceinline__ void root_geometry(const double* __restrict__ partial
 }
 
 __global__ void __launch_bounds__(kBoundsThreads) bounds_final_kernel(
-    const double* __restrict__ partial, int blocks, size_t n, double* __restrict__ geometry) {
+    const double* __restrict__ partial, int blocks, size_t n, double* __restrict__ geometry,
+    unsigned long long* end) {
   __shared__ double sh[kBoundsVals][kBoundsThreads / 32];
   root_geometry(partial, blocks, n, sh, geometry);
+  if (end != nullptr && threadIdx.x == 0) *end = gpu_clock();
 }
 
 // ---------------------------------------------------------------------------
@@ -422,9 +425,9 @@ __global__ void __launch_bounds__(256) keys_kernel(
     uint64_t* __restrict__ keys, uint32_t* __restrict__ index, float4* __restrict__ unsorted,
     uint32_t* __restrict__ hist, const double* __restrict__ ax, const double* __restrict__ ay,
     const double* __restrict__ az, double tol_scale, float* __restrict__ unsorted_tol, Tree tree,
-    unsigned long long* counters, unsigned long long* stamp) {
+    unsigned long long* counters) {
   __shared__ uint32_t h[kSortPasses][kRadix];
-  start_tree(tree, counters, stamp);
+  start_tree(tree, counters, nullptr);
   for (int k = threadIdx.x; k < kSortPasses * kRadix; k += blockDim.x) (&h[0][0])[k] = 0;
   __syncthreads();
   double geo[8];
@@ -3051,7 +3054,7 @@ extern "C" {
 void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n, double* partial,
                     double* geometry, int* status, const double* ax, const double* ay,
                     const double* az, int rms_of_a, const NbspLeapfrogFusion* leapfrog,
-                    unsigned long long* stamp, cudaStream_t stream) {
+                    unsigned long long* stamp, unsigned long long* end, cudaStream_t stream) {
   const int blocks = bounds_blocks(n);
   if (leapfrog != nullptr && leapfrog->vx != nullptr) {
     NBSP_COUNT_LAUNCH(1), bounds_kernel<true><<<blocks, kBoundsThreads, 0, stream>>>(
@@ -3063,8 +3066,8 @@ void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n, 
         0.0, 0.0, stamp);
   }
   if (geometry != nullptr)
-    NBSP_COUNT_LAUNCH(1), bounds_final_kernel<<<1, kBoundsThreads, 0, stream>>>(partial, blocks, n,
-                                                                              geometry);
+    NBSP_COUNT_LAUNCH(1), bounds_final_kernel<<<1, kBoundsThreads, 0, stream>>>(
+                              partial, blocks, n, geometry, end);
 }
 
 void nbsp_bh_small_keys(const double* x, const double* y, const double* z, const double* m,
@@ -3099,7 +3102,7 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
                   const double* geometry, uint64_t* keys, uint32_t* index, void* unsorted,
                   uint32_t* scratch, const double* ax, const double* ay, const double* az,
                   double tol_scale, float* unsorted_tol, void* tree,
-                  unsigned long long* counters, unsigned long long* stamp, cudaStream_t stream) {
+                  unsigned long long* counters, cudaStream_t stream) {
   cudaMemsetAsync(scratch, 0, sort_scratch_words(n) * sizeof(uint32_t), stream);
   const SortScratch sc = sort_scratch(scratch);
   size_t blocks = (n + 255) / 256;
@@ -3107,7 +3110,7 @@ void nbsp_bh_keys(const double* x, const double* y, const double* z, const doubl
   if (blocks > (size_t)kKeysBlocks) blocks = kKeysBlocks;
   NBSP_COUNT_LAUNCH(1), keys_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
       x, y, z, m, n, geometry, keys, index, (float4*)unsorted, sc.hist, ax, ay, az, tol_scale,
-      unsorted_tol, tree_view(tree, n), counters, stamp);
+      unsorted_tol, tree_view(tree, n), counters);
 }
 
 void nbsp_bh_sort(uint64_t* keys, uint32_t* index, uint64_t* keys_alt, uint32_t* index_alt,

@@ -127,11 +127,14 @@ enum {
 NBSP_HIDDEN void nbsp_bh_bounds(double* x, double* y, double* z, const double* m, size_t n,
                                 double* partial, double* geometry, int* status, const double* ax,
                                 const double* ay, const double* az, int rms_of_a,
-                                const NbspLeapfrogFusion* leapfrog, unsigned long long* stamp, cudaStream_t stream);
+                                const NbspLeapfrogFusion* leapfrog, unsigned long long* stamp,
+                                unsigned long long* end, cudaStream_t stream);
 /* geometry: root centre [0..2], half side [3], centre of mass [4..6], and with
  * rms_of_a the rms |a| [7] of (ax, ay, az) (the relative test's floor); with a
  * leapfrog fusion (NULL: none) the kick and drift come first and the rest is of
- * the drifted positions */
+ * the drifted positions; end (NULL: not timed): the clock when the geometry is
+ * there, where the keys' phase begins, to which the clearing of the sort's scratch
+ * belongs */
 
 /* Morton keys, the identity index, the 7 digit histograms (into sort_scratch)
  * and the walk's float4 (x - c, y - c, z - c, m) with c the centre of mass, in
@@ -141,7 +144,7 @@ NBSP_HIDDEN void nbsp_bh_keys(const double* x, const double* y, const double* z,
                               void* unsorted, uint32_t* sort_scratch, const double* ax,
                               const double* ay, const double* az, double tol_scale,
                               float* unsorted_tol, void* tree, unsigned long long* counters,
-                              unsigned long long* stamp, cudaStream_t stream);
+                              cudaStream_t stream);
 /* (with unsorted_tol != NULL also the relative opening test's tolerance of each
  * particle, tol_scale |a| from the previous accelerations, +inf where |a| = 0;
  * the tree's masks and leaf counts and the 8 counters are set to zero) */

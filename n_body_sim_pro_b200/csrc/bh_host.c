@@ -179,7 +179,7 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
     const int small = s->n <= NBSP_BH_SMALL_SORT;
     nbsp_bh_bounds(s->x, s->y, s->z, s->m, s->n, b->partial, small ? NULL : b->geometry, status,
                    with_a ? s->ax : NULL, with_a ? s->ay : NULL, with_a ? s->az : NULL, rel, lf,
-                   stamp_of(b, unread, NBSP_BH_BOUNDS), stream);
+                   stamp_of(b, unread, NBSP_BH_BOUNDS), stamp_of(b, unread, NBSP_BH_KEYS), stream);
     if (small) {
         nbsp_bh_small_keys(s->x, s->y, s->z, s->m, s->n, b->partial, b->geometry, b->keys_alt,
                            b->index_alt, b->unsorted, s->ax, s->ay, s->az, tol_scale,
@@ -192,7 +192,7 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
     }
     nbsp_bh_keys(s->x, s->y, s->z, s->m, s->n, b->geometry, b->keys_alt, b->index_alt, b->unsorted,
                  b->hist, s->ax, s->ay, s->az, tol_scale, rel ? b->tol_unsorted : NULL, b->tree,
-                 b->counters, stamp_of(b, unread, NBSP_BH_KEYS), stream);
+                 b->counters, stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status,
                  stamp_of(b, unread, NBSP_BH_SORT), stream);
     nbsp_bh_gather(b->unsorted, b->index, s->n, b->pos4, rel ? b->tol_unsorted : NULL,
