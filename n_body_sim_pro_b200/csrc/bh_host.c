@@ -169,8 +169,9 @@ static unsigned long long* stamp_of(NbspBarnesHut* b, int unread, int phase) {
     return unread ? NULL : b->counters + NBSP_BH_COUNTERS + phase;
 }
 
-/* The bounds, the sorted keys and permutation, and the walk's records in that
- * order.  tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
+/* The bounds, the sorted keys and permutation, and the walk's records: up to
+ * NBSP_BH_SMALL_SORT particles in that order too, beyond in input order, for the
+ * gather.  tol_scale > 0: also the relative opening test's tolerances (alpha / G). */
 static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, double tol_scale,
                                 int unread, int* status, cudaStream_t stream) {
     const int rel = tol_scale > 0.0;
@@ -195,8 +196,6 @@ static NBodySimProStatus morton(NbspBarnesHut* b, const NbspBarnesHutState* s, d
                  b->counters, stream);
     nbsp_bh_sort(b->keys, b->index, b->keys_alt, b->index_alt, s->n, b->hist, status,
                  stamp_of(b, unread, NBSP_BH_SORT), stream);
-    nbsp_bh_gather(b->unsorted, b->index, s->n, b->pos4, rel ? b->tol_unsorted : NULL,
-                   rel ? b->tol : NULL, status, stamp_of(b, unread, NBSP_BH_BUILD), stream);
     return N_BODY_SIM_PRO_STATUS_OK;
 }
 
@@ -227,9 +226,13 @@ NBodySimProStatus nbsp_bh_accelerations(NbspBarnesHut** handle, const NbspBarnes
     const int rel = tol_scale > 0.0;
     const int late = rel && s->late != NULL;
     if (late) BH_TRY(cudaEventRecord(s->late->before, stream));
-    morton(b, s, late ? 0.0 : tol_scale, unread, status, stream);
+    const int gathered = n <= NBSP_BH_SMALL_SORT, early = rel && !late; /* early: tolerances */
+    morton(b, s, early ? tol_scale : 0.0, unread, status, stream);
+    if (!gathered)
+        nbsp_bh_gather(b->unsorted, b->index, n, b->pos4, early ? b->tol_unsorted : NULL,
+                       early ? b->tol : NULL, status, stamp_of(b, unread, NBSP_BH_BUILD), stream);
     nbsp_bh_build(b->keys, b->index, s->x, s->y, s->z, n, p->leaf_capacity, b->tree, status,
-                  n <= NBSP_BH_SMALL_SORT ? stamp_of(b, unread, NBSP_BH_BUILD) : NULL, stream);
+                  gathered ? stamp_of(b, unread, NBSP_BH_BUILD) : NULL, stream);
     if (late) {
         BH_TRY(fetch_late(s, stream));
         nbsp_bh_late_tolerances(s->ax, s->ay, s->az, n, tol_scale, b->index, b->partial, b->tol,

@@ -3,7 +3,6 @@ faked on the CPU: a launcher's work takes 1 us times a power of two, so that a s
 of them says which ones a phase holds."""
 import ctypes as C
 
-import numpy as np
 import pytest
 
 import host_build
@@ -127,3 +126,10 @@ def test_each_launcher_counts_in_its_own_phase(host, n):
     assert held(t.walk_ms) == {"walk"}
     assert held(t.integrate_ms) == {"unsort"}
     assert held(t.total_ms) == set(WORK) - (set() if large else {"clear", "gather"})
+
+
+@pytest.mark.parametrize("n", [2, 98305])
+def test_an_order_alone_gathers_no_records(host, n):
+    before = host.fake_gather_count()
+    assert host.fake_evaluate(n, 1, None) == nb.Status.OK
+    assert host.fake_gather_count() == before
