@@ -654,19 +654,22 @@ static ArrayKind byte_kind(const char* at, char** device) {
 
 /* by_kernel: the array is read or written through *device, so each of its pages has
  * to be page-locked and at its place there (memory is mapped by pages of 4 KiB or
- * more); for the copies, which check their range themselves, the two ends tell. */
+ * more: one byte of each is asked about, from the last page to the first, and both
+ * ends); for the copies, which check their range themselves, the two ends tell.
+ * The questions cost a call on page-locked arrays 1 us at 1000 particles. */
 static ArrayKind array_kind(const double* array, size_t n, int by_kernel, double** device) {
     const char* const first = (const char*)array;
     const char* const last = first + n * sizeof(double) - 1;
     char *origin, *there;
     const ArrayKind kind = byte_kind(first, &origin);
     *device = (double*)origin;
-    for (const char* at = last; at > first;) {
+    const uintptr_t page = 4095;
+    for (const char* at = last; at > first; at -= ((uintptr_t)at & page) + 1) {
+        if (at != last && ((uintptr_t)at | page) == ((uintptr_t)first | page)) break;
         if (byte_kind(at, &there) != kind) return ARRAY_OTHER;
         if (kind != ARRAY_LOCKED) break;
         if (there - origin != at - first) return ARRAY_OTHER;
         if (!by_kernel) break;
-        at -= ((uintptr_t)at & 4095) + 1; /* the end of the page before */
     }
     return kind;
 }
