@@ -195,9 +195,10 @@ typedef enum NBodySimProCudaAlgorithm {
 } NBodySimProCudaAlgorithm;
 
 /* Per-phase device time of the most recent evaluation, milliseconds: Barnes-Hut
- * phases from the GPU's clock at each phase's start (it ticks every 1 to 2 us), the
- * rest from CUDA events.  A plugin call's wait for its accelerations, which come in
- * while the tree is built, counts with build_ms. */
+ * phases from the GPU's clock at each phase's start (it ticks every 1 to 2 us, which
+ * in systems of some thousand particles is much of a phase), the rest and the total
+ * from CUDA events.  A plugin call's wait for its accelerations, which come in while
+ * the tree is built, counts with build_ms. */
 typedef struct NBodySimProCudaTimings {
     double bounds_ms;      /* bbox + centre-of-mass reduction */
     double keys_ms;        /* Morton keys */
@@ -605,7 +606,9 @@ N_BODY_SIM_PRO_CUDA_API NBodySimProStatus n_body_sim_pro_cuda_context_set_correc
  * gravity, leapfrog KDK: src/c/physics/gravity.c:37-67 and
  * src/c/physics/integrator.c:47-85 per system) advanced together.  The
  * reference has no ensemble driver: a user would loop
- * n_body_sim_pro_integrator_advance over the systems.
+ * n_body_sim_pro_integrator_advance over the systems.  A system evolves to the same
+ * bits whatever other systems are uploaded with it and whichever tile shape the
+ * autotuner takes (one_launch_per_system rounds differently).
  */
 typedef struct NBodySimProCudaEnsemble NBodySimProCudaEnsemble;
 
@@ -613,7 +616,7 @@ typedef struct NBodySimProCudaEnsembleInfo {
     size_t systems;
     size_t particles;
     int threads_per_block;      /* autotuned tile shape */
-    int targets_per_thread;
+    int targets_per_thread;     /* of a system of 4096 particles */
     int grid;                   /* persistent CTAs (one resident wave) */
     int work_items;             /* system bundles, longest first */
     double last_advance_ms;     /* device time of the last advance */

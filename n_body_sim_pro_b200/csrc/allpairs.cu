@@ -347,7 +347,8 @@ __global__ void finalize_kernel(const float4* __restrict__ hi, const float4* __r
 // the kernels read the inputs and write the accelerations where the caller (or
 // the context's page-locked staging) has them, through the mapped addresses of
 // page-locked memory: a plugin call at 1000 particles 106 -> 42 us, at 2000
-// 116 -> 47.
+// 116 -> 47 (of the 42 the packing kernel 6.5 and the forces 14; the rest is two
+// launches, the wait, and the host's questions and copies of the arrays).
 
 // Centre of mass and packed sources, one CTA.  *report (mapped host memory) is
 // the status of the call.

@@ -2273,8 +2273,9 @@ static_assert(kCtaStack + kFrontier <= 3 * kListStack, "frontier inside warp 2's
 // from the group centre (so one evaluation there stands for all 32 targets),
 // is appended to the group's list; the walk itself computes the plain
 // monopole, exactly as without the correction.
-// Register budgets: monopole walk 64 (8 blocks of 4 warps per SM), quadrupole
-// walk 102 (5 blocks).
+// Register budgets: monopole walk 56 (9 blocks of 4 warps per SM; the shared-top
+// walk and the corrected walk under the relative test 64, 8 blocks), quadrupole
+// walk 96 (5 blocks); the latency forms 80 (6 blocks) and 119 to 125 (4 blocks).
 //
 // SHARED: the top of the tree is traversed once for the block's 4 groups.  The
 // 128 threads test up to 128 nodes at a time against the 4 group boxes: a node

@@ -3,9 +3,9 @@
  *
  * Upload: systems are concatenated SoA ranges [offsets[k], offsets[k+1]).
  * Advance, persistent mode: one CUDA-graph launch of ensemble.cu's persistent
- * kernel runs `steps` leapfrog steps of every system; the tile shape (threads
- * per CTA x targets per thread) is chosen by a measuring autotuner on the
- * uploaded ensemble, and the work items are ordered longest-first.
+ * kernel runs `steps` leapfrog steps of every system; the threads per CTA are
+ * chosen by a measuring autotuner on the uploaded ensemble (no bit of a system's
+ * result depends on them), and the work items are ordered longest-first.
  * Advance, per-system mode (the baseline): the single-system all-pairs path,
  * launched system by system and step by step.
  */
@@ -34,7 +34,8 @@ NBSP_HIDDEN void nbsp_ensemble_advance(int block, int grid, double* x, double* y
 enum { ENS_MAX_SYSTEM = 4096, ENS_SHAPES = 3, ENS_TILE = 64 /* = kTile in ensemble.cu */,
        ENS_TILES = ENS_MAX_SYSTEM / ENS_TILE /* tiles of a CTA's particle slots */ };
 
-/* threads per CTA; targets per thread of a system that fills the CTA's slots */
+/* threads per CTA; what the info reports as targets per thread: a thread's share,
+ * rounded up, of a system that fills the CTA's slots (it holds two at a time) */
 static const int kEnsShapes[ENS_SHAPES][2] = {{1024, 4}, {768, 6}, {512, 8}};
 
 typedef struct Items {

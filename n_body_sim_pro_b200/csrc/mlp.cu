@@ -10,7 +10,8 @@
 // weights and of the BF16 fragments.
 //
 // A step of a small minibatch is bound by latency (1024 rows: 8 CTAs, 3e7 flop),
-// so an epoch is one cooperative launch instead of three a step: with it, the
+// so an epoch is one launch instead of three a step: of one cluster up to 8 CTAs,
+// a cooperative one up to 32 (4096 rows; beyond, three a step).  With it, the
 // ldmatrix fragments and the forward-only losses an epoch of 245,760 rows in
 // steps of 1024, its shuffle and losses included, takes 3.1 ms instead of 8.7
 // (1.2 of them the shuffle, on the host).
@@ -492,10 +493,11 @@ __device__ __forceinline__ RowInputs fetched_rows(const uint32_t* rows, int warp
 }
 
 // All the steps of an epoch in one launch (one cluster, or a cooperative launch),
-// a CTA per 128 rows of the minibatch.  A step: every CTA's gradient into its slot; then every CTA sums all
-// slots for its share of the parameters, in the slots' order, updates them and
-// their moments (its own, in shared memory until the end) and puts their new
-// BF16 forms into the fragments in global memory; then every CTA takes those.
+// a CTA per 128 rows of the minibatch.  A step: every CTA's gradient into its slot;
+// then every CTA sums all slots for its share of the parameters, in the slots'
+// order, updates them and their moments (its own, in shared memory until the end)
+// and puts their new BF16 forms into the fragments in global memory; then every
+// CTA takes those.
 // (Each CTA updating all parameters for itself saves the second wait, but the
 // update is division-bound: 6.3 us of a step at 8 CTAs against 2.4, the second wait
 // and the copy included.)

@@ -380,7 +380,7 @@ NBodySimProStatus n_body_sim_pro_cuda_correction_train(NBodySimProCudaCorrection
     const int ctas = batch / per;
     const size_t n = c->train_rows;
     const int steps = (int)(n / (size_t)batch);
-    /* an epoch in one cooperative launch, up to the minibatch its blocks sum */
+    /* an epoch in one launch, up to the minibatch whose gradients its blocks sum */
     const int one_launch = ctas <= nbsp_mlp_epoch_ctas() && steps > 0;
     NBodySimProStatus st = ensure_slots(c, ctas, error);
     if (st != N_BODY_SIM_PRO_STATUS_OK) return st;
