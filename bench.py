@@ -129,12 +129,12 @@ DRIFT_STEPS = 10
 # capture of exactly this configuration (the file under profiles/ gives the command).
 PROFILED_TRAFFIC = {
     ("bh_collision_1m", 0.7, 1, "lists", 16, 0.0): (
-        31_626_240, "profiles/walk_lists_kernel_bh_collision_1m.md"),
+        27_629_312, "profiles/walk_lists_kernel_bh_collision_1m.md"),
     ("allpairs_plummer_16k", None, 1, "lists", 16, 0.0): (
         296_960, "profiles/allpairs_force_paired_kernel_plummer_16k.md"),
     # one-pass DRAM capture of the full 10M walk launch
     ("bh_matched_10m", 5.0, 1, "lists", 32, 0.0045): (
-        622_074_624, "profiles/bh_step_launches_relative_10m.md"),
+        601_478_912, "profiles/bh_step_launches_relative_10m.md"),
 }
 
 FP32_LANES_PER_SM = 128  # FFMA lanes per Blackwell SM
